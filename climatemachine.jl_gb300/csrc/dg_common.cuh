@@ -212,13 +212,54 @@ __device__ __forceinline__ Level<float> load_level<float>(const KParams& P, int 
     return l;
 }
 
-// Reciprocal and square root in the working precision: correctly rounded in
-// FP64; the hardware approximations (a few ulp) in FP32, where every other
-// operation already carries FP32 rounding.
-__device__ __forceinline__ double rcp_r(double x) { return 1.0 / x; }
+// Reciprocal and square root in the working precision.  FP32: the hardware
+// approximations (a few ulp), where every other operation already carries
+// FP32 rounding.  FP64: the pipe is the bound of every FP64 kernel (1/72 of
+// the FP32 rate), so the seed comes from the hardware's approximation
+// instructions (about 20 correct bits, off that pipe) and one step of
+// Householder's third-order iteration (the binomial series of (1 - h)^-1 and
+// (1 - h)^-1/2 about the seed, cut after h^2) takes its error e to e^3, under
+// FP64 rounding: 3 FP64 operations for a reciprocal, 5 for a root.  The
+// results stay within 2 ulp of the correctly rounded ones.
+__device__ __forceinline__ double rcp_r(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double h = fma(-x, y, 1.0);
+    return fma(y, fma(h, h, h), y);
+}
 __device__ __forceinline__ float rcp_r(float x) { return __fdividef(1.0f, x); }
-__device__ __forceinline__ double sqrt_r(double x) { return sqrt(x); }
+// len = sqrt(x), rlen = 1 / sqrt(x) for x > 0
+__device__ __forceinline__ void sqrt_rsqrt_r(double x, double& len, double& rlen) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double t = x * y;
+    const double h = fma(-t, y, 1.0);
+    const double g = h * fma(h, 0.375, 0.5);
+    len = fma(t, g, t);
+    rlen = fma(y, g, y);
+}
+__device__ __forceinline__ void sqrt_rsqrt_r(float x, float& len, float& rlen) {
+    len = x * rsqrtf(x);
+    rlen = __fdividef(1.0f, len);
+}
+// FP64: zero (and the subnormals the seed instruction flushes) gives zero
+__device__ __forceinline__ double sqrt_r(double x) {
+    double len, rlen;
+    sqrt_rsqrt_r(x, len, rlen);
+    return (unsigned)__double2hiint(x) >= 0x00100000u ? len : 0.0;
+}
 __device__ __forceinline__ float sqrt_r(float x) { return x * rsqrtf(x); }
+
+// finiteness and the larger of two non-negative values; in FP64 on the
+// integer pipe (comparisons of doubles issue on the FP64 pipe)
+__device__ __forceinline__ bool finite_r(float x) { return isfinite(x); }
+__device__ __forceinline__ bool finite_r(double x) {
+    return ((unsigned)__double2hiint(x) & 0x7FF00000u) != 0x7FF00000u;
+}
+__device__ __forceinline__ float max_nonneg(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+    return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;
+}
 
 // Pointwise thermodynamics of dry air (PhaseDry: T = T0 + e_int/cv, p = rho R T,
 // c = sqrt(gamma R T)) for a conserved state q, which is the full state
@@ -232,7 +273,7 @@ struct Thermo {
     R c;      // sound speed
 };
 
-template <typename R, bool MIXED>
+template <typename R, bool MIXED, bool VEL = true>
 __device__ __forceinline__ Thermo<R, MIXED> thermo(const R q[NSTATE], const Level<R>& lv, const KParams& P) {
     Thermo<R, MIXED> t;
     const Physics& ph = P.ph;
@@ -242,7 +283,10 @@ __device__ __forceinline__ Thermo<R, MIXED> thermo(const R q[NSTATE], const Leve
     t.u[0] = q[1] * t.rinv;
     t.u[1] = q[2] * t.rinv;
     t.u[2] = q[3] * t.rinv;
-    R ke2 = q[1] * t.u[0] + q[2] * t.u[1] + q[3] * t.u[2];
+    // VEL: the caller uses the velocities; otherwise they are dead and the
+    // kinetic energy is formed without them
+    R ke2 = VEL ? q[1] * t.u[0] + q[2] * t.u[1] + q[3] * t.u[2]
+                : (q[1] * q[1] + q[2] * q[2] + q[3] * q[3]) * t.rinv;
     R p;
     if (MIXED) {
         // p' = gm1 (rhoe' - ke/2) + rho' crho ; p = p_ref + p'
@@ -272,6 +316,38 @@ __device__ __forceinline__ R flux_d(const R q[NSTATE], const Thermo<R, MIXED>& t
 template <typename R>
 __device__ __forceinline__ R pick3(int d, R a, R b, R c) {
     return d == 0 ? a : (d == 1 ? b : c);
+}
+
+// S = Fm + F_d(q): the sum of the two sides' fluxes along +xi_d across a face
+// normal to xi_d, the far side from its state and thermodynamics (the
+// momentum flux as u_d q, so that the sum is one FMA per field)
+template <typename R, bool MIXED>
+__device__ __forceinline__ void add_flux_d(const R Fm[NSTATE], const R q[NSTATE], R mn, R un, R pflux, R H, int d,
+                                           R S[NSTATE]) {
+    S[0] = Fm[0] + mn;
+    S[1] = fma(un, q[1], Fm[1]);
+    S[2] = fma(un, q[2], Fm[2]);
+    S[3] = fma(un, q[3], Fm[3]);
+    const R sn = pick3(d, S[1], S[2], S[3]) + pflux;
+    S[1] = d == 0 ? sn : S[1];
+    S[2] = d == 1 ? sn : S[2];
+    S[3] = d == 2 ? sn : S[3];
+    S[4] = fma(un, H, Fm[4]);
+}
+
+// lifted numerical flux hl S + pl ((qm - qp) + jr) of one face node: hl half
+// the signed lift, pl the penalty's weight, jr the reference-state jumps of
+// the density and the energy (mixed precision only)
+template <typename R, bool MIXED>
+__device__ __forceinline__ void lifted_flux(const R S[NSTATE], const R qm[NSTATE], const R qp[NSTATE], R jr_rho,
+                                            R jr_rhoe, R hl, R pl, R fs[NSTATE]) {
+#pragma unroll
+    for (int s = 0; s < NSTATE; ++s) {
+        R dq = qm[s] - qp[s];
+        if (MIXED && s == 0) dq += jr_rho;
+        if (MIXED && s == 4) dq += jr_rhoe;
+        fs[s] = fma(hl, S[s], pl * dq);
+    }
 }
 
 // normal first-order flux F_d (all 5 fields) for a face normal to xi_d

@@ -241,16 +241,16 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
         const R j1 = ge[(KG_JXI + fd * 3 + 1) * Np + vM];
         const R j2 = ge[(KG_JXI + fd * 3 + 2) * Np + vM];
         const R iJm = ge[KG_INVJ * Np + vM];
-        const R sJ = sqrt_r(j0 * j0 + j1 * j1 + j2 * j2);
-        const R rs = rcp_r(sJ);
-        const R nv[3] = {sgn * j0 * rs, sgn * j1 * rs, sgn * j2 * rs};
-        R qm[NSTATE], Fm[NSTATE], qp[NSTATE], Fp[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
+        R sJ, rs;
+        sqrt_rsqrt_r(j0 * j0 + j1 * j1 + j2 * j2, sJ, rs);
+        rs *= sgn;
+        const R nv[3] = {j0 * rs, j1 * rs, j2 * rs};
+        R qm[NSTATE], Fm[NSTATE], qp[NSTATE], S[NSTATE], jr_rho = 0, jr_rhoe = 0;
         PL::ld(s_node, Np, vM, qm);
         const CRV cr = s_cr[vM];
         const R c_m = cr.x, ri_m = cr.y;
         PL::ld(s_F + fd * SM::P5N, Np, vM, Fm);
-#pragma unroll
-        for (int s = 0; s < NSTATE; ++s) Fm[s] *= sgn * rs;
+        R am = rs;  // Fm = am times the staged contravariant flux (on some walls Fm is the normal flux, am = 1)
         const R mn_m = qm[1] * nv[0] + qm[2] * nv[1] + qm[3] * nv[2];
         const R lam_m = fabs(mn_m * ri_m) + c_m;
         const int nb = __ldg(nbr + f);
@@ -265,8 +265,8 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
                 if (MIXED && ph.numflux == CMDG_FLUX_RUSANOV) {
                     const int ej = fside ? ezp : ez;
                     const R sj = fside ? R(-1) : R(1);
-                    jr[0] = sj * (R)P.jump32[2 * ej + 0];
-                    jr[4] = sj * (R)P.jump32[2 * ej + 1];
+                    jr_rho = sj * (R)P.jump32[2 * ej + 0];
+                    jr_rhoe = sj * (R)P.jump32[2 * ej + 1];
                 }
             } else {
                 vP = shell_partner<N>(nbr, f, fn);
@@ -285,6 +285,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
                 // the staged flux holds the second-order part too: walls take the first-order one
                 const Level<R> lvm = shell_level<R, MIXED>(P, ge, Np, vM, ez * Nq + kM);
                 const Thermo<R, MIXED> thm = thermo<R, MIXED>(qm, lvm, P);
+                am = R(1);
                 Fm[0] = mn_m;
 #pragma unroll
                 for (int c = 0; c < 3; ++c) Fm[1 + c] = mn_m * thm.u[c] + thm.pflux * nv[c];
@@ -304,27 +305,29 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
             }
             if (MIXED && ph.numflux == CMDG_FLUX_RUSANOV) {
                 // per-node part of the reference jump q_ref(-) - q_ref(+)
-                jr[0] += ge[KG_DRHO * Np + vM] - drp;
-                jr[4] += ge[KG_DRHOE * Np + vM] - dep;
+                jr_rho += ge[KG_DRHO * Np + vM] - drp;
+                jr_rhoe += ge[KG_DRHOE * Np + vM] - dep;
             }
         }
-        const Thermo<R, MIXED> thp = thermo<R, MIXED>(qp, lvp, P);
+        const Thermo<R, MIXED> thp = thermo<R, MIXED, false>(qp, lvp, P);
         const R mn_p = qp[1] * nv[0] + qp[2] * nv[1] + qp[3] * nv[2];
         const R un_p = mn_p * thp.rinv;
-        Fp[0] = mn_p;
+        // S: the two sides' normal fluxes added up
+        S[0] = fma(am, Fm[0], mn_p);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) Fp[1 + c] = mn_p * thp.u[c] + thp.pflux * nv[c];
-        Fp[4] = un_p * thp.H;
+        for (int c = 0; c < 3; ++c) S[1 + c] = fma(am, Fm[1 + c], fma(un_p, qp[1 + c], thp.pflux * nv[c]));
+        S[4] = fma(am, Fm[4], un_p * thp.H);
         R cL = 0;  // REM, faces normal to xi3: the linear model's Rusanov speed
         if (REM && fd == 2) {
             // F - F_L of the node across the face (or of the reflected state on a wall)
-            const R pke_p = KConst<R>::gm1(P) * R(0.5) * (qp[1] * thp.u[0] + qp[2] * thp.u[1] + qp[3] * thp.u[2]);
+            const R pke_p =
+                KConst<R>::gm1(P) * R(0.5) * ((qp[1] * qp[1] + qp[2] * qp[2] + qp[3] * qp[3]) * thp.rinv);
             const R hrem_p =
                 ((qp[4] + thp.pflux) * lvp.rho_ref - lvp.href * qp[0]) * thp.rinv * rcp_r(lvp.rho_ref);
-            Fp[0] = 0;
+            S[0] = am * Fm[0];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) Fp[1 + c] = mn_p * thp.u[c] - pke_p * nv[c];
-            Fp[4] = mn_p * hrem_p;
+            for (int c = 0; c < 3; ++c) S[1 + c] = fma(am, Fm[1 + c], fma(un_p, qp[1 + c], -(pke_p * nv[c])));
+            S[4] = fma(am, Fm[4], mn_p * hrem_p);
             const Level<R> lvm = shell_level<R, MIXED>(P, ge, Np, vM, ez * Nq + kM);
             const R gam = KConst<R>::gamma(P);
             cL = fmax(sqrt_r(gam * lvm.p_ref * rcp_r(lvm.rho_ref)), sqrt_r(gam * lvp.p_ref * rcp_r(lvp.rho_ref)));
@@ -338,25 +341,30 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
                 hn_n[c] = nv[0] * hn[(3 * c + 0) * Np] + nv[1] * hn[(3 * c + 1) * Np] + nv[2] * hn[(3 * c + 2) * Np];
             const R rho_p = MIXED ? lvp.rho_ref + qp[0] : qp[0];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) Fp[1 + c] += rho_p * hn_n[c];
-            Fp[4] += (hn_n[0] * qp[1] + hn_n[1] * qp[2] + hn_n[2] * qp[3]) + hn_n[3] * rho_p;
+            for (int c = 0; c < 3; ++c) S[1 + c] += rho_p * hn_n[c];
+            S[4] += (hn_n[0] * qp[1] + hn_n[1] * qp[2] + hn_n[2] * qp[3]) + hn_n[3] * rho_p;
         }
         if (VISC && nb >= 0) {
             // neighbour's viscous flux . n
             R Fv[3][NSTATE];
             shell_visc_flux<R, MIXED, VT>(P, nb, vP, Np, qp, lvp, thp.rinv, Fv);
 #pragma unroll
-            for (int s2 = 0; s2 < NSTATE; ++s2) Fp[s2] += nv[0] * Fv[0][s2] + nv[1] * Fv[1][s2] + nv[2] * Fv[2][s2];
+            for (int s2 = 0; s2 < NSTATE; ++s2) S[s2] += nv[0] * Fv[0][s2] + nv[1] * Fv[1][s2] + nv[2] * Fv[2][s2];
         }
         const R lam_p = fabs(un_p) + thp.c;
         const R lift = sJ * iJm * KConst<R>::inv_w0(P);
-        const R hmw = (ph.numflux == CMDG_FLUX_RUSANOV) ? R(0.5) * fmax(lam_m, lam_p) : R(0);
-        const R hl = R(0.5) * lift, pl = hmw * lift;
+        const R hl = R(0.5) * lift;
+        const R pl = (ph.numflux == CMDG_FLUX_RUSANOV) ? hl * max_nonneg(lam_m, lam_p) : R(0);
         // REM: the linear model's penalty cL/2 on the perturbation jump comes off
-        const R pq = (REM && fd == 2) ? (hmw - R(0.5) * cL) * lift : pl;
+        const R pq = (REM && fd == 2) ? pl - hl * cL : pl;
         R fs[NSTATE];
+        if constexpr (MIXED) {
 #pragma unroll
-        for (int s = 0; s < NSTATE; ++s) fs[s] = hl * (Fm[s] + Fp[s]) + (pq * (qm[s] - qp[s]) + pl * jr[s]);
+            for (int s = 0; s < NSTATE; ++s)
+                fs[s] = fma(hl, S[s], fma(pq, qm[s] - qp[s], s == 0 ? pl * jr_rho : (s == 4 ? pl * jr_rhoe : R(0))));
+        } else {
+            lifted_flux<R, MIXED>(S, qm, qp, R(0), R(0), hl, pl, fs);
+        }
         PL::st(s_fs, NFN, f * Nfp + fn, fs);
     }
     __syncthreads();
@@ -396,7 +404,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
         const R rkb_dt = KConst<R>::rkb_dt(P);
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) {
-            if (!isfinite(rhs[s])) bad = 1;
+            if (!finite_r(rhs[s])) bad = 1;
             const size_t idx = ebase + s * Np;
             if (MODE == 0) {
                 double out = P.alpha * (double)rhs[s];

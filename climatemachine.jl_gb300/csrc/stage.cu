@@ -39,6 +39,13 @@
 // which is exact algebra for dry air (T = T0 + e_int/cv, p = rho R T), the
 // reference-state jump across vertical faces enters the Rusanov penalty
 // from an FP64-computed table, and the RK register dQ stays FP64.
+//
+// The FP64 form is bound by the FP64 pipe (1.8 lane operations per cycle and
+// SM), so its operations are counted: reciprocals and roots of 3 and 5
+// operations (rcp_r, sqrt_r), one FMA per field for the sum of a face's two
+// fluxes, the metric folded into the derivative coefficients, comparisons on
+// the integer pipe.  About 240 operations per node became 185 and a step of
+// the 1 M-node bubble went from 2.304 to 1.852 ms.
 #include <cooperative_groups.h>
 
 #include "dg_common.cuh"
@@ -84,7 +91,8 @@ struct Smem {
     static constexpr int FLUX = CR + planar_pad<R>(2 * Np);
     static constexpr int FACE = FLUX + 3 * P5N;
     static constexpr int DMAT = FACE + planar_pad<R>(3 * 5 * Np);
-    static constexpr int TOTAL = DMAT + Nq * Nq;
+    // FP64: the derivative already scaled by the metric, one copy per direction
+    static constexpr int TOTAL = DMAT + (sizeof(R) == 8 ? 3 : 1) * Nq * Nq;
     static constexpr size_t BYTES = sizeof(R) * TOTAL;
 };
 
@@ -223,7 +231,11 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
     };
     const R sgn = fside ? R(1) : R(-1);
 
-    if (!PARAM_D && t < Nq * Nq) s_D[t] = static_cast<const R*>(P.Dhat)[t];
+    // FP64: the element's metric goes into the derivative coefficients (three
+    // copies, one multiplication per coefficient of the element instead of
+    // three per node and field)
+    constexpr bool SCALED_D = sizeof(R) == 8;
+    if (!PARAM_D && !SCALED_D && t < Nq * Nq) s_D[t] = static_cast<const R*>(P.Dhat)[t];
 
     auto fetch = [&](int e, Ahead<R>& a) {
         const int* nbr = P.nbr + NBR_STRIDE * e;
@@ -354,6 +366,12 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
         const int ez = cur.ez;
         const R xi[3] = {KConst<R>::metric(P, e, 0), KConst<R>::metric(P, e, 1), KConst<R>::metric(P, e, 2)};
 
+        if (SCALED_D && t < Nq * Nq) {
+            const R d = static_cast<const R*>(P.Dhat)[t];
+#pragma unroll
+            for (int dd = 0; dd < 3; ++dd) s_D[dd * Nq * Nq + t] = d * xi[dd];
+        }
+
         // ---------------- phase 1: node thermodynamics and volume fluxes
         R gsrc = 0;
         if (node_thread) {
@@ -380,13 +398,15 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
 
         // ---------------- phase 2: one numerical flux per face node
         if (face_thread) {
-            R qm[NSTATE], Fm[NSTATE], Fp[NSTATE], qp[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
+            R qm[NSTATE], Fm[NSTATE], Fp[NSTATE], S[NSTATE], qp[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
             PL::ld(s_node, Np, vM, qm);
             const CRV cr = s_cr[vM];
             const R c_m = cr.x, ri_m = cr.y;
             PL::ld(s_F + fd * SM::P5N, Np, fside * N * Nfp + fn, Fm);  // dir_rec(fd) of vM
+            if (MIXED) {
 #pragma unroll
-            for (int s = 0; s < NSTATE; ++s) Fm[s] *= sgn;
+                for (int s = 0; s < NSTATE; ++s) Fm[s] *= sgn;
+            }
             const R lam_m = fabs(pick3(fd, qm[1], qm[2], qm[3]) * ri_m) + c_m;
             int ezp = ez;
             if (cur.nb >= 0) {
@@ -423,20 +443,36 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
                 const CRV crp = cl.map_shared_rank(s_cr, (unsigned)nrank)[vP];
                 PL::ld(cl.map_shared_rank(s_F + fd * SM::P5N, (unsigned)nrank), Np, oside * N * Nfp + fn, Fp);
 #pragma unroll
-                for (int s = 0; s < NSTATE; ++s) Fp[s] *= sgn;
+                for (int s = 0; s < NSTATE; ++s) {
+                    if (MIXED) Fp[s] *= sgn;
+                    else S[s] = Fm[s] + Fp[s];
+                }
                 lam_p = fabs(pick3(fd, qp[1], qp[2], qp[3]) * crp.y) + crp.x;
             } else {
                 const Level<R> lvp = load_level<R>(P, ezp * Nq + (cur.nb >= 0 ? kP : kM));
-                const Thermo<R, MIXED> thp = thermo<R, MIXED>(qp, lvp, P);
-                normal_flux<R, MIXED>(qp, thp, fd, sgn, Fp);
-                lam_p = fabs(pick3(fd, thp.u[0], thp.u[1], thp.u[2])) + thp.c;
+                const Thermo<R, MIXED> thp = thermo<R, MIXED, MIXED>(qp, lvp, P);
+                if (MIXED) {
+                    normal_flux<R, MIXED>(qp, thp, fd, sgn, Fp);
+                    lam_p = fabs(pick3(fd, thp.u[0], thp.u[1], thp.u[2])) + thp.c;
+                } else {
+                    const R mn = pick3(fd, qp[1], qp[2], qp[3]);
+                    const R un = mn * thp.rinv;
+                    add_flux_d<R, MIXED>(Fm, qp, mn, un, thp.pflux, thp.H, fd, S);
+                    lam_p = fabs(un) + thp.c;
+                }
             }
             const R lift = pick3(fd, xi[0], xi[1], xi[2]) * KConst<R>::inv_w0(P);
-            const R hmw = (ph.numflux == CMDG_FLUX_RUSANOV) ? R(0.5) * fmax(lam_m, lam_p) : R(0);
+            const R hmw = (ph.numflux == CMDG_FLUX_RUSANOV) ? R(0.5) * max_nonneg(lam_m, lam_p) : R(0);
             const R hl = R(0.5) * lift, pl = hmw * lift;
             R fs[NSTATE];
+            if (MIXED) {
+                // FP32: the fluxes with the face's sign; the FP64 form below
+                // measured 3.8% slower here at N = 5 and the same at N = 4
 #pragma unroll
-            for (int s = 0; s < NSTATE; ++s) fs[s] = hl * (Fm[s] + Fp[s]) + pl * ((qm[s] - qp[s]) + jr[s]);
+                for (int s = 0; s < NSTATE; ++s) fs[s] = hl * (Fm[s] + Fp[s]) + pl * ((qm[s] - qp[s]) + jr[s]);
+            } else {
+                lifted_flux<R, MIXED>(S, qm, qp, R(0), R(0), sgn * hl, pl, fs);
+            }
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) s_fs[(fd * NSTATE + s) * Np + vM] = fs[s];
         }
@@ -448,29 +484,40 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
         // ---------------- phase 3: volume contraction, face terms, source, update
         int bad = 0;
         if (node_thread) {
-            R acc1[NSTATE] = {0, 0, 0, 0, 0}, acc2[NSTATE] = {0, 0, 0, 0, 0}, acc3[NSTATE] = {0, 0, 0, 0, 0};
+            R rhs[NSTATE];
             const int L1 = nj + Nq * nk;  // line along xi1 (records n Nfp + L1)
             const int L2 = ni + Nq * nk;  // line along xi2 (records n Nfp + L2)
             const int L3 = ni + Nq * nj;         // line along xi3 (stride Nfp)
+            R acc1[NSTATE] = {0, 0, 0, 0, 0}, acc2[NSTATE] = {0, 0, 0, 0, 0}, acc3[NSTATE] = {0, 0, 0, 0, 0};
 #pragma unroll
             for (int n = 0; n < Nq; ++n) {
                 R v1[NSTATE], v2[NSTATE], v3[NSTATE];
                 PL::ld(s_F, Np, L1 + n * Nfp, v1);
                 PL::ld(s_F + SM::P5N, Np, L2 + n * Nfp, v2);
                 PL::ld(s_F + 2 * SM::P5N, Np, L3 + n * Nfp, v3);
-                const R d1 = PARAM_D ? dhat_const<R>(P, ni * Nq + n) : s_D[ni * Nq + n];
-                const R d2 = PARAM_D ? dhat_const<R>(P, nj * Nq + n) : s_D[nj * Nq + n];
-                const R d3 = PARAM_D ? dhat_const<R>(P, nk * Nq + n) : s_D[nk * Nq + n];
+                if constexpr (SCALED_D) {
+                    const R d1 = s_D[ni * Nq + n], d2 = s_D[Nq * Nq + nj * Nq + n], d3 = s_D[2 * Nq * Nq + nk * Nq + n];
 #pragma unroll
-                for (int s = 0; s < NSTATE; ++s) {
-                    acc1[s] = fma(d1, v1[s], acc1[s]);
-                    acc2[s] = fma(d2, v2[s], acc2[s]);
-                    acc3[s] = fma(d3, v3[s], acc3[s]);
+                    for (int s = 0; s < NSTATE; ++s) {
+                        acc1[s] = fma(d1, v1[s], acc1[s]);
+                        acc1[s] = fma(d2, v2[s], acc1[s]);
+                        acc1[s] = fma(d3, v3[s], acc1[s]);
+                    }
+                } else {
+                    const R d1 = PARAM_D ? dhat_const<R>(P, ni * Nq + n) : s_D[ni * Nq + n];
+                    const R d2 = PARAM_D ? dhat_const<R>(P, nj * Nq + n) : s_D[nj * Nq + n];
+                    const R d3 = PARAM_D ? dhat_const<R>(P, nk * Nq + n) : s_D[nk * Nq + n];
+#pragma unroll
+                    for (int s = 0; s < NSTATE; ++s) {
+                        acc1[s] = fma(d1, v1[s], acc1[s]);
+                        acc2[s] = fma(d2, v2[s], acc2[s]);
+                        acc3[s] = fma(d3, v3[s], acc3[s]);
+                    }
                 }
             }
-            R rhs[NSTATE];
 #pragma unroll
-            for (int s = 0; s < NSTATE; ++s) rhs[s] = xi[0] * acc1[s] + xi[1] * acc2[s] + xi[2] * acc3[s];
+            for (int s = 0; s < NSTATE; ++s)
+                rhs[s] = SCALED_D ? acc1[s] : xi[0] * acc1[s] + xi[1] * acc2[s] + xi[2] * acc3[s];
             // face terms (vMI sM F*, lifted in phase 2), in face order 1..6:
             // at most one face per direction holds the node
             auto sub_face = [&](int dd) {
@@ -484,7 +531,7 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
             const R rkb_dt = KConst<R>::rkb_dt(P);
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) {
-                if (!isfinite(rhs[s])) bad = 1;
+                if (!finite_r(rhs[s])) bad = 1;
                 const size_t idx = ebase + s * Np;
                 if (MODE == 0) {
                     double out = P.alpha * (double)rhs[s];

@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
     const int fa = fn % Nq, fb = fn / Nq;
     const int vM = fd == 0 ? fside * N + Nq * fn : (fd == 1 ? fa + Nq * (fside * N + Nq * fb) : fn + Nfp * (fside * N));
     const int vP = fd == 0 ? oside * N + Nq * fn : (fd == 1 ? fa + Nq * (oside * N + Nq * fb) : fn + Nfp * (oside * N));
-    const R sgn = fside ? R(1) : R(-1);
+    const R hsgn = fside ? R(0.5) : R(-0.5);
 
     // record of this node in the direction-d flux plane (contraction index slowest)
     auto dir_rec = [&](int d) {
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
 
     // phase 2: numerical flux per face node (Rusanov/central + central second order)
     if (face_thread) {
-        R qm[NSTATE], Fm[NSTATE], Fp[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
+        R qm[NSTATE], Fm[NSTATE], S[NSTATE], jr_rho = 0, jr_rhoe = 0;
         PL::ld(s_node, Np, vM, qm);
         const CRV cr = s_cr[vM];
         const R c_m = cr.x, ri_m = cr.y;
@@ -361,18 +361,16 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
         const Level<R> lvm = load_level<R>(P, ez * Nq + vM / Nfp);
         if (nb >= 0) {
             PL::ld(s_F + fd * P5N, Np, fside * N * Nfp + fn, Fm);  // dir_rec(fd) of vM
-#pragma unroll
-            for (int s = 0; s < NSTATE; ++s) Fm[s] *= sgn;
             if (MIXED && fd == 2 && ph.numflux == CMDG_FLUX_RUSANOV) {
                 const int ej = fside ? ezp : ez;
                 const R sj = fside ? R(-1) : R(1);
-                jr[0] = sj * (R)P.jump32[2 * ej + 0];
-                jr[4] = sj * (R)P.jump32[2 * ej + 1];
+                jr_rho = sj * (R)P.jump32[2 * ej + 0];
+                jr_rhoe = sj * (R)P.jump32[2 * ej + 1];
             }
         } else {
             // walls: first-order flux only on both sides
             const Thermo<R, MIXED> thm = thermo<R, MIXED>(qm, lvm, P);
-            normal_flux<R, MIXED>(qm, thm, fd, sgn, Fm);
+            normal_flux<R, MIXED>(qm, thm, fd, R(1), Fm);
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) qp[s] = qm[s];
             qp[1] = (fd == 0) ? -qm[1] : qm[1];
@@ -380,28 +378,27 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
             qp[3] = (fd == 2) ? -qm[3] : qm[3];
         }
         const Level<R> lvp = nb >= 0 ? load_level<R>(P, ezp * Nq + vP / Nfp) : lvm;
-        const Thermo<R, MIXED> thp = thermo<R, MIXED>(qp, lvp, P);
-        normal_flux<R, MIXED>(qp, thp, fd, sgn, Fp);
+        const Thermo<R, MIXED> thp = thermo<R, MIXED, false>(qp, lvp, P);
+        const R mn = pick3(fd, qp[1], qp[2], qp[3]);
+        const R un = mn * thp.rinv;
+        add_flux_d<R, MIXED>(Fm, qp, mn, un, thp.pflux, thp.H, fd, S);
         if (nb >= 0) {
             const R rho = MIXED ? lvp.rho_ref + qp[0] : qp[0];
-            const R ru[3] = {qp[1], qp[2], qp[3]};
             if (VISC) {
 #pragma unroll
-                for (int s = 1; s < NSTATE; ++s) Fp[s] += sgn * f2p[s - 1];
+                for (int s = 1; s < NSTATE; ++s) S[s] += f2p[s - 1];
             }
             if (HYPER) {
-                Fp[1] += sgn * (rho * hdp[0]);
-                Fp[2] += sgn * (rho * hdp[1]);
-                Fp[4] += sgn * ((hdp[0] * ru[0] + hdp[1] * ru[1]) + hdp[2] * rho);
+                S[1] += rho * hdp[0];
+                S[2] += rho * hdp[1];
+                S[4] += (hdp[0] * qp[1] + hdp[1] * qp[2]) + hdp[2] * rho;
             }
         }
-        const R lam_p = fabs(pick3(fd, thp.u[0], thp.u[1], thp.u[2])) + thp.c;
+        const R lam_p = fabs(un) + thp.c;
         const R lift = pick3(fd, xi[0], xi[1], xi[2]) * KConst<R>::inv_w0(P);
-        const R hmw = (ph.numflux == CMDG_FLUX_RUSANOV) ? R(0.5) * fmax(lam_m, lam_p) : R(0);
-        const R hl = R(0.5) * lift, pl = hmw * lift;
+        const R pl = (ph.numflux == CMDG_FLUX_RUSANOV) ? (R(0.5) * lift) * max_nonneg(lam_m, lam_p) : R(0);
         R fs[NSTATE];
-#pragma unroll
-        for (int s = 0; s < NSTATE; ++s) fs[s] = hl * (Fm[s] + Fp[s]) + pl * ((qm[s] - qp[s]) + jr[s]);
+        lifted_flux<R, MIXED>(S, qm, qp, jr_rho, jr_rhoe, hsgn * lift, pl, fs);
         PL::st(s_fs, NFN, f * Nfp + fn, fs);
     }
     __syncthreads();
@@ -444,7 +441,7 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
         const R rkb_dt = KConst<R>::rkb_dt(P);
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) {
-            if (!isfinite(rhs[s])) bad = 1;
+            if (!finite_r(rhs[s])) bad = 1;
             const size_t idx = ebase + s * Np;
             if (MODE == 0) {
                 double out = P.alpha * (double)rhs[s];
