@@ -76,15 +76,6 @@ struct LinNode {
     double pL, h, c;
 };
 
-__device__ __forceinline__ void lin_normal_flux(const LinNode& a, const double n[3], double F[5]) {
-    const double un = a.q[1] * n[0] + a.q[2] * n[1] + a.q[3] * n[2];
-    F[0] = un;
-    F[1] = a.pL * n[0];
-    F[2] = a.pL * n[1];
-    F[3] = a.pL * n[2];
-    F[4] = a.h * un;
-}
-
 template <int Nq>
 __device__ __forceinline__ void lin_load(const LinParams& P, int64_t e, int node, LinNode& a) {
     constexpr int Np = Nq * Nq * Nq;
@@ -99,25 +90,41 @@ __device__ __forceinline__ void lin_load(const LinParams& P, int64_t e, int node
     a.c = L[LT_C * Np + node];
 }
 
-// Rusanov flux of the linear model across one face node; qP from the facing
-// node, or the FreeSlip reflection of qM on a wall (aux+ = aux-).
-__device__ __forceinline__ void lin_face(const LinNode& M, const LinNode* P, const double n[3], double fl[5]) {
-    LinNode W;
-    if (P == nullptr) {
-        W = M;
-        const double dn = M.q[1] * n[0] + M.q[2] * n[1] + M.q[3] * n[2];
+// Lifted Rusanov flux of the linear model across one face node,
+// fl = lift ((F- + F+) . n / 2 + max(c-, c+) (q- - q+) / 2); qP from the
+// facing node, or the FreeSlip reflection of qM on a wall (aux+ = aux-).
+__device__ __forceinline__ void lin_face(const LinNode& M, const LinNode& Pn, bool wall, const double n[3],
+                                         double lift, double fl[5]) {
+    const double unm = M.q[1] * n[0] + M.q[2] * n[1] + M.q[3] * n[2];
+    double qp[5], pP = M.pL, hP = M.h, cP = M.c;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) W.q[1 + c] = M.q[1 + c] - 2 * dn * n[c];
-        P = &W;
+    for (int s = 0; s < 5; ++s) qp[s] = M.q[s];
+    if (wall) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) qp[1 + c] = fma(-2 * unm, n[c], M.q[1 + c]);
+    } else {
+#pragma unroll
+        for (int s = 0; s < 5; ++s) qp[s] = Pn.q[s];
+        pP = Pn.pL;
+        hP = Pn.h;
+        cP = Pn.c;
     }
-    double FM[5], FP[5];
-    lin_normal_flux(M, n, FM);
-    lin_normal_flux(*P, n, FP);
-    const double mw = fmax(M.c, P->c);
+    const double unp = qp[1] * n[0] + qp[2] * n[1] + qp[3] * n[2];
+    const double hl = 0.5 * lift;
+    // reference sound speeds: positive, ordered as their bits
+    const double pl = hl * (__double_as_longlong(M.c) > __double_as_longlong(cP) ? M.c : cP);
+    const double hp = hl * (M.pL + pP);
+    fl[0] = fma(pl, M.q[0] - qp[0], hl * (unm + unp));
 #pragma unroll
-    for (int s = 0; s < 5; ++s) fl[s] = (FM[s] + FP[s]) * 0.5 + mw * (M.q[s] - P->q[s]) * 0.5;
+    for (int c = 0; c < 3; ++c) fl[1 + c] = fma(pl, M.q[1 + c] - qp[1 + c], hp * n[c]);
+    fl[4] = fma(pl, M.q[4] - qp[4], hl * fma(M.h, unm, hP * unp));
 }
 
+// One thread per (element, i, j) node line.  The FP64 pipe bounds it (1/72 of
+// the FP32 rate): the energy flux is h_ref times the mass flux, 1/M and alpha
+// multiply the finished contraction, and a face's lift goes into its two
+// weights: 67 operations per node, 94 us on 648,000 nodes against 102 us with
+// 80 (that pipe is 81% busy).
 template <int Nq>
 __global__ void __launch_bounds__(128) linear_tendency_kernel(const LinParams P) {
     constexpr int Nfp = Nq * Nq, Np = Nfp * Nq;
@@ -126,7 +133,9 @@ __global__ void __launch_bounds__(128) linear_tendency_kernel(const LinParams P)
     const int ij = (int)(tid % Nfp);
     if (e >= P.nelem) return;
     const double* L = P.lt + (size_t)e * LT_NFIELDS * Np;
+    const int ez = (int)(e % P.nz);
     double F3[Nq][5], rho[Nq];
+    double flb[5], flt[5];  // lifted face fluxes of the bottom (k = 0) and top (k = Nq - 1) nodes of the line
 #pragma unroll
     for (int k = 0; k < Nq; ++k) {
         const int node = ij + Nfp * k;
@@ -138,45 +147,39 @@ __global__ void __launch_bounds__(128) linear_tendency_kernel(const LinParams P)
         F3[k][1] = m0 * a.pL;
         F3[k][2] = m1 * a.pL;
         F3[k][3] = m2 * a.pL;
-        F3[k][4] = m0 * (a.h * a.q[1]) + m1 * (a.h * a.q[2]) + m2 * (a.h * a.q[3]);
+        F3[k][4] = a.h * F3[k][0];
         rho[k] = a.q[0];
-    }
-    // face fluxes of the bottom (k = 0) and top (k = Nq - 1) nodes of the line
-    double flb[5], flt[5];
-    const int ez = (int)(e % P.nz);
-#pragma unroll
-    for (int side = 0; side < 2; ++side) {
-        const int k = side ? Nq - 1 : 0;
-        const double* F = P.lf + ((size_t)e * 2 + side) * LF_NFIELDS * Nfp;
-        const double n[3] = {F[ij], F[Nfp + ij], F[2 * Nfp + ij]};
-        LinNode M, Pn;
-        lin_load<Nq>(P, e, ij + Nfp * k, M);
-        const bool wall = side ? (ez == P.nz - 1) : (ez == 0);
-        if (!wall) lin_load<Nq>(P, side ? e + 1 : e - 1, ij + Nfp * (Nq - 1 - k), Pn);
-        lin_face(M, wall ? nullptr : &Pn, n, side ? flt : flb);
+        if (k == 0 || k == Nq - 1) {
+            const int side = k ? 1 : 0;
+            const double* F = P.lf + ((size_t)e * 2 + side) * LF_NFIELDS * Nfp;
+            const double n[3] = {F[ij], F[Nfp + ij], F[2 * Nfp + ij]};
+            LinNode Pn;
+            const bool wall = side ? (ez == P.nz - 1) : (ez == 0);
+            if (!wall) lin_load<Nq>(P, side ? e + 1 : e - 1, ij + Nfp * (Nq - 1 - k), Pn);
+            lin_face(a, Pn, wall, n, F[3 * Nfp + ij], side ? flt : flb);
+        }
     }
     double* Te = P.T + (size_t)e * 5 * Np;
+    const bool unit_beta = __double_as_longlong(P.beta) == __double_as_longlong(1.0);
+    const bool zero_beta = __double_as_longlong(P.beta) << 1 == 0;
 #pragma unroll
     for (int k = 0; k < Nq; ++k) {
         const int node = ij + Nfp * k;
-        const double MI = L[LT_MI * Np + node];
-        double lv[5];
+        const double aMI = P.alpha * L[LT_MI * Np + node], arho = P.alpha * rho[k];
 #pragma unroll
         for (int s = 0; s < 5; ++s) {
-            double acc = 0;
+            double acc = P.D[k] * F3[0][s];
 #pragma unroll
-            for (int kk = 0; kk < Nq; ++kk) acc += MI * P.D[kk * Nq + k] * F3[kk][s];
-            lv[s] = acc;
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) lv[1 + c] += -rho[k] * L[(LT_G0 + c) * Np + node];
-        const double* F = P.lf + ((size_t)e * 2 + (k == 0 ? 0 : 1)) * LF_NFIELDS * Nfp;
-        const double lift = F[3 * Nfp + ij];
-#pragma unroll
-        for (int s = 0; s < 5; ++s) {
-            double v = (P.beta != 0) ? P.alpha * lv[s] + P.beta * Te[s * Np + node] : P.alpha * lv[s];
-            if (k == 0) v -= P.alpha * lift * flb[s];
-            if (k == Nq - 1) v -= P.alpha * lift * flt[s];
+            for (int kk = 1; kk < Nq; ++kk) acc = fma(P.D[kk * Nq + k], F3[kk][s], acc);
+            double v = 0.0;
+            if (!zero_beta) {
+                v = Te[s * Np + node];
+                if (!unit_beta) v *= P.beta;
+            }
+            v = fma(aMI, acc, v);
+            if (s >= 1 && s <= 3) v = fma(-arho, L[(LT_G0 + s - 1) * Np + node], v);
+            if (k == 0) v = fma(-P.alpha, flb[s], v);
+            if (k == Nq - 1) v = fma(-P.alpha, flt[s], v);
             Te[s * Np + node] = v;
         }
     }
@@ -257,18 +260,20 @@ __global__ void band_lu_kernel(double* AB, LineMap lm, int bw, unsigned* err) {
 
 // Structure of the factors.  The vertical operator couples the unknowns of
 // one element densely and neighbouring elements only through their facing
-// nodes: the bottom layer (k = 0, 5 unknowns, block positions 0..4) of
-// element v + 1 and the top layer of element v.  With block size
-// NB = 5 (N + 1) = bw + 1, the LU factors of a column at block position p
-// then have their non-zero band entries in contiguous runs:
-//   L(j + i, j), i = 1 .. fwd_len(p) = bw - max(0, p - 5)
-//   U(j - i, j), i = 1 .. bwd_len(p) = p < 5 ? bw : p
-// (the sub-diagonal block A(v+1, v) U(v, v)^-1 has rows only in the bottom
-// layer of v + 1; the super-diagonal block L(v, v)^-1 A(v, v+1) columns only
-// there).  Every other band entry is an exact zero, which
-// band_pattern_kernel verifies after the factorization.
-__host__ __device__ constexpr int fwd_len(int p, int bw) { return bw - (p > 5 ? p - 5 : 0); }
-__host__ __device__ constexpr int bwd_len(int p, int bw) { return p < 5 ? bw : p; }
+// nodes: A(v+1, v) has entries in the rows of the bottom layer of element
+// v + 1 (k = 0, 5 unknowns, block positions 0..4) and the columns of the top
+// layer of element v (positions NB - 5 .. NB - 1, block size NB = 5 (N + 1) =
+// bw + 1), and A(v, v+1) the transposed pattern.  The elimination keeps both
+// patterns: a row that is zero left of the top layer's columns stays zero
+// there when it is divided by the upper triangle U(v, v), and the same for
+// the columns of the super-diagonal block and L(v, v).  At block position p
+// the non-zero band entries are then contiguous runs:
+//   L(j + i, j), i = 1 .. fwd_len(p) = bw - p, five more in the top layer
+//   U(j - i, j), i = 1 .. bwd_len(p) = p, five more in the bottom layer
+// Every other band entry is an exact zero, which band_pattern_kernel verifies
+// after the factorization.
+__host__ __device__ constexpr int fwd_len(int p, int bw) { return bw - p + (p > bw - 5 ? 5 : 0); }
+__host__ __device__ constexpr int bwd_len(int p, int bw) { return p + (p < 5 ? 5 : 0); }
 
 // checks the zero pattern and turns the pivots into their reciprocals (the
 // back substitution multiplies)
@@ -289,8 +294,8 @@ __global__ void band_pattern_kernel(double* AB, LineMap lm, int bw, unsigned* er
 
 // SingleColumnLU: every line's factors must equal the first line's to
 // rounding (entries within 1e-10 of the larger of the entry and the pivot
-// row's scale); copies the first line's factors out
-__global__ void band_single_kernel(const double* AB, double* AB1, LineMap lm, int bw, unsigned* err) {
+// row's scale)
+__global__ void band_single_kernel(const double* AB, LineMap lm, int bw, unsigned* err) {
     const int64_t line = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (line >= lm.nline) return;
     const int nb = 2 * bw + 1;
@@ -301,92 +306,167 @@ __global__ void band_single_kernel(const double* AB, double* AB1, LineMap lm, in
             const double v = AB[i0 + line], v0 = AB[i0];
             const double scale = fabs(v0) + fabs(1.0 / AB[((size_t)bw * lm.n + col) * lm.nline]);
             bad |= !(fabs(v - v0) <= 1e-10 * scale);
-            if (line == 0) AB1[(size_t)b * lm.n + col] = v0;
         }
     if (bad) atomicOr(err, 8u);
+}
+
+// The factors as the substitution reads them: only the structurally non-zero
+// entries, per group of L lines and element level v the forward entries of
+// the NB columns (distance 1, 2, ... below the pivot), then the backward ones
+// (reciprocal pivot, then distance 1, 2, ... above it), each entry L lines
+// wide: a warp's loads are whole 256-byte rows at compile-time offsets from
+// one pointer per level.  L = 32 (a warp), or 1 when one factorization serves
+// every line (SingleColumnLU).
+template <int Nq>
+struct PackedLU {
+    static constexpr int NB = 5 * Nq, BW = NB - 1;
+    __host__ __device__ static constexpr int fwd_off(int p) {
+        int o = 0;
+        for (int q = 0; q < p; ++q) o += fwd_len(q, BW);
+        return o;
+    }
+    __host__ __device__ static constexpr int bwd_off(int p) {
+        int o = fwd_off(NB);
+        for (int q = 0; q < p; ++q) o += 1 + bwd_len(q, BW);
+        return o;
+    }
+    static constexpr int PER = bwd_off(NB);  // entries of a line and level
+};
+
+// band storage into PackedLU, one thread per (line, column)
+template <int Nq>
+__global__ void band_pack_kernel(double* AB, double* F, LineMap lm, int L, int64_t nlines) {
+    using PK = PackedLU<Nq>;
+    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (tid >= nlines * lm.n) return;
+    const int64_t line = tid % nlines;
+    const int col = (int)(tid / nlines), v = col / PK::NB, p = col % PK::NB;
+    double* dst = F + ((size_t)(line / L) * lm.nz + v) * PK::PER * L + line % L;
+    for (int i = 1; i <= fwd_len(p, PK::BW); ++i)
+        dst[(size_t)(PK::fwd_off(p) + i - 1) * L] = col + i < lm.n ? band_at(AB, lm, PK::BW, line, col + i, col) : 0.0;
+    for (int i = 0; i <= bwd_len(p, PK::BW); ++i)
+        dst[(size_t)(PK::bwd_off(p) + i) * L] = col >= i ? band_at(AB, lm, PK::BW, line, col - i, col) : 0.0;
 }
 
 // one warp per CTA: the column count is small (a few warps per SM), so the
 // grid is spread evenly over the SMs
 constexpr int SOLVE_THREADS = 32;
 
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-
 // columns ahead whose factor entries are prefetched into L2
-constexpr int SOLVE_PREFETCH = 3;
+#ifndef CMDG_SOLVE_PREFETCH
+#define CMDG_SOLVE_PREFETCH 6
+#endif
+constexpr int SOLVE_PREFETCH = CMDG_SOLVE_PREFETCH;
 
 // band_forward! then band_back! (Golub & Van Loan Alg. 4.3.2, 4.3.3), one
-// thread per line (all lanes do useful FP64 work), the factors read
-// coalesced across neighbouring lines.  The window of bw + 1 right-hand-side
-// values (the reference's l_b) is a register ring: row r lives in slot
-// r mod NB, and the loop over the NB positions of an element block is
-// unrolled, so every slot index and every run length is a compile-time
-// constant and only the structurally non-zero band entries are touched.
-// The factor entries SOLVE_PREFETCH columns ahead are prefetched into L2 (a
-// column count of a few warps per SM leaves nothing else to hide the DRAM
-// latency).  y is a state-sized scratch; out may alias b; accumulate adds
-// x to out.
-template <int Nq>
-__global__ void __launch_bounds__(SOLVE_THREADS) band_solve_kernel(const double* __restrict__ AB, const double* b,
-                                                                   double* __restrict__ y, double* out, LineMap lm,
-                                                                   int accumulate, int single) {
-    constexpr int NB = 5 * Nq, BW = NB - 1;
-    const int64_t line = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// thread per line (all lanes do useful FP64 work).  The window of bw + 1
+// right-hand-side values (the reference's l_b) is a register ring: row r
+// lives in slot r mod NB, and the loop over the NB positions of an element
+// block is unrolled, so every slot index, run length and factor offset is a
+// compile-time constant and only the non-zero entries are touched.
+//
+// The lines are few (4.4 warps per SM on the 21,600-line acoustic-wave
+// mesh), so no other warp hides a thread's loads: the entries of the next
+// column are loaded into registers while the current column's updates run,
+// and one bulk prefetch per column brings those SOLVE_PREFETCH columns ahead
+// into L2 (6 ahead; without it the acoustic-wave step took 1.129 against
+// 1.101 ms, 12 ahead 1.111 ms).  Bound by the FP64 pipe, 70% busy: 4,900
+// operations per line at 16 cycles per warp, and an SM has 4 or 5 warps.
+// Measured on that mesh: 0.251 ms per solve, against 0.474 ms when the
+// factors were read from the band storage through computed addresses with a
+// quarter more entries.  y is scratch, (n, 32) per warp; out may alias b;
+// accumulate adds x to out.
+template <int Nq, int L>
+__global__ void __launch_bounds__(SOLVE_THREADS) band_solve_kernel(const double* __restrict__ F, const double* b,
+                                                                   double* y, double* out, LineMap lm,
+                                                                   int accumulate) {
+    static_assert(L == 1 || L == SOLVE_THREADS, "a warp reads one group of lines, or the same line");
+    using PK = PackedLU<Nq>;
+    constexpr int NB = PK::NB, BW = PK::BW, Nfp = Nq * Nq, Np = Nfp * Nq;
+    constexpr size_t FV = (size_t)PK::PER * L, QV = (size_t)5 * Np, YV = (size_t)NB * SOLVE_THREADS;
+    const int64_t line = (int64_t)blockIdx.x * SOLVE_THREADS + threadIdx.x;
     if (line >= lm.nline) return;
-    const int n = lm.n, nz = lm.nz;
-    // column and band-row strides: one factorization per line, or the
-    // first line's for all (SingleColumnLU)
-    const size_t NL = single ? 1 : (size_t)lm.nline, RS = (size_t)n * NL;
-    const double* A = single ? AB : AB + line;
-    double w[NB];
+    const int nz = lm.nz;
+    const double* Fv = F + (L == 1 ? 0 : (size_t)blockIdx.x * nz * FV + threadIdx.x);  // level v of this line
+    const size_t q0 = (size_t)(line / Nfp) * nz * QV + (size_t)(line % Nfp);           // state of level 0
+    double* yv = y + (size_t)blockIdx.x * nz * YV + threadIdx.x;
+    // row p of a level in the state
+    auto row = [](int p) { return (size_t)((p % 5) * Np + (p / 5) * Nfp); };
+    auto prefetch = [&](const double* a, int off, int len) {
+        if (L > 1 && threadIdx.x == 0)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a + (size_t)off * L), "r"(len * L * 8));
+    };
+    double w[NB], cur[NB], nxt[NB];  // entry i of a column: distance i from its pivot
+    const double* bv = b + q0;
 #pragma unroll
-    for (int i = 0; i < NB; ++i) w[i] = b[line_index<Nq>(lm, line, i)];
-    for (int d = 0; d < SOLVE_PREFETCH && d < n; ++d)
-        for (int i = 1; i <= BW; ++i) prefetch_l2(A + (size_t)(BW + i) * RS + (size_t)d * NL);
+    for (int i = 0; i < NB; ++i) w[i] = bv[row(i)];
+#pragma unroll
+    for (int i = 1; i <= fwd_len(0, BW); ++i) cur[i] = Fv[(PK::fwd_off(0) + i - 1) * L];
     for (int v = 0; v < nz; ++v) {
+        const bool more = v + 1 < nz;
 #pragma unroll
         for (int p = 0; p < NB; ++p) {
-            const int jj = v * NB + p;
-            if (jj + SOLVE_PREFETCH < n) {
-                const double* Ap = A + (size_t)(jj + SOLVE_PREFETCH) * NL;
+            constexpr int AH = SOLVE_PREFETCH;
+            if (p + AH < NB) prefetch(Fv, PK::fwd_off(p + AH), fwd_len(p + AH, BW));
+            else if (more) prefetch(Fv + FV, PK::fwd_off(p + AH - NB), fwd_len(p + AH - NB, BW));
+            if (p + 1 < NB || more) {
+                const double* Fn = p + 1 < NB ? Fv : Fv + FV;
+                const int pn = (p + 1) % NB;
 #pragma unroll
                 for (int i = 1; i <= BW; ++i)
-                    if (i <= fwd_len((p + SOLVE_PREFETCH) % NB, BW)) prefetch_l2(Ap + (size_t)(BW + i) * RS);
+                    if (i <= fwd_len(pn, BW)) nxt[i] = Fn[(PK::fwd_off(pn) + i - 1) * L];
             }
-            const double* Aj = A + (size_t)jj * NL;
             const double w0 = w[p];
 #pragma unroll
             for (int i = 1; i <= BW; ++i)
-                if (i <= fwd_len(p, BW)) w[(p + i) % NB] -= Aj[(size_t)(BW + i) * RS] * w0;
-            y[line_index<Nq>(lm, line, jj)] = w0;
-            w[p] = (jj + NB < n) ? b[line_index<Nq>(lm, line, jj + NB)] : 0.0;
-        }
-    }
+                if (i <= fwd_len(p, BW)) w[(p + i) % NB] -= cur[i] * w0;
+            yv[p * SOLVE_THREADS] = w0;
+            w[p] = more ? bv[QV + row(p)] : 0.0;
 #pragma unroll
-    for (int i = 0; i < NB; ++i) w[BW - i] = y[line_index<Nq>(lm, line, n - 1 - i)];
-    for (int d = 0; d < SOLVE_PREFETCH && d < n; ++d)
-        for (int i = 0; i <= BW; ++i) prefetch_l2(A + (size_t)(BW - i) * RS + (size_t)(n - 1 - d) * NL);
+            for (int i = 0; i < NB; ++i) cur[i] = nxt[i];
+        }
+        Fv += FV;
+        yv += YV;
+        bv += QV;
+    }
+    // the last level again, downwards
+    Fv -= FV;
+    yv -= YV;
+    double* ov = out + q0 + (size_t)(nz - 1) * QV;
+#pragma unroll
+    for (int i = 0; i < NB; ++i) w[i] = yv[i * SOLVE_THREADS];
+#pragma unroll
+    for (int i = 0; i <= bwd_len(BW, BW); ++i) cur[i] = Fv[(PK::bwd_off(BW) + i) * L];
+    double add = accumulate ? ov[row(BW)] : 0.0;  // of the current row
     for (int v = nz - 1; v >= 0; --v) {
+        const bool more = v > 0;
 #pragma unroll
         for (int p = NB - 1; p >= 0; --p) {
-            const int jj = v * NB + p;
-            if (jj - SOLVE_PREFETCH >= 0) {
-                const double* Ap = A + (size_t)(jj - SOLVE_PREFETCH) * NL;
+            constexpr int AH = SOLVE_PREFETCH;
+            if (p >= AH) prefetch(Fv, PK::bwd_off(p - AH), 1 + bwd_len(p - AH, BW));
+            else if (more) prefetch(Fv - FV, PK::bwd_off(p - AH + NB), 1 + bwd_len(p - AH + NB, BW));
+            double add_nxt = 0.0;
+            if (p > 0 || more) {
+                const double* Fn = p > 0 ? Fv : Fv - FV;
+                const int pn = (p + NB - 1) % NB;
 #pragma unroll
                 for (int i = 0; i <= BW; ++i)
-                    if (i <= bwd_len((p + NB - SOLVE_PREFETCH) % NB, BW)) prefetch_l2(Ap + (size_t)(BW - i) * RS);
+                    if (i <= bwd_len(pn, BW)) nxt[i] = Fn[(PK::bwd_off(pn) + i) * L];
+                if (accumulate) add_nxt = p > 0 ? ov[row(pn)] : *(ov + row(pn) - QV);
             }
-            const double* Aj = A + (size_t)jj * NL;
-            const double x = w[p] * Aj[(size_t)BW * RS];  // reciprocal pivot
+            const double x = w[p] * cur[0];  // reciprocal pivot
 #pragma unroll
             for (int i = 1; i <= BW; ++i)
-                if (i <= bwd_len(p, BW)) w[(p - i + NB) % NB] -= Aj[(size_t)(BW - i) * RS] * x;
-            const size_t o = line_index<Nq>(lm, line, jj);
-            out[o] = accumulate ? out[o] + x : x;
-            w[p] = (jj - NB >= 0) ? y[line_index<Nq>(lm, line, jj - NB)] : 0.0;
+                if (i <= bwd_len(p, BW)) w[(p - i + NB) % NB] -= cur[i] * x;
+            ov[row(p)] = accumulate ? add + x : x;
+            add = add_nxt;
+            w[p] = more ? *(yv + p * SOLVE_THREADS - YV) : 0.0;
+#pragma unroll
+            for (int i = 0; i < NB; ++i) cur[i] = nxt[i];
         }
+        Fv -= FV;
+        yv -= YV;
+        ov -= QV;
     }
 }
 
@@ -618,9 +698,10 @@ struct Hevi {
     LineMap lm{};
     int bw = 0;
     size_t len = 0;
-    double* d_AB = nullptr;   // band matrix, then its LU factors (reciprocal pivots), line-fastest
-    int single = 0;           // SingleColumnLU: d_AB1 holds the first line's factors, (2 bw + 1, n)
-    double* d_AB1 = nullptr;
+    double* d_AB = nullptr;   // set-up: band matrix, then its LU factors (reciprocal pivots), line-fastest
+    int single = 0;           // SingleColumnLU: d_F holds the first line's factors
+    double* d_F = nullptr;    // the factors as the substitution reads them (PackedLU)
+    double* d_y = nullptr;    // the substitution's scratch, (n, 32) per warp of lines
     double* d_buf = nullptr;  // S1, S2, R0, R1, R2, Qhat, Y
     float* d_Sp = nullptr;    // mixed models: FP32 perturbation of the stage state
     int rem = 0;              // mixed cubed shell: explicit part from the fused remainder f - l
@@ -658,10 +739,22 @@ int hevi_assemble_N(Hevi* h, cudaStream_t s) {
     band_pattern_kernel<<<(unsigned)((h->lm.nline + 127) / 128), 128, 0, s>>>(h->d_AB, h->lm, h->bw, h->d_err);
     CMDG_CUDA_CHECK(cudaGetLastError());
     if (h->single) {
-        band_single_kernel<<<(unsigned)((h->lm.nline + 127) / 128), 128, 0, s>>>(h->d_AB, h->d_AB1, h->lm, h->bw,
-                                                                                h->d_err);
+        band_single_kernel<<<(unsigned)((h->lm.nline + 127) / 128), 128, 0, s>>>(h->d_AB, h->lm, h->bw, h->d_err);
         CMDG_CUDA_CHECK(cudaGetLastError());
     }
+    // the factors in the substitution's layout
+    const int L = h->single ? 1 : SOLVE_THREADS;
+    const int64_t nlines = h->single ? 1 : h->lm.nline, groups = (nlines + L - 1) / L;
+    const size_t entries = (size_t)groups * h->lm.nz * PackedLU<Nq>::PER * L;
+    const int64_t warps = (h->lm.nline + SOLVE_THREADS - 1) / SOLVE_THREADS;
+    if (cudaMalloc(&h->d_F, sizeof(double) * entries) != cudaSuccess ||
+        cudaMalloc(&h->d_y, sizeof(double) * (size_t)warps * SOLVE_THREADS * h->lm.n) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("allocation of the column factors (%zu bytes) failed", sizeof(double) * entries);
+        return CMDG_ERR_ALLOC;
+    }
+    band_pack_kernel<Nq><<<(unsigned)((nlines * h->lm.n + 127) / 128), 128, 0, s>>>(h->d_AB, h->d_F, h->lm, L, nlines);
+    CMDG_CUDA_CHECK(cudaGetLastError());
     return CMDG_OK;
 }
 
@@ -677,8 +770,10 @@ int hevi_assemble(Hevi* h, cudaStream_t s) {
 template <int Nq>
 int hevi_solve_N(Hevi* h, const double* b, double* out, int accumulate, cudaStream_t s) {
     const unsigned grid = (unsigned)((h->lm.nline + SOLVE_THREADS - 1) / SOLVE_THREADS);
-    band_solve_kernel<Nq><<<grid, SOLVE_THREADS, 0, s>>>(h->single ? h->d_AB1 : h->d_AB, b, h->Y(), out, h->lm,
-                                                         accumulate, h->single);
+    if (h->single)
+        band_solve_kernel<Nq, 1><<<grid, SOLVE_THREADS, 0, s>>>(h->d_F, b, h->d_y, out, h->lm, accumulate);
+    else
+        band_solve_kernel<Nq, SOLVE_THREADS><<<grid, SOLVE_THREADS, 0, s>>>(h->d_F, b, h->d_y, out, h->lm, accumulate);
     CMDG_CUDA_CHECK(cudaGetLastError());
     return CMDG_OK;
 }
@@ -842,8 +937,7 @@ int cmdg_hevi_create(cmdg_model* model, double dt, int split_explicit_implicit, 
     cudaError_t e2 = cudaMalloc(&h->d_buf, sizeof(double) * 7 * h->len);
     cudaError_t e3 = cudaMalloc(&h->d_err, sizeof(unsigned));
     cudaError_t e4 = md->precision == CMDG_MIXED ? cudaMalloc(&h->d_Sp, sizeof(float) * h->len) : cudaSuccess;
-    cudaError_t e5 = h->single ? cudaMalloc(&h->d_AB1, sizeof(double) * (2 * h->bw + 1) * h->lm.n) : cudaSuccess;
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess || e5 != cudaSuccess) {
+    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess) {
         cudaGetLastError();
         cmdg_hevi_destroy(ho);
         set_error("HEVI: device allocation of %zu bytes failed", sizeof(double) * (ab + 7 * h->len));
@@ -897,10 +991,8 @@ int cmdg_hevi_create(cmdg_model* model, double dt, int split_explicit_implicit, 
         cmdg_hevi_destroy(ho);
         return rc;
     }
-    if (h->single) {  // only the first line's factors are kept
-        cudaFree(h->d_AB);
-        h->d_AB = nullptr;
-    }
+    cudaFree(h->d_AB);  // d_F holds what the substitution reads
+    h->d_AB = nullptr;
     *out = ho;
     return CMDG_OK;
 }
@@ -908,7 +1000,8 @@ int cmdg_hevi_create(cmdg_model* model, double dt, int split_explicit_implicit, 
 int cmdg_hevi_destroy(cmdg_hevi* hevi) {
     if (!hevi) return CMDG_OK;
     cudaFree(hevi->h.d_AB);
-    cudaFree(hevi->h.d_AB1);
+    cudaFree(hevi->h.d_F);
+    cudaFree(hevi->h.d_y);
     cudaFree(hevi->h.d_buf);
     cudaFree(hevi->h.d_Sp);
     cudaFree(hevi->h.d_lref);
