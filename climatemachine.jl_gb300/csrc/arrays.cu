@@ -91,6 +91,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     // ---------------- phase 1: node thermodynamics, contravariant fluxes, gravity
     R q[NSTATE], src[3] = {0, 0, 0}, invJ = 0;
     double dq_old[NSTATE];
+    chain_wait();
     if (node_thread) {
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) q[s] = Qin[ebase + s * Np];
@@ -241,6 +242,8 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     }
     __syncthreads();
 
+    chain_release();
+
     // ---------------- phase 3: volume contraction, face terms, source, update
     int bad = 0;
     if (node_thread) {
@@ -315,8 +318,7 @@ cudaError_t launch_arrays_typed(const KParams& P, cudaStream_t s) {
     constexpr size_t bytes = ArraysSmem<N, R>::BYTES;
     cudaError_t e = opt_in_smem(arrays_stage_kernel<N, R, MIXED, MODE, VT>, bytes);
     if (e != cudaSuccess) return e;
-    arrays_stage_kernel<N, R, MIXED, MODE, VT><<<(unsigned)P.nelem, ShellDims<N>::NT, bytes, s>>>(P);
-    return cudaGetLastError();
+    return launch_chained(s, arrays_stage_kernel<N, R, MIXED, MODE, VT>, (unsigned)P.nelem, ShellDims<N>::NT, bytes, P);
 }
 
 // closures run FP64 on grid-arrays meshes (cmdg_model_create)

@@ -5,6 +5,7 @@
 #pragma once
 
 #include "cmdg_internal.h"
+#include "launch.cuh"
 
 namespace cmdg {
 

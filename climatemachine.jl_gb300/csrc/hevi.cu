@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "cmdg_internal.h"
+#include "launch.cuh"
 
 namespace cmdg {
 
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(128) linear_tendency_kernel(const LinParams P)
     if (e >= P.nelem) return;
     const double* L = P.lt + (size_t)e * LT_NFIELDS * Np;
     const int ez = (int)(e % P.nz);
+    chain_wait();
     double F3[Nq][5], rho[Nq];
     double flb[5], flt[5];  // lifted face fluxes of the bottom (k = 0) and top (k = Nq - 1) nodes of the line
 #pragma unroll
@@ -159,6 +161,7 @@ __global__ void __launch_bounds__(128) linear_tendency_kernel(const LinParams P)
             lin_face(a, Pn, wall, n, F[3 * Nfp + ij], side ? flt : flb);
         }
     }
+    chain_release();
     double* Te = P.T + (size_t)e * 5 * Np;
     const bool unit_beta = __double_as_longlong(P.beta) == __double_as_longlong(1.0);
     const bool zero_beta = __double_as_longlong(P.beta) << 1 == 0;
@@ -399,9 +402,12 @@ __global__ void __launch_bounds__(SOLVE_THREADS) band_solve_kernel(const double*
     double w[NB], cur[NB], nxt[NB];  // entry i of a column: distance i from its pivot
     const double* bv = b + q0;
 #pragma unroll
-    for (int i = 0; i < NB; ++i) w[i] = bv[row(i)];
-#pragma unroll
     for (int i = 1; i <= fwd_len(0, BW); ++i) cur[i] = Fv[(PK::fwd_off(0) + i - 1) * L];
+#pragma unroll
+    for (int p = 1; p < SOLVE_PREFETCH; ++p) prefetch(Fv, PK::fwd_off(p), fwd_len(p, BW));
+    chain_wait();
+#pragma unroll
+    for (int i = 0; i < NB; ++i) w[i] = bv[row(i)];
     for (int v = 0; v < nz; ++v) {
         const bool more = v + 1 < nz;
 #pragma unroll
@@ -478,7 +484,9 @@ struct StageCoef {
     int nprev;
 };
 
-__global__ void ark_stage_kernel(const double* __restrict__ Q, StageCoef c, double* Sis, double* Qhat, size_t len) {
+__global__ void ark_stage_kernel(const double* Q, StageCoef c, double* Sis, double* Qhat, size_t len) {
+    chain_release();
+    chain_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (size_t)gridDim.x * blockDim.x) {
         double qh = Q[i], qs = -0.0;
         for (int js = 0; js < c.nprev; ++js) {
@@ -494,6 +502,8 @@ __global__ void ark_stage_kernel(const double* __restrict__ Q, StageCoef c, doub
 // solution_update!(::LowStorageVariant) (:642-662)
 __global__ void ark_solution_kernel(double* Q, const double* R0, const double* R1, const double* R2, double b0,
                                     double b1, double b2, size_t len) {
+    chain_release();
+    chain_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (size_t)gridDim.x * blockDim.x) {
         double q = Q[i];
         q += b0 * R0[i];
@@ -666,8 +676,7 @@ int launch_linear_N(Model* md, const double* Q, double* T, double alpha, double 
     P.kv = p.R_d / p.cv_d;
     for (int i = 0; i < Nq * Nq; ++i) P.D[i] = m.D[i];
     const int64_t threads = m.nelem * (int64_t)m.Nfp;
-    linear_tendency_kernel<Nq><<<(unsigned)((threads + 127) / 128), 128, 0, s>>>(P);
-    CMDG_CUDA_CHECK(cudaGetLastError());
+    CMDG_CUDA_CHECK(launch_chained(s, linear_tendency_kernel<Nq>, (unsigned)((threads + 127) / 128), 128, 0, P));
     return CMDG_OK;
 }
 
@@ -787,7 +796,9 @@ int hevi_solve(Hevi* h, const double* b, double* out, int accumulate, cudaStream
     }
 }
 
-__global__ void axpy_kernel(double* __restrict__ y, double a, const double* __restrict__ x, size_t n) {
+__global__ void axpy_kernel(double* y, double a, const double* x, size_t n) {
+    chain_release();
+    chain_wait();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         y[i] = fma(a, x[i], y[i]);
 }
@@ -813,8 +824,7 @@ int hevi_rhs(Hevi* h, double* R, const double* Q, cudaStream_t s) {
         rc = launch_stage(h->md, a, s);
         if (rc) return rc;
         if (!h->split) return launch_linear_tendency(h->md, Qd, R, 1.0, 1.0, s);
-        axpy_kernel<<<elementwise_grid(h->len), 256, 0, s>>>(R, -1.0, h->d_lref, h->len);
-        CMDG_CUDA_CHECK(cudaGetLastError());
+        CMDG_CUDA_CHECK(launch_chained(s, axpy_kernel, elementwise_grid(h->len), 256, 0, R, -1.0, h->d_lref, h->len));
         return CMDG_OK;
     }
     if (h->md->precision == CMDG_MIXED) {
@@ -850,8 +860,8 @@ int hevi_step(Hevi* h, double* Q, cudaStream_t s) {
             c.rk[js] = h->split ? h->Ai[is][js] / h->Ai[is][is] : (h->Ai[is][js] - h->Ae[is][js]) / h->Ai[is][is];
             c.dtAe[js] = dt * h->Ae[is][js];
         }
-        ark_stage_kernel<<<elementwise_grid(h->len), 256, 0, s>>>(Q, c, h->S(is), h->Qhat(), h->len);
-        CMDG_CUDA_CHECK(cudaGetLastError());
+        CMDG_CUDA_CHECK(
+            launch_chained(s, ark_stage_kernel, elementwise_grid(h->len), 256, 0, Q, c, h->S(is), h->Qhat(), h->len));
         rc = hevi_solve(h, h->Qhat(), h->S(is), 1, s);
         if (rc) return rc;
         rc = hevi_rhs(h, h->R(is), h->S(is), s);
@@ -862,9 +872,8 @@ int hevi_step(Hevi* h, double* Q, cudaStream_t s) {
             rc = launch_linear_tendency(h->md, Sst[is], h->R(is), 1.0, 1.0, s);
             if (rc) return rc;
         }
-    ark_solution_kernel<<<elementwise_grid(h->len), 256, 0, s>>>(Q, h->R(0), h->R(1), h->R(2), h->B[0] * dt,
-                                                                  h->B[1] * dt, h->B[2] * dt, h->len);
-    CMDG_CUDA_CHECK(cudaGetLastError());
+    CMDG_CUDA_CHECK(launch_chained(s, ark_solution_kernel, elementwise_grid(h->len), 256, 0, Q, h->R(0), h->R(1), h->R(2),
+                                   h->B[0] * dt, h->B[1] * dt, h->B[2] * dt, h->len));
     return CMDG_OK;
 }
 

@@ -85,17 +85,18 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_grad_kernel(const KParams 
 
     const int e = blockIdx.x, t = threadIdx.x;
     const Ix x(t);
-    const R* __restrict__ Qin = static_cast<const R*>(Qv);
+    const R* Qin = static_cast<const R*>(Qv);
     const int* nbr = P.nbr + NBR_STRIDE * e;
     const int ez = __ldg(nbr + 6);
     if (t < Nq * Nq) s_D[t] = VConst<R>::D(P, t);
+    const int nb = x.face ? __ldg(nbr + x.f) : -1;
     R q[NSTATE], qp[NSTATE];
+    chain_wait();
     if (x.node) {
         const R* qe = Qin + (size_t)e * ESTRIDE + t;
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) q[s] = qe[s * Np];
     }
-    const int nb = x.face ? __ldg(nbr + x.f) : -1;
     int levp = ez * Nq + x.vM / Nfp;
     if (nb >= 0) {
         const R* qn = Qin + (size_t)nb * ESTRIDE + x.vP;
@@ -143,6 +144,7 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_grad_kernel(const KParams 
         for (int s = 0; s < 3; ++s) s_dH[s * NFN + t] = w * (Hp[s] - s_H[s * Np + x.vM]);
     }
     __syncthreads();
+    chain_release();
 
     if (x.node) {
         R g1[3] = {0, 0, 0}, g2[3] = {0, 0, 0}, g3[3] = {0, 0, 0};
@@ -185,8 +187,7 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_grad_kernel(const KParams 
 }
 
 template <int N, typename R>
-__global__ void __launch_bounds__(VDims<N>::NT) hyper_div_kernel(const KParams P, const R* __restrict__ hg,
-                                                                 R* __restrict__ hl) {
+__global__ void __launch_bounds__(VDims<N>::NT) hyper_div_kernel(const KParams P, const R* hg, R* hl) {
     using Ix = HypIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -198,12 +199,13 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_div_kernel(const KParams P
     const Ix x(t);
     const int* nbr = P.nbr + NBR_STRIDE * e;
     if (t < Nq * Nq) s_Dh[t] = static_cast<const R*>(P.Dhat)[t];
+    const int nb = x.face ? __ldg(nbr + x.f) : -1;
+    chain_wait();
     if (x.node) {
         const R* ge = hg + (size_t)e * 9 * Np + t;
 #pragma unroll
         for (int w = 0; w < 9; ++w) s_G[w * Np + t] = ge[w * Np];
     }
-    const int nb = x.face ? __ldg(nbr + x.f) : -1;
     R Gp[3];
     if (nb >= 0) {
         // the neighbour's gradient components normal to the face
@@ -226,6 +228,7 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_div_kernel(const KParams P
         }
     }
     __syncthreads();
+    chain_release();
 
     if (x.node) {
         R a1[3] = {0, 0, 0}, a2[3] = {0, 0, 0}, a3[3] = {0, 0, 0};
@@ -261,8 +264,7 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_div_kernel(const KParams P
 }
 
 template <int N, typename R, bool MIXED>
-__global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams P, const R* __restrict__ hl,
-                                                                  R* __restrict__ hd) {
+__global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams P, const R* hl, R* hd) {
     using Ix = HypIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -275,12 +277,13 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams 
     const int* nbr = P.nbr + NBR_STRIDE * e;
     const int ez = __ldg(nbr + 6);
     if (t < Nq * Nq) s_D[t] = VConst<R>::D(P, t);
+    const int nb = x.face ? __ldg(nbr + x.f) : -1;
+    chain_wait();
     if (x.node) {
         const R* le = hl + (size_t)e * 3 * Np + t;
 #pragma unroll
         for (int s = 0; s < 3; ++s) s_L[s * Np + t] = le[s * Np];
     }
-    const int nb = x.face ? __ldg(nbr + x.f) : -1;
     R Lp[3];
     if (nb >= 0) {
         const R* ln = hl + (size_t)nb * 3 * Np + x.vP;
@@ -304,6 +307,7 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams 
             s_dL[s * NFN + t] = nb >= 0 ? w * (Lp[s] - s_L[s * Np + x.vM]) / R(2) : R(0);
     }
     __syncthreads();
+    chain_release();
 
     if (x.node) {
         R g1[3] = {0, 0, 0}, g2[3] = {0, 0, 0}, g3[3] = {0, 0, 0};
@@ -358,10 +362,10 @@ cudaError_t launch_passes_typed(const KParams& P, const void* Q, void* hd, void*
     if ((e = opt_in(hyper_glap_kernel<N, R, MIXED>, b3)) != cudaSuccess) return e;
     R* g = static_cast<R*>(hd);
     R* l = static_cast<R*>(hl);
-    hyper_grad_kernel<N, R, MIXED><<<P.nelem, NT, b1, s>>>(P, Q, g);
-    hyper_div_kernel<N, R><<<P.nelem, NT, b2, s>>>(P, g, l);
-    hyper_glap_kernel<N, R, MIXED><<<P.nelem, NT, b3, s>>>(P, l, g);
-    return cudaGetLastError();
+    const unsigned grid = (unsigned)P.nelem;
+    if ((e = launch_chained(s, hyper_grad_kernel<N, R, MIXED>, grid, NT, b1, P, Q, g)) != cudaSuccess) return e;
+    if ((e = launch_chained(s, hyper_div_kernel<N, R>, grid, NT, b2, P, g, l)) != cudaSuccess) return e;
+    return launch_chained(s, hyper_glap_kernel<N, R, MIXED>, grid, NT, b3, P, l, g);
 }
 
 template <int N>

@@ -186,19 +186,20 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
 
     const int e = blockIdx.x, t = threadIdx.x;
     const Ix x(t);
-    const R* __restrict__ Qin = static_cast<const R*>(Qv);
+    const R* Qin = static_cast<const R*>(Qv);
     const R* __restrict__ geo = static_cast<const R*>(P.geo);
     const R* ge = geo + (size_t)e * GSTRIDE;
     const int* nbr = P.nbr + NBR_STRIDE * e;
     const int ez = __ldg(nbr + 6);
     if (t < Nq * Nq) s_D[t] = VConst<R>::D(P, t);
+    const int nb = x.face ? __ldg(nbr + x.f) : -1;
     R q[NSTATE], qp[NSTATE];
+    chain_wait();
     if (x.node) {
         const R* qe = Qin + (size_t)e * ESTRIDE + t;
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) q[s] = qe[s * Np];
     }
-    const int nb = x.face ? __ldg(nbr + x.f) : -1;
     const int vP = nb < 0 ? x.vM
                    : ARRAYS ? __ldg(P.fpart + ((size_t)e * 6 + x.f) * Nfp + x.fn)
                             : shell_partner<N>(nbr, x.f, x.fn);
@@ -254,6 +255,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
         }
     }
     __syncthreads();
+    chain_release();
 
     if (x.node) {
         R g[3 * NA];
@@ -265,8 +267,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
 }
 
 template <int N, typename R>
-__global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const KParams P, const R* __restrict__ hg,
-                                                                           R* __restrict__ hl) {
+__global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const KParams P, const R* hg, R* hl) {
     using Ix = ShellIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp, GSTRIDE = KG_NFIELDS * Np;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -281,6 +282,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
     const R* ge = geo + (size_t)e * GSTRIDE;
     const int* nbr = P.nbr + NBR_STRIDE * e;
     if (t < Nq * Nq) s_Dh[t] = static_cast<const R*>(P.Dhat)[t];
+    chain_wait();
     if (x.node) {
         const R* gn = hg + (size_t)e * 12 * Np + t;
         R G[12];
@@ -325,6 +327,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
         }
     }
     __syncthreads();
+    chain_release();
 
     if (x.node) {
         R a[4] = {0, 0, 0, 0}, av[4] = {0, 0, 0, 0};
@@ -364,8 +367,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
 }
 
 template <int N, typename R, bool MIXED>
-__global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(const KParams P, const R* __restrict__ hl,
-                                                                            R* __restrict__ hd) {
+__global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(const KParams P, const R* hl, R* hd) {
     using Ix = ShellIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp, GSTRIDE = KG_NFIELDS * Np;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -379,6 +381,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
     const R* ge = geo + (size_t)e * GSTRIDE;
     const int* nbr = P.nbr + NBR_STRIDE * e;
     if (t < Nq * Nq) s_D[t] = VConst<R>::D(P, t);
+    chain_wait();
     if (x.node) {
         const R* ln = hl + (size_t)e * 4 * Np + t;
 #pragma unroll
@@ -406,6 +409,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
         }
     }
     __syncthreads();
+    chain_release();
 
     if (x.node) {
         R g[12];
@@ -433,10 +437,10 @@ cudaError_t launch_shell_passes_typed(const KParams& P, const void* Q, void* hd,
     if ((e = opt_in(shell_hyper_glap_kernel<N, R, MIXED>, b3)) != cudaSuccess) return e;
     R* g = static_cast<R*>(hd);
     R* l = static_cast<R*>(hl);
-    shell_hyper_grad_kernel<N, R, MIXED><<<P.nelem, NT, b1, s>>>(P, Q, g);
-    shell_hyper_div_kernel<N, R><<<P.nelem, NT, b2, s>>>(P, g, l);
-    shell_hyper_glap_kernel<N, R, MIXED><<<P.nelem, NT, b3, s>>>(P, l, g);
-    return cudaGetLastError();
+    const unsigned grid = (unsigned)P.nelem;
+    if ((e = launch_chained(s, shell_hyper_grad_kernel<N, R, MIXED>, grid, NT, b1, P, Q, g)) != cudaSuccess) return e;
+    if ((e = launch_chained(s, shell_hyper_div_kernel<N, R>, grid, NT, b2, P, g, l)) != cudaSuccess) return e;
+    return launch_chained(s, shell_hyper_glap_kernel<N, R, MIXED>, grid, NT, b3, P, l, g);
 }
 
 // the viscous gradient pass: grad u, grad h_tot (Np, 12, nelem)
@@ -446,8 +450,8 @@ cudaError_t launch_shell_visc_typed(const KParams& P, const void* Q, void* gout,
     constexpr size_t b1 = sizeof(R) * (planar_pad<R>(5 * Np) + NA * Np + 3 * NA * NFN + Nq * Nq);
     cudaError_t e;
     if ((e = opt_in(shell_hyper_grad_kernel<N, R, MIXED, false, NA, ARRAYS>, b1)) != cudaSuccess) return e;
-    shell_hyper_grad_kernel<N, R, MIXED, false, NA, ARRAYS><<<P.nelem, NT, b1, s>>>(P, Q, static_cast<R*>(gout));
-    return cudaGetLastError();
+    return launch_chained(s, shell_hyper_grad_kernel<N, R, MIXED, false, NA, ARRAYS>, (unsigned)P.nelem, NT, b1, P, Q,
+                          static_cast<R*>(gout));
 }
 
 // grid-arrays meshes: grad u, grad h_tot (and grad theta_v with smag); the

@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     // ---------------- phase 1: node thermodynamics, contravariant fluxes, gravity
     R q[NSTATE], src[3] = {0, 0, 0}, invJ = 0;
     double dq_old[NSTATE];
+    chain_wait();
     if (node_thread) {
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) q[s] = Qin[ebase + s * Np];
@@ -369,6 +370,8 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     }
     __syncthreads();
 
+    chain_release();
+
     // ---------------- phase 3: volume contraction, face terms, source, update
     int bad = 0;
     if (node_thread) {
@@ -445,8 +448,7 @@ cudaError_t launch_shell_typed(const KParams& P, cudaStream_t s) {
         if (e != cudaSuccess) return e;
         configured |= 1ull << (dev & 63);
     }
-    shell_stage_kernel<N, R, MIXED, MODE, HYPER, VT, REM><<<(unsigned)P.nelem, ShellDims<N>::NT, bytes, s>>>(P);
-    return cudaGetLastError();
+    return launch_chained(s, shell_stage_kernel<N, R, MIXED, MODE, HYPER, VT, REM>, (unsigned)P.nelem, ShellDims<N>::NT, bytes, P);
 }
 
 template <int N, bool HYPER, int VT>

@@ -240,12 +240,13 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
     auto fetch = [&](int e, Ahead<R>& a) {
         const int* nbr = P.nbr + NBR_STRIDE * e;
         a.ez = __ldg(nbr + 6);
+        a.nb = face_thread ? __ldg(nbr + f) : -1;
+        chain_wait();
         if (node_thread) {
             const R* qe = Qin + (size_t)e * ESTRIDE + t;
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) a.q[s] = qe[s * Np];
         }
-        a.nb = face_thread ? __ldg(nbr + f) : -1;
         if (a.nb >= 0 && !remote) {
             const R* qn = Qin + (size_t)a.nb * ESTRIDE + vP;
 #pragma unroll
@@ -296,6 +297,7 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
     int e = e_first;
     Ahead<R> cur;
     if (PERSIST) {
+        chain_wait();
         if (t == 0) {
             mbar_init(&bars[0], 1);
             mbar_init(&bars[1], 1);
@@ -480,6 +482,8 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
         // while another may still read it
         if constexpr (CL > 0) cg::this_cluster().sync();
         else __syncthreads();
+
+        chain_release();
 
         // ---------------- phase 3: volume contraction, face terms, source, update
         int bad = 0;
@@ -670,8 +674,7 @@ cudaError_t launch_mode(const KParams& P, int grid_ctas, cudaStream_t s) {
     }
     int grid = PERSIST ? (grid_ctas > 0 ? grid_ctas : resident[dev]) : P.nelem;
     if (grid > P.nelem) grid = P.nelem;
-    stage_kernel<N, R, MIXED, MODE, PERSIST><<<(unsigned)grid, Dims<N>::NT, bytes, s>>>(P);
-    return cudaGetLastError();
+    return launch_chained(s, stage_kernel<N, R, MIXED, MODE, PERSIST>, (unsigned)grid, Dims<N>::NT, bytes, P);
 }
 
 template <int N, typename R, bool MIXED>
@@ -706,6 +709,7 @@ template <int N>
 __global__ void __launch_bounds__(Dims<N>::NT, batch_min_ctas<N>())
     batch_stage_kernel(const KParams* __restrict__ params, const BatchTile* __restrict__ tiles, int ntiles) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    chain_wait();
     for (int it = blockIdx.x; it < ntiles; it += gridDim.x) {
         const BatchTile T = tiles[it];
         stage_body<N, float, true, 1, false, false>(params[T.member], smem_raw, T.e0, 1, T.e1);
@@ -724,8 +728,7 @@ cudaError_t launch_batch_N(const KParams* d_params, const BatchTile* d_tiles, in
         if (e != cudaSuccess) return e;
         configured |= 1ull << (dev & 63);
     }
-    batch_stage_kernel<N><<<grid, Dims<N>::NT, bytes, s>>>(d_params, d_tiles, ntiles);
-    return cudaGetLastError();
+    return launch_chained(s, batch_stage_kernel<N>, (unsigned)grid, Dims<N>::NT, bytes, d_params, d_tiles, ntiles);
 }
 
 template <int N>

@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
     if (threadIdx.x < Nq * Nq) s_D[threadIdx.x] = VConst<R>::D(P, threadIdx.x);
 
     const int e = blockIdx.x, t = threadIdx.x;
-    const R* __restrict__ Qin = static_cast<const R*>(Qv);
+    const R* Qin = static_cast<const R*>(Qv);
     const bool node_thread = t < Np, face_thread = t < 6 * Nfp;
     const int* nbr = P.nbr + NBR_STRIDE * e;
     const int ez = __ldg(nbr + 6);
@@ -78,13 +78,14 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
     const int vM = fd == 0 ? fside * N + Nq * fn : (fd == 1 ? fa + Nq * (fside * N + Nq * fb) : fn + Nfp * (fside * N));
     const int vP = fd == 0 ? oside * N + Nq * fn : (fd == 1 ? fa + Nq * (oside * N + Nq * fb) : fn + Nfp * (oside * N));
 
+    const int nb = face_thread ? __ldg(nbr + f) : -1;
     R q[NSTATE], qp[NSTATE];
+    chain_wait();
     if (node_thread) {
         const R* qe = Qin + (size_t)e * ESTRIDE + t;
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) q[s] = qe[s * Np];
     }
-    const int nb = face_thread ? __ldg(nbr + f) : -1;
     int levp = ez * Nq + vM / Nfp;
     if (nb >= 0) {
         const R* qn = Qin + (size_t)nb * ESTRIDE + vP;
@@ -135,6 +136,8 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
         PL::st(s_dG, NFN, f * Nfp + fn, out);
     }
     __syncthreads();
+
+    chain_release();
 
     // phase 3: volume gradient (strong form), face terms, reference part, transform
     if (node_thread) {
@@ -226,8 +229,7 @@ cudaError_t launch_grad_kernel(const KParams& P, const void* Q, void* gf, cudaSt
     auto k = gradient_kernel<N, R, MIXED, SMAG, FLUX>;
     cudaError_t e;
     if ((e = opt_in(k, bytes)) != cudaSuccess) return e;
-    k<<<P.nelem, VDims<N>::NT, bytes, s>>>(P, Q, static_cast<R*>(gf));
-    return cudaGetLastError();
+    return launch_chained(s, k, (unsigned)P.nelem, VDims<N>::NT, bytes, P, Q, static_cast<R*>(gf));
 }
 
 template <int N, typename R, bool MIXED>

@@ -275,6 +275,8 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
     const size_t ebase = (size_t)e * ESTRIDE + t;
     R q[NSTATE], f2[NF2], hd[9];
     double dq_old[NSTATE];
+    const int nb = face_thread ? __ldg(nbr + f) : -1;
+    chain_wait();
     if (node_thread) {
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) q[s] = Qin[ebase + s * Np];
@@ -293,7 +295,6 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
             for (int s = 0; s < NSTATE; ++s) dq_old[s] = P.dQ[ebase + s * Np];
         }
     }
-    const int nb = face_thread ? __ldg(nbr + f) : -1;
     R qp[NSTATE], f2p[4], hdp[3];
     int ezp = ez;
     if (nb >= 0) {
@@ -403,6 +404,8 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
     }
     __syncthreads();
 
+    chain_release();
+
     // phase 3: volume contraction, face terms, source, update
     int bad = 0;
     if (node_thread) {
@@ -486,21 +489,21 @@ cudaError_t launch_vstage_typed(const KParams& P, int turb, cudaStream_t s) {
     if (turb == CMDG_TURB_SMAGORINSKY) {
         auto k = viscous_stage_kernel<N, R, MIXED, MODE, CMDG_TURB_SMAGORINSKY, HYPER>;
         if ((e = opt_in(k, bytes)) != cudaSuccess) return e;
-        k<<<P.nelem, VDims<N>::NT, bytes, s>>>(P);
+        e = launch_chained(s, k, (unsigned)P.nelem, VDims<N>::NT, bytes, P);
     } else if (turb == CMDG_TURB_CONSTANT) {
         auto k = viscous_stage_kernel<N, R, MIXED, MODE, CMDG_TURB_CONSTANT, HYPER>;
         if ((e = opt_in(k, bytes)) != cudaSuccess) return e;
-        k<<<P.nelem, VDims<N>::NT, bytes, s>>>(P);
+        e = launch_chained(s, k, (unsigned)P.nelem, VDims<N>::NT, bytes, P);
     } else {
         if constexpr (HYPER) {
             auto k = viscous_stage_kernel<N, R, MIXED, MODE, CMDG_TURB_NONE, true>;
             if ((e = opt_in(k, bytes)) != cudaSuccess) return e;
-            k<<<P.nelem, VDims<N>::NT, bytes, s>>>(P);
+            e = launch_chained(s, k, (unsigned)P.nelem, VDims<N>::NT, bytes, P);
         } else {
             return cudaErrorInvalidValue;
         }
     }
-    return cudaGetLastError();
+    return e;
 }
 
 template <int N, bool HYPER>
