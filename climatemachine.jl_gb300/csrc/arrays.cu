@@ -145,19 +145,30 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
         const R j0 = ge[(KG_JXI + fd * 3 + 0) * Np + vM];
         const R j1 = ge[(KG_JXI + fd * 3 + 1) * Np + vM];
         const R j2 = ge[(KG_JXI + fd * 3 + 2) * Np + vM];
-        const R iJm = ge[KG_INVJ * Np + vM];
-        R sJ, rs;
-        sqrt_rsqrt_r(j0 * j0 + j1 * j1 + j2 * j2, sJ, rs);
-        rs *= sgn;
-        const R nv[3] = {j0 * rs, j1 * rs, j2 * rs};
-        R qm[NSTATE], Fm[NSTATE], qp[NSTATE], S[NSTATE], jr_rho = 0, jr_rhoe = 0;
+        // |J dxi_fd/dx| n = +-J dxi_fd/dx: the normal is never normalised.  The
+        // face terms below are over 1/J, which multiplies the sum of them and
+        // the volume term, and without the interior half of the central part,
+        // which is left out with the diagonal of the derivative
+        // (KParams::DhatC).
+        const R n2 = j0 * j0 + j1 * j1 + j2 * j2;
+        const R sJ = sqrt_r(n2);
+        R qm[NSTATE], qp[NSTATE], S[NSTATE], jr_rho = 0, jr_rhoe = 0;
         PL::ld(s_node, Np, vM, qm);
         const CRV cr = s_cr[vM];
-        const R c_m = cr.x, ri_m = cr.y;
-        PL::ld(s_F + fd * SM::P5N, Np, vM, Fm);
-        R am = rs;  // Fm = am times the staged contravariant flux (on some walls Fm is the normal flux, am = 1)
-        const R mn_m = qm[1] * nv[0] + qm[2] * nv[1] + qm[3] * nv[2];
-        const R lam_m = fabs(mn_m * ri_m) + c_m;
+        const R mn_m = qm[1] * j0 + qm[2] * j1 + qm[3] * j2;
+        const R lam_m = fma(cr.x, sJ, fabs(mn_m * cr.y));
+        R F1[NSTATE] = {0, 0, 0, 0, 0};  // what stays of the interior half on some walls
+        // J dxi_fd/dx . (first-order flux) of the interior side less the staged flux
+        auto first_less_staged = [&](const Level<R>& lvm) {
+            const Thermo<R, MIXED> thm = thermo<R, MIXED>(qm, lvm, P);
+            R Ft[NSTATE];
+            PL::ld(s_F + fd * SM::P5N, Np, vM, Ft);
+            F1[0] = mn_m - Ft[0];
+            F1[1] = mn_m * thm.u[0] + thm.pflux * j0 - Ft[1];
+            F1[2] = mn_m * thm.u[1] + thm.pflux * j1 - Ft[2];
+            F1[3] = mn_m * thm.u[2] + thm.pflux * j2 - Ft[3];
+            F1[4] = mn_m * thm.rinv * thm.H - Ft[4];
+        };
         const int nb = __ldg(nbr + f);
         const R* gp = ge;  // geometry of the node across the face (own node on a wall)
         int vP = vM;
@@ -180,28 +191,22 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
             for (int s = 0; s < NSTATE; ++s) qp[s] = (R)w[s * Np];
             if (VISC) {
                 const Level<R> lvm = node_ref<R>(P, ge, Np, vM);
-                const Thermo<R, MIXED> thm = thermo<R, MIXED>(qm, lvm, P);
-                am = R(1);
-                Fm[0] = mn_m;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) Fm[1 + c] = mn_m * thm.u[c] + thm.pflux * nv[c];
-                Fm[4] = mn_m * thm.rinv * thm.H;
+                first_less_staged(lvm);
             }
         } else {
             // Impenetrable(FreeSlip) + Insulating wall
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) qp[s] = qm[s];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) qp[1 + c] = qm[1 + c] - R(2) * mn_m * nv[c];
+            for (int c = 0; c < 3; ++c) qp[1 + c] = qm[1 + c];
+            const R refl = R(2) * mn_m * rcp_r(n2);
+            qp[1] -= refl * j0;
+            qp[2] -= refl * j1;
+            qp[3] -= refl * j2;
             if (VISC) {
-                // the staged flux holds the second-order part too: walls take the first-order one
+                // the staged flux holds the second-order part too, walls take the first-order one
                 const Level<R> lvm = node_ref<R>(P, ge, Np, vM);
-                const Thermo<R, MIXED> thm = thermo<R, MIXED>(qm, lvm, P);
-                am = R(1);
-                Fm[0] = mn_m;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) Fm[1 + c] = mn_m * thm.u[c] + thm.pflux * nv[c];
-                Fm[4] = mn_m * thm.rinv * thm.H;
+                first_less_staged(lvm);
             }
         }
         const Level<R> lvp = node_ref<R>(P, gp, Np, vP);
@@ -209,19 +214,24 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
         // fewer FP64 operations; in FP32 that order measured 0.231 against
         // 0.225 ms per step (720,000 nodes)
         const Thermo<R, MIXED> thp = thermo<R, MIXED, MIXED>(qp, lvp, P);
-        const R mn_p = qp[1] * nv[0] + qp[2] * nv[1] + qp[3] * nv[2];
+        const R jv[3] = {j0, j1, j2};
+        const R mn_p = qp[1] * j0 + qp[2] * j1 + qp[3] * j2;
         const R un_p = mn_p * thp.rinv;
-        // S: the two sides' normal fluxes added up
-        S[0] = fma(am, Fm[0], mn_p);
+        // J dxi_fd/dx . (flux of the far side)
+        S[0] = mn_p;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) S[1 + c] = fma(am, Fm[1 + c], fma(un_p, qp[1 + c], thp.pflux * nv[c]));
-        S[4] = fma(am, Fm[4], un_p * thp.H);
+        for (int c = 0; c < 3; ++c) S[1 + c] = fma(un_p, qp[1 + c], thp.pflux * jv[c]);
+        S[4] = un_p * thp.H;
+        if (VISC) {
+#pragma unroll
+            for (int s = 0; s < NSTATE; ++s) S[s] += F1[s];
+        }
         if (VISC && nb >= 0) {
             // facing node's viscous flux . n
             R Fv[3][NSTATE];
             shell_visc_flux<R, MIXED, VT>(P, nb, vP, Np, qp, lvp, thp.rinv, Fv);
 #pragma unroll
-            for (int s2 = 0; s2 < NSTATE; ++s2) S[s2] += nv[0] * Fv[0][s2] + nv[1] * Fv[1][s2] + nv[2] * Fv[2][s2];
+            for (int s2 = 0; s2 < NSTATE; ++s2) S[s2] += j0 * Fv[0][s2] + j1 * Fv[1][s2] + j2 * Fv[2][s2];
         } else if (VISC && P.mms_wall) {
             // InitStateBC second order: the one-sided flux of the wall state with
             // the interior gradient state (NumericalFluxes.jl:872-966); the face
@@ -230,12 +240,11 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
             shell_visc_flux<R, MIXED, VT>(P, e, vM, Np, qp, lvp, thp.rinv, Fv);
 #pragma unroll
             for (int s2 = 0; s2 < NSTATE; ++s2)
-                S[s2] += R(2) * (nv[0] * Fv[0][s2] + nv[1] * Fv[1][s2] + nv[2] * Fv[2][s2]);
+                S[s2] += R(2) * (j0 * Fv[0][s2] + j1 * Fv[1][s2] + j2 * Fv[2][s2]);
         }
-        const R lam_p = fabs(un_p) + thp.c;
-        const R lift = sJ * iJm * KConst<R>::inv_w0(P);
-        const R hl = R(0.5) * lift;
-        const R pl = (ph.numflux == CMDG_FLUX_RUSANOV) ? hl * max_nonneg(lam_m, lam_p) : R(0);
+        const R lam_p = fma(thp.c, sJ, fabs(un_p));
+        const R hw = R(0.5) * KConst<R>::inv_w0(P), hl = sgn * hw;
+        const R pl = (ph.numflux == CMDG_FLUX_RUSANOV) ? hw * max_nonneg(lam_m, lam_p) : R(0);
         R fs[NSTATE];
         lifted_flux<R, MIXED>(S, qm, qp, jr_rho, jr_rhoe, hl, pl, fs);
         PL::st(s_fs, NFN, f * Nfp + fn, fs);
@@ -249,24 +258,23 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     if (node_thread) {
         R acc[NSTATE] = {0, 0, 0, 0, 0};
         const int L1 = Nq * (nj + Nq * nk), L2 = ni + Nfp * nk, L3 = ni + Nq * nj;
+        constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
-        for (int n = 0; n < Nq; ++n) {
+        for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+            const int n1 = SKIP ? others(n, ni) : n, n2 = SKIP ? others(n, nj) : n, n3 = SKIP ? others(n, nk) : n;
             R v1[NSTATE], v2[NSTATE], v3[NSTATE];
-            PL::ld(s_F, Np, L1 + n, v1);
-            PL::ld(s_F + SM::P5N, Np, L2 + n * Nq, v2);
-            PL::ld(s_F + 2 * SM::P5N, Np, L3 + n * Nfp, v3);
-            const R d1 = s_D[ni * Nq + n], d2 = s_D[nj * Nq + n], d3 = s_D[nk * Nq + n];
+            PL::ld(s_F, Np, L1 + n1, v1);
+            PL::ld(s_F + SM::P5N, Np, L2 + n2 * Nq, v2);
+            PL::ld(s_F + 2 * SM::P5N, Np, L3 + n3 * Nfp, v3);
+            const R d1 = s_D[ni * Nq + n1], d2 = s_D[nj * Nq + n2], d3 = s_D[nk * Nq + n3];
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) acc[s] = fma(d1, v1[s], fma(d2, v2[s], fma(d3, v3[s], acc[s])));
         }
-        R rhs[NSTATE];
-#pragma unroll
-        for (int s = 0; s < NSTATE; ++s) rhs[s] = invJ * acc[s];
         auto sub_face = [&](int ff, int idx) {
             R v[NSTATE];
             PL::ld(s_fs, NFN, ff * Nfp + idx, v);
 #pragma unroll
-            for (int s = 0; s < NSTATE; ++s) rhs[s] -= v[s];
+            for (int s = 0; s < NSTATE; ++s) acc[s] -= v[s];
         };
         if (ni == 0) sub_face(0, nj + Nq * nk);
         if (ni == N) sub_face(1, nj + Nq * nk);
@@ -274,6 +282,9 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
         if (nj == N) sub_face(3, ni + Nq * nk);
         if (nk == 0) sub_face(4, ni + Nq * nj);
         if (nk == N) sub_face(5, ni + Nq * nj);
+        R rhs[NSTATE];
+#pragma unroll
+        for (int s = 0; s < NSTATE; ++s) rhs[s] = invJ * acc[s];
 #pragma unroll
         for (int c = 0; c < 3; ++c) rhs[1 + c] += src[c];
         if (P.mms_src) {

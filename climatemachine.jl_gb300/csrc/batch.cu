@@ -148,7 +148,7 @@ static void build_dhat(EnsDhat& d) {
         m.N = N;
         m.Nq = N + 1;
         lgl_derivative(&m);
-        for (int i = 0; i < m.Nq * m.Nq; ++i) rows[N - BATCH_NMIN][i] = (float)m.Dhat[i];
+        for (int i = 0; i < m.Nq * m.Nq; ++i) rows[N - BATCH_NMIN][i] = i % (m.Nq + 1) == 0 ? 0.0f : (float)m.Dhat[i];
     }
 }
 

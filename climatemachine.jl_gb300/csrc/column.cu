@@ -77,9 +77,10 @@ __device__ __forceinline__ double dhat_c<double>(const KParams& P, int idx) {
 }
 
 // Numerical flux F*.n (Rusanov or central) of one face node, lifted:
-// out = lift * (1/2 (Fm + Fp) + 1/2 max(lam_m, lam_p) ((qm - qp) + jr)).
+// out = lift * (1/2 Fp + 1/2 max(lam_m, lam_p) ((qm - qp) + jr)), the interior
+// half of the central part left out with the diagonal of Dhat.
 template <typename R, bool MIXED>
-__device__ __forceinline__ void face_flux(const KParams& P, const R qm[NSTATE], const R Fm[NSTATE], R lam_m,
+__device__ __forceinline__ void face_flux(const KParams& P, const R qm[NSTATE], R lam_m,
                                           const R qp_in[NSTATE], bool wall, const Level<R>& lvp, int d, R sgn,
                                           const R jr[NSTATE], R lift, R out[NSTATE]) {
     R qp[NSTATE];
@@ -99,7 +100,7 @@ __device__ __forceinline__ void face_flux(const KParams& P, const R qm[NSTATE], 
     const R hmw = (P.ph.numflux == CMDG_FLUX_RUSANOV) ? R(0.5) * fmax(lam_m, lam_p) : R(0);
     const R hl = R(0.5) * lift, pl = hmw * lift;
 #pragma unroll
-    for (int s = 0; s < NSTATE; ++s) out[s] = hl * (Fm[s] + Fp[s]) + pl * ((qm[s] - qp[s]) + jr[s]);
+    for (int s = 0; s < NSTATE; ++s) out[s] = hl * Fp[s] + pl * ((qm[s] - qp[s]) + jr[s]);
 }
 
 template <int N, typename R, bool MIXED, int MODE>
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(ColCfg<N>::EPB*(N + 1) * (N + 1), ColCfg<N>::M
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) acc[m][s] = 0;
     R gsrc[Nq];
-    R qend[2][NSTATE], Fend[2][NSTATE], c_end[2], ri_end[2];
+    R qend[2][NSTATE], c_end[2], ri_end[2];
 #pragma unroll
     for (int k = 0; k < Nq; ++k) {
         R qk[NSTATE];
@@ -172,10 +173,7 @@ __global__ void __launch_bounds__(ColCfg<N>::EPB*(N + 1) * (N + 1), ColCfg<N>::M
         if (k == 0 || k == N) {
             const int side = k == 0 ? 0 : 1;
 #pragma unroll
-            for (int s = 0; s < NSTATE; ++s) {
-                qend[side][s] = qk[s];
-                Fend[side][s] = F[s];
-            }
+            for (int s = 0; s < NSTATE; ++s) qend[side][s] = qk[s];
             c_end[side] = th.c;
             ri_end[side] = th.rinv;
         }
@@ -213,9 +211,7 @@ __global__ void __launch_bounds__(ColCfg<N>::EPB*(N + 1) * (N + 1), ColCfg<N>::M
             const int k = side ? N : 0;
             const R sgn = side ? R(1) : R(-1);
             const int nbv = side ? nbt : nbb;
-            R Fm[NSTATE], qv[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
-#pragma unroll
-            for (int s = 0; s < NSTATE; ++s) Fm[s] = sgn * Fend[side][s];
+            R qv[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
             const R lam_m = fabs(qend[side][3] * ri_end[side]) + c_end[side];
             int lev_p = ez * Nq + k;
             if (nbv >= 0) {
@@ -234,7 +230,7 @@ __global__ void __launch_bounds__(ColCfg<N>::EPB*(N + 1) * (N + 1), ColCfg<N>::M
             }
             const Level<R> lvp = load_level<R>(P, lev_p);
             R fs[NSTATE];
-            face_flux<R, MIXED>(P, qend[side], Fm, lam_m, qv, nbv < 0, lvp, 2, sgn, jr, lift3, fs);
+            face_flux<R, MIXED>(P, qend[side], lam_m, qv, nbv < 0, lvp, 2, sgn, jr, lift3, fs);
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) acc[k][s] -= fs[s];
         }
@@ -245,7 +241,6 @@ __global__ void __launch_bounds__(ColCfg<N>::EPB*(N + 1) * (N + 1), ColCfg<N>::M
     {
         const int ca = c % Nq, cb = c / Nq;
         const int vPh[4] = {N + Nq * c, Nq * c, ca + Nq * (N + Nq * cb), ca + Nq * (Nq * cb)};
-        const int vMh[4] = {Nq * c, N + Nq * c, ca + Nfp * cb, ca + Nq * N + Nfp * cb};
         const R inv_w0 = KConst<R>::inv_w0(P);
         const Level<R> lvh = load_level<R>(P, ez * Nq + cb);
 #pragma unroll
@@ -258,17 +253,14 @@ __global__ void __launch_bounds__(ColCfg<N>::EPB*(N + 1) * (N + 1), ColCfg<N>::M
 #pragma unroll
                 for (int s = 0; s < NSTATE; ++s) qh[s] = qn[s * Np];
             }
-            R qm[NSTATE], Fm[NSTATE];
+            R qm[NSTATE];
             PL::ld(sNode, NH, f * Nfp + c, qm);
             const CRV cr = sCR[f * Nfp + c];
             const R c_m = cr.x, ri_m = cr.y;
-            PL::ld(d == 0 ? sF1 : sF2, Np, vMh[f], Fm);
-#pragma unroll
-            for (int s = 0; s < NSTATE; ++s) Fm[s] *= sgn;
             const R lam_m = fabs(qm[1 + d] * ri_m) + c_m;
             const R jr[NSTATE] = {0, 0, 0, 0, 0};
             R fs[NSTATE];
-            face_flux<R, MIXED>(P, qm, Fm, lam_m, qh, nbf[f] < 0, lvh, d, sgn, jr, xi[d] * inv_w0, fs);
+            face_flux<R, MIXED>(P, qm, lam_m, qh, nbf[f] < 0, lvh, d, sgn, jr, xi[d] * inv_w0, fs);
             PL::st(sFace, NH, f * Nfp + c, fs);
         }
         R Di[Nq], Dj[Nq];

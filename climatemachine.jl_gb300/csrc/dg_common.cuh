@@ -29,7 +29,13 @@ struct KParams {
     int first_stage, last_stage;
     Physics ph;
     // weak-form derivative Dhat[i][n] = D[n][i] w_n / w_i (row-major, N <= MAX_N),
-    // in the parameter bank so compile-time indexed reads cost no instruction
+    // in the parameter bank so compile-time indexed reads cost no instruction.
+    // The derivative tables of the kernels (Dhat, DhatC, DC) have a zero
+    // diagonal: by summation by parts on LGL points it is zero at interior
+    // nodes and -+1/(2 w_0) at the two ends, where the term it makes is the
+    // negative of the interior side's half of the central face term (the
+    // lift is 1/w_0 times the same metric).  Both are left out, and the face
+    // terms take the far side only.
     float DhatC32[(MAX_N + 1) * (MAX_N + 1)];
     double DhatC64[(MAX_N + 1) * (MAX_N + 1)];
     // diffusive passes: gradient-flux state, reference rows, strong-form D
@@ -319,26 +325,27 @@ __device__ __forceinline__ R pick3(int d, R a, R b, R c) {
     return d == 0 ? a : (d == 1 ? b : c);
 }
 
-// S = Fm + F_d(q): the sum of the two sides' fluxes along +xi_d across a face
-// normal to xi_d, the far side from its state and thermodynamics (the
-// momentum flux as u_d q, so that the sum is one FMA per field)
-template <typename R, bool MIXED>
-__device__ __forceinline__ void add_flux_d(const R Fm[NSTATE], const R q[NSTATE], R mn, R un, R pflux, R H, int d,
-                                           R S[NSTATE]) {
-    S[0] = Fm[0] + mn;
-    S[1] = fma(un, q[1], Fm[1]);
-    S[2] = fma(un, q[2], Fm[2]);
-    S[3] = fma(un, q[3], Fm[3]);
-    const R sn = pick3(d, S[1], S[2], S[3]) + pflux;
-    S[1] = d == 0 ? sn : S[1];
-    S[2] = d == 1 ? sn : S[2];
-    S[3] = d == 2 ? sn : S[3];
-    S[4] = fma(un, H, Fm[4]);
+// n-th position of a line other than i (n = 0 .. N - 1): the terms of a
+// contraction with a zero diagonal.  The FP64 kernels skip the diagonal this
+// way (integer work is free beside their FP64 pipe), the FP32 kernels
+// multiply by the zero.
+__device__ __forceinline__ int others(int n, int i) { return n + (n >= i ? 1 : 0); }
+
+// flux along +xi_d of the far side of a face normal to xi_d (the momentum
+// flux as u_d q)
+template <typename R>
+__device__ __forceinline__ void far_flux_d(const R q[NSTATE], R mn, R un, R pflux, R H, int d, R S[NSTATE]) {
+    S[0] = mn;
+    const R sn = fma(un, mn, pflux);
+    S[1] = d == 0 ? sn : un * q[1];
+    S[2] = d == 1 ? sn : un * q[2];
+    S[3] = d == 2 ? sn : un * q[3];
+    S[4] = un * H;
 }
 
-// lifted numerical flux hl S + pl ((qm - qp) + jr) of one face node: hl half
-// the signed lift, pl the penalty's weight, jr the reference-state jumps of
-// the density and the energy (mixed precision only)
+// lifted numerical flux hl S + pl ((qm - qp) + jr) of one face node: S the far
+// side's flux, hl half the signed lift, pl the penalty's weight, jr the
+// reference-state jumps of the density and the energy (mixed precision only)
 template <typename R, bool MIXED>
 __device__ __forceinline__ void lifted_flux(const R S[NSTATE], const R qm[NSTATE], const R qp[NSTATE], R jr_rho,
                                             R jr_rhoe, R hl, R pl, R fs[NSTATE]) {

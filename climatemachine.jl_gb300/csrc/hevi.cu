@@ -92,15 +92,17 @@ __device__ __forceinline__ void lin_load(const LinParams& P, int64_t e, int node
 }
 
 // Lifted Rusanov flux of the linear model across one face node,
-// fl = lift ((F- + F+) . n / 2 + max(c-, c+) (q- - q+) / 2); qP from the
-// facing node, or the FreeSlip reflection of qM on a wall (aux+ = aux-).
+// fl = lift (F+ . n / 2 + max(c-, c+) (q- - q+) / 2) (the interior half of
+// the central part is the negative of the diagonal term of the weak
+// derivative at an end node, and both are left out); qP from the facing node,
+// or the FreeSlip reflection of qM on a wall (aux+ = aux-).
 __device__ __forceinline__ void lin_face(const LinNode& M, const LinNode& Pn, bool wall, const double n[3],
                                          double lift, double fl[5]) {
-    const double unm = M.q[1] * n[0] + M.q[2] * n[1] + M.q[3] * n[2];
     double qp[5], pP = M.pL, hP = M.h, cP = M.c;
 #pragma unroll
     for (int s = 0; s < 5; ++s) qp[s] = M.q[s];
     if (wall) {
+        const double unm = M.q[1] * n[0] + M.q[2] * n[1] + M.q[3] * n[2];
 #pragma unroll
         for (int c = 0; c < 3; ++c) qp[1 + c] = fma(-2 * unm, n[c], M.q[1 + c]);
     } else {
@@ -114,18 +116,17 @@ __device__ __forceinline__ void lin_face(const LinNode& M, const LinNode& Pn, bo
     const double hl = 0.5 * lift;
     // reference sound speeds: positive, ordered as their bits
     const double pl = hl * (__double_as_longlong(M.c) > __double_as_longlong(cP) ? M.c : cP);
-    const double hp = hl * (M.pL + pP);
-    fl[0] = fma(pl, M.q[0] - qp[0], hl * (unm + unp));
+    const double hp = hl * pP;
+    fl[0] = fma(pl, M.q[0] - qp[0], hl * unp);
 #pragma unroll
     for (int c = 0; c < 3; ++c) fl[1 + c] = fma(pl, M.q[1 + c] - qp[1 + c], hp * n[c]);
-    fl[4] = fma(pl, M.q[4] - qp[4], hl * fma(M.h, unm, hP * unp));
+    fl[4] = fma(pl, M.q[4] - qp[4], hl * (hP * unp));
 }
 
 // One thread per (element, i, j) node line.  The FP64 pipe bounds it (1/72 of
 // the FP32 rate): the energy flux is h_ref times the mass flux, 1/M and alpha
-// multiply the finished contraction, and a face's lift goes into its two
-// weights: 67 operations per node, 94 us on 648,000 nodes against 102 us with
-// 80 (that pipe is 81% busy).
+// multiply the finished contraction, a face's lift goes into its two weights,
+// and the contraction leaves out its diagonal.
 template <int Nq>
 __global__ void __launch_bounds__(128) linear_tendency_kernel(const LinParams P) {
     constexpr int Nfp = Nq * Nq, Np = Nfp * Nq;
@@ -171,9 +172,11 @@ __global__ void __launch_bounds__(128) linear_tendency_kernel(const LinParams P)
         const double aMI = P.alpha * L[LT_MI * Np + node], arho = P.alpha * rho[k];
 #pragma unroll
         for (int s = 0; s < 5; ++s) {
-            double acc = P.D[k] * F3[0][s];
+            double acc = 0.0;
 #pragma unroll
-            for (int kk = 1; kk < Nq; ++kk) acc = fma(P.D[kk * Nq + k], F3[kk][s], acc);
+            for (int kk = 0; kk < Nq; ++kk)
+                if (kk != k) acc = (kk == 0 || (k == 0 && kk == 1)) ? P.D[kk * Nq + k] * F3[kk][s]
+                                                                    : fma(P.D[kk * Nq + k], F3[kk][s], acc);
             double v = 0.0;
             if (!zero_beta) {
                 v = Te[s * Np + node];

@@ -76,10 +76,8 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_grad_kernel(const KParams 
                                                                   R* __restrict__ hg) {
     using Ix = HypIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp, ESTRIDE = NSTATE * Np;
-    using PL = Planar5<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R* const s_q = reinterpret_cast<R*>(smem_raw);  // planar records: states
-    R* const s_H = s_q + planar_pad<R>(5 * Np);      // [3][Np] arguments
+    R* const s_H = reinterpret_cast<R*>(smem_raw);   // [3][Np] arguments
     R* const s_dH = s_H + 3 * Np;                    // [3][NFN] lifted face terms
     R* const s_D = s_dH + 3 * NFN;                   // strong-form D
 
@@ -116,32 +114,36 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_grad_kernel(const KParams 
     if (x.node) {
         R H[3];
         hyper_args<R, MIXED>(P, q, ez * Nq + x.nk, H);
-        PL::st(s_q, Np, t, q);
 #pragma unroll
         for (int s = 0; s < 3; ++s) s_H[s * Np + t] = H[s];
     }
     __syncthreads();
 
-    // face terms c n (H+ - H-) lifted, c = 1/2 inside, 1 on walls
+    // face terms c n (H+ - H-) / w_0, c = 1/2 inside, 1 on walls, as an addition
+    // to the derivative along xi_fd and without what the diagonal of D leaves
+    // out (KParams::DC)
     if (x.face) {
-        R Hp[3], c;
+        R Hp[3];
         if (nb >= 0) {
             hyper_args<R, MIXED>(P, qp, levp, Hp);
-            c = R(0.5);
+#pragma unroll
+            for (int s = 0; s < 3; ++s) Hp[s] *= R(0.5);
         } else {
             // FreeSlip state of the gradient flux: rhou+ = rhou- - (rhou-.n) n
+            const R* qn = Qin + (size_t)e * ESTRIDE + x.vM;
             R qb[NSTATE];
-            PL::ld(s_q, Np, x.vM, qb);
-            if (x.fd == 0) qb[1] = R(0);
-            if (x.fd == 1) qb[2] = R(0);
-            if (x.fd == 2) qb[3] = R(0);
-            hyper_args<R, MIXED>(P, qb, levp, Hp);
-            c = R(1);
-        }
-        const R sgn = x.fside ? R(1) : R(-1);
-        const R w = c * sgn * pick3(x.fd, xi[0], xi[1], xz) * KConst<R>::inv_w0(P);
 #pragma unroll
-        for (int s = 0; s < 3; ++s) s_dH[s * NFN + t] = w * (Hp[s] - s_H[s * Np + x.vM]);
+            for (int s = 0; s < NSTATE; ++s) qb[s] = qn[s * Np];
+            qb[1] = x.fd == 0 ? R(0) : qb[1];
+            qb[2] = x.fd == 1 ? R(0) : qb[2];
+            qb[3] = x.fd == 2 ? R(0) : qb[3];
+            hyper_args<R, MIXED>(P, qb, levp, Hp);
+#pragma unroll
+            for (int s = 0; s < 3; ++s) Hp[s] = fma(R(-0.5), s_H[s * Np + x.vM], Hp[s]);
+        }
+        const R w = (x.fside ? R(1) : R(-1)) * KConst<R>::inv_w0(P);
+#pragma unroll
+        for (int s = 0; s < 3; ++s) s_dH[s * NFN + t] = w * Hp[s];
     }
     __syncthreads();
     chain_release();
@@ -149,21 +151,17 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_grad_kernel(const KParams 
     if (x.node) {
         R g1[3] = {0, 0, 0}, g2[3] = {0, 0, 0}, g3[3] = {0, 0, 0};
         const int L1 = Nq * (x.nj + Nq * x.nk), L2 = x.ni + Nfp * x.nk, L3 = x.ni + Nq * x.nj;
+        constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
-        for (int n = 0; n < Nq; ++n) {
-            const R d1 = s_D[x.ni * Nq + n], d2 = s_D[x.nj * Nq + n], d3 = s_D[x.nk * Nq + n];
+        for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+            const int n1 = SKIP ? others(n, x.ni) : n, n2 = SKIP ? others(n, x.nj) : n, n3 = SKIP ? others(n, x.nk) : n;
+            const R d1 = s_D[x.ni * Nq + n1], d2 = s_D[x.nj * Nq + n2], d3 = s_D[x.nk * Nq + n3];
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
-                g1[s] = fma(d1, s_H[s * Np + L1 + n], g1[s]);
-                g2[s] = fma(d2, s_H[s * Np + L2 + n * Nq], g2[s]);
-                g3[s] = fma(d3, s_H[s * Np + L3 + n * Nfp], g3[s]);
+                g1[s] = fma(d1, s_H[s * Np + L1 + n1], g1[s]);
+                g2[s] = fma(d2, s_H[s * Np + L2 + n2 * Nq], g2[s]);
+                g3[s] = fma(d3, s_H[s * Np + L3 + n3 * Nfp], g3[s]);
             }
-        }
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            g1[s] *= xi[0];
-            g2[s] *= xi[1];
-            g3[s] *= xz;
         }
         auto add = [&](int ff, R* gd) {
             const int idx = ff * Nfp + x.on_face(ff);
@@ -176,6 +174,12 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_grad_kernel(const KParams 
         if (x.nj == N) add(3, g2);
         if (x.nk == 0) add(4, g3);
         if (x.nk == N) add(5, g3);
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+            g1[s] *= xi[0];
+            g2[s] *= xi[1];
+            g3[s] *= xz;
+        }
         R* o = hg + (size_t)e * 9 * Np + t;
 #pragma unroll
         for (int s = 0; s < 3; ++s) {
@@ -219,13 +223,10 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_div_kernel(const KParams P
     __syncthreads();
 
     if (x.face) {
-        const R sgn = x.fside ? R(1) : R(-1);
-        const R w = sgn * pick3(x.fd, xi[0], xi[1], xz) * KConst<R>::inv_w0(P);
+        // the far side's half of the central term (KParams::DhatC)
+        const R w = (x.fside ? R(0.5) : R(-0.5)) * pick3(x.fd, xi[0], xi[1], xz) * KConst<R>::inv_w0(P);
 #pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            const R Gm = s_G[(3 * s + x.fd) * Np + x.vM];
-            s_dF[s * NFN + t] = w * ((nb >= 0 ? Gp[s] : Gm) + Gm) / R(2);
-        }
+        for (int s = 0; s < 3; ++s) s_dF[s * NFN + t] = w * (nb >= 0 ? Gp[s] : s_G[(3 * s + x.fd) * Np + x.vM]);
     }
     __syncthreads();
     chain_release();
@@ -233,14 +234,16 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_div_kernel(const KParams P
     if (x.node) {
         R a1[3] = {0, 0, 0}, a2[3] = {0, 0, 0}, a3[3] = {0, 0, 0};
         const int L1 = Nq * (x.nj + Nq * x.nk), L2 = x.ni + Nfp * x.nk, L3 = x.ni + Nq * x.nj;
+        constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
-        for (int n = 0; n < Nq; ++n) {
-            const R d1 = s_Dh[x.ni * Nq + n], d2 = s_Dh[x.nj * Nq + n], d3 = s_Dh[x.nk * Nq + n];
+        for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+            const int n1 = SKIP ? others(n, x.ni) : n, n2 = SKIP ? others(n, x.nj) : n, n3 = SKIP ? others(n, x.nk) : n;
+            const R d1 = s_Dh[x.ni * Nq + n1], d2 = s_Dh[x.nj * Nq + n2], d3 = s_Dh[x.nk * Nq + n3];
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
-                a1[s] = fma(d1, s_G[(3 * s + 0) * Np + L1 + n], a1[s]);
-                a2[s] = fma(d2, s_G[(3 * s + 1) * Np + L2 + n * Nq], a2[s]);
-                a3[s] = fma(d3, s_G[(3 * s + 2) * Np + L3 + n * Nfp], a3[s]);
+                a1[s] = fma(d1, s_G[(3 * s + 0) * Np + L1 + n1], a1[s]);
+                a2[s] = fma(d2, s_G[(3 * s + 1) * Np + L2 + n2 * Nq], a2[s]);
+                a3[s] = fma(d3, s_G[(3 * s + 2) * Np + L3 + n3 * Nfp], a3[s]);
             }
         }
         R lap[3];
@@ -300,11 +303,11 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams 
     __syncthreads();
 
     if (x.face) {
-        const R sgn = x.fside ? R(1) : R(-1);
-        const R w = sgn * pick3(x.fd, xi[0], xi[1], xz) * KConst<R>::inv_w0(P);
+        // n (L+ - L-) / (2 w_0) added to the derivative along xi_fd, without
+        // what the diagonal of D leaves out (KParams::DC)
+        const R w = (x.fside ? R(0.5) : R(-0.5)) * KConst<R>::inv_w0(P);
 #pragma unroll
-        for (int s = 0; s < 3; ++s)
-            s_dL[s * NFN + t] = nb >= 0 ? w * (Lp[s] - s_L[s * Np + x.vM]) / R(2) : R(0);
+        for (int s = 0; s < 3; ++s) s_dL[s * NFN + t] = w * (nb >= 0 ? Lp[s] : s_L[s * Np + x.vM]);
     }
     __syncthreads();
     chain_release();
@@ -312,21 +315,17 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams 
     if (x.node) {
         R g1[3] = {0, 0, 0}, g2[3] = {0, 0, 0}, g3[3] = {0, 0, 0};
         const int L1 = Nq * (x.nj + Nq * x.nk), L2 = x.ni + Nfp * x.nk, L3 = x.ni + Nq * x.nj;
+        constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
-        for (int n = 0; n < Nq; ++n) {
-            const R d1 = s_D[x.ni * Nq + n], d2 = s_D[x.nj * Nq + n], d3 = s_D[x.nk * Nq + n];
+        for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+            const int n1 = SKIP ? others(n, x.ni) : n, n2 = SKIP ? others(n, x.nj) : n, n3 = SKIP ? others(n, x.nk) : n;
+            const R d1 = s_D[x.ni * Nq + n1], d2 = s_D[x.nj * Nq + n2], d3 = s_D[x.nk * Nq + n3];
 #pragma unroll
             for (int s = 0; s < 3; ++s) {
-                g1[s] = fma(d1, s_L[s * Np + L1 + n], g1[s]);
-                g2[s] = fma(d2, s_L[s * Np + L2 + n * Nq], g2[s]);
-                g3[s] = fma(d3, s_L[s * Np + L3 + n * Nfp], g3[s]);
+                g1[s] = fma(d1, s_L[s * Np + L1 + n1], g1[s]);
+                g2[s] = fma(d2, s_L[s * Np + L2 + n2 * Nq], g2[s]);
+                g3[s] = fma(d3, s_L[s * Np + L3 + n3 * Nfp], g3[s]);
             }
-        }
-#pragma unroll
-        for (int s = 0; s < 3; ++s) {
-            g1[s] *= xi[0];
-            g2[s] *= xi[1];
-            g3[s] *= xz;
         }
         auto add = [&](int ff, R* gd) {
             const int idx = ff * Nfp + x.on_face(ff);
@@ -339,6 +338,12 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams 
         if (x.nj == N) add(3, g2);
         if (x.nk == 0) add(4, g3);
         if (x.nk == N) add(5, g3);
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+            g1[s] *= xi[0];
+            g2[s] *= xi[1];
+            g3[s] *= xz;
+        }
         if (MIXED) g3[2] += P.glap_ref32[ez * Nq + x.nk];
         R* o = hd + (size_t)e * 9 * Np + t;
 #pragma unroll
@@ -353,7 +358,7 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams 
 template <int N, typename R, bool MIXED>
 cudaError_t launch_passes_typed(const KParams& P, const void* Q, void* hd, void* hl, cudaStream_t s) {
     constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp, NFN = 6 * Nfp, NT = VDims<N>::NT;
-    constexpr size_t b1 = sizeof(R) * (planar_pad<R>(5 * Np) + 3 * Np + 3 * NFN + Nq * Nq);
+    constexpr size_t b1 = sizeof(R) * (3 * Np + 3 * NFN + Nq * Nq);
     constexpr size_t b2 = sizeof(R) * (9 * Np + 3 * NFN + Nq * Nq);
     constexpr size_t b3 = sizeof(R) * (3 * Np + 3 * NFN + Nq * Nq);
     cudaError_t e;

@@ -56,20 +56,18 @@ struct ShellIdx {
     }
 };
 
-// Unit outward normal, and the lift weight vMI sM = |J dxi_fd/dx| / (J w_0),
-// of face node vM (face direction fd, sign sgn) from the element's kernel
-// geometry g.
+// Unit normal (of either sign) of face node vM, face direction fd, from the
+// element's kernel geometry g.
 template <typename R>
-__device__ __forceinline__ R shell_face_normal(const KParams& P, const R* g, int Np, int fd, R sgn, int vM, R nv[3]) {
+__device__ __forceinline__ void shell_face_normal(const R* g, int Np, int fd, int vM, R nv[3]) {
     const R j0 = g[(KG_JXI + fd * 3 + 0) * Np + vM];
     const R j1 = g[(KG_JXI + fd * 3 + 1) * Np + vM];
     const R j2 = g[(KG_JXI + fd * 3 + 2) * Np + vM];
-    const R sJ = sqrt_r(j0 * j0 + j1 * j1 + j2 * j2);
-    const R rs = rcp_r(sJ);
-    nv[0] = sgn * j0 * rs;
-    nv[1] = sgn * j1 * rs;
-    nv[2] = sgn * j2 * rs;
-    return sJ * g[KG_INVJ * Np + vM] * KConst<R>::inv_w0(P);
+    R sJ, rs;
+    sqrt_rsqrt_r(j0 * j0 + j1 * j1 + j2 * j2, sJ, rs);
+    nv[0] = j0 * rs;
+    nv[1] = j1 * rs;
+    nv[2] = j2 * rs;
 }
 
 // GradientLaplacian arguments (u_h[0..2], h_tot) of a state at a node with
@@ -117,7 +115,12 @@ __device__ __forceinline__ void shell_hyper_args(const KParams& P, const R q[NST
 }
 
 // strong-form gradient of 4 node fields s_X[4][Np] at this node thread,
-// dxi_d/dx_j dX/dxi_d, plus the staged face terms s_dF[(3 s + j) NFN + face node]
+// dxi_d/dx_j dX/dxi_d, with the staged face terms s_dF[s NFN + face node] added
+// to the derivatives along xi_d: vMI sM n_j = +-dxi_d/dx_j / w_0 at a face
+// normal to xi_d, so a central face correction is one number per field, not a
+// vector, and needs no normal (a third of the shared words; with the same in
+// the divergence pass, the GCM step with hyperdiffusion went from 347 to
+// 318 us)
 template <int N, typename R, int NA = 4>
 __device__ __forceinline__ void shell_strong_gradient(const ShellIdx<N>& x, const R* s_X, const R* s_dF, const R* s_D,
                                                       const R* g, int t, bool horiz, R out[3 * NA]) {
@@ -126,16 +129,29 @@ __device__ __forceinline__ void shell_strong_gradient(const ShellIdx<N>& x, cons
 #pragma unroll
     for (int s = 0; s < NA; ++s) a[s][0] = a[s][1] = a[s][2] = R(0);
     const int L1 = Nq * (x.nj + Nq * x.nk), L2 = x.ni + Nfp * x.nk, L3 = x.ni + Nq * x.nj;
+    constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
-    for (int n = 0; n < Nq; ++n) {
-        const R d1 = s_D[x.ni * Nq + n], d2 = s_D[x.nj * Nq + n], d3 = s_D[x.nk * Nq + n];
+    for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+        const int n1 = SKIP ? others(n, x.ni) : n, n2 = SKIP ? others(n, x.nj) : n, n3 = SKIP ? others(n, x.nk) : n;
+        const R d1 = s_D[x.ni * Nq + n1], d2 = s_D[x.nj * Nq + n2], d3 = s_D[x.nk * Nq + n3];
 #pragma unroll
         for (int s = 0; s < NA; ++s) {
-            a[s][0] = fma(d1, s_X[s * Np + L1 + n], a[s][0]);
-            a[s][1] = fma(d2, s_X[s * Np + L2 + n * Nq], a[s][1]);
-            a[s][2] = fma(d3, s_X[s * Np + L3 + n * Nfp], a[s][2]);
+            a[s][0] = fma(d1, s_X[s * Np + L1 + n1], a[s][0]);
+            a[s][1] = fma(d2, s_X[s * Np + L2 + n2 * Nq], a[s][1]);
+            a[s][2] = fma(d3, s_X[s * Np + L3 + n3 * Nfp], a[s][2]);
         }
     }
+    auto add = [&](int ff) {
+        const int idx = ff * Nfp + x.on_face(ff);
+#pragma unroll
+        for (int s = 0; s < NA; ++s) a[s][ff >> 1] += s_dF[s * NFN + idx];
+    };
+    if (x.ni == 0) add(0);
+    if (x.ni == N) add(1);
+    if (x.nj == 0) add(2);
+    if (x.nj == N) add(3);
+    if (x.nk == 0) add(4);
+    if (x.nk == N) add(5);
     R Jx[9];
 #pragma unroll
     for (int w = 0; w < 9; ++w) Jx[w] = g[(KG_JXI + w) * Np + t];
@@ -148,17 +164,6 @@ __device__ __forceinline__ void shell_strong_gradient(const ShellIdx<N>& x, cons
     for (int s = 0; s < NA; ++s)
 #pragma unroll
         for (int j = 0; j < 3; ++j) out[3 * s + j] = iJ * (Jx[j] * a[s][0] + Jx[3 + j] * a[s][1] + Jx[6 + j] * a[s][2]);
-    auto add = [&](int ff) {
-        const int idx = ff * Nfp + x.on_face(ff);
-#pragma unroll
-        for (int w = 0; w < 3 * NA; ++w) out[w] += s_dF[w * NFN + idx];
-    };
-    if (x.ni == 0) add(0);
-    if (x.ni == N) add(1);
-    if (x.nj == 0) add(2);
-    if (x.nj == N) add(3);
-    if (x.nk == 0) add(4);
-    if (x.nk == N) add(5);
 }
 
 // level and kernel geometry of the node across face x.f (nb >= 0)
@@ -177,12 +182,10 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
     using Ix = ShellIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp, ESTRIDE = NSTATE * Np;
     constexpr int GSTRIDE = KG_NFIELDS * Np;
-    using PL = Planar5<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R* const s_q = reinterpret_cast<R*>(smem_raw);  // planar records: states
-    R* const s_H = s_q + planar_pad<R>(5 * Np);      // [NA][Np] arguments
-    R* const s_dF = s_H + NA * Np;                   // [3 NA][NFN] lifted face terms
-    R* const s_D = s_dF + 3 * NA * NFN;              // strong-form D
+    R* const s_H = reinterpret_cast<R*>(smem_raw);   // [NA][Np] arguments
+    R* const s_dF = s_H + NA * Np;                   // [NA][NFN] face terms of the reference derivatives
+    R* const s_D = s_dF + NA * NFN;                  // strong-form D
 
     const int e = blockIdx.x, t = threadIdx.x;
     const Ix x(t);
@@ -212,22 +215,22 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
         R H[NA];
         const Level<R> lv = ARRAYS ? node_ref<R>(P, ge, Np, t) : shell_level<R, MIXED>(P, ge, Np, t, ez * Nq + x.nk);
         shell_hyper_args<R, MIXED, PROJECT, NA>(P, q, lv, ge, Np, t, H);
-        PL::st(s_q, Np, t, q);
 #pragma unroll
         for (int s = 0; s < NA; ++s) s_H[s * Np + t] = H[s];
     }
     __syncthreads();
 
     if (x.face) {
-        R nv[3], Hp[NA], c;
-        R lift = shell_face_normal<R>(P, ge, Np, x.fd, x.fside ? R(1) : R(-1), x.vM, nv);
-        if (PROJECT && P.hyper_horizontal && x.fd == 2) lift = R(0);  // HorizontalDirection: no xi3 face terms
+        // c n (H+ - H-) / w_0 (c = 1/2 inside, 1 on walls) for the derivative
+        // along xi_fd, without what the diagonal of D leaves out (KParams::DC)
+        R Hp[NA];
         if (nb >= 0) {
             const R* gp = geo + (size_t)nb * GSTRIDE;
             const Level<R> lvp = ARRAYS ? node_ref<R>(P, gp, Np, vP)
                                         : shell_level<R, MIXED>(P, gp, Np, vP, shell_partner_level<N>(x, ez, vP));
             shell_hyper_args<R, MIXED, PROJECT, NA>(P, qp, lvp, gp, Np, vP, Hp);
-            c = R(0.5);
+#pragma unroll
+            for (int s = 0; s < NA; ++s) Hp[s] *= R(0.5);
         } else {
             R qb[NSTATE];
             if (ARRAYS && P.mms_wall) {
@@ -237,7 +240,11 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
                 for (int cc = 0; cc < NSTATE; ++cc) qb[cc] = (R)w[cc * Np];
             } else {
                 // FreeSlip state of the gradient flux: rhou+ = rhou- - (rhou-.n) n
-                PL::ld(s_q, Np, x.vM, qb);
+                const R* qn = Qin + (size_t)e * ESTRIDE + x.vM;
+#pragma unroll
+                for (int cc = 0; cc < NSTATE; ++cc) qb[cc] = qn[cc * Np];
+                R nv[3];
+                shell_face_normal<R>(ge, Np, x.fd, x.vM, nv);
                 const R mn = qb[1] * nv[0] + qb[2] * nv[1] + qb[3] * nv[2];
 #pragma unroll
                 for (int cc = 0; cc < 3; ++cc) qb[1 + cc] -= mn * nv[cc];
@@ -245,14 +252,12 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
             const Level<R> lvm =
                 ARRAYS ? node_ref<R>(P, ge, Np, x.vM) : shell_level<R, MIXED>(P, ge, Np, x.vM, ez * Nq + x.kM);
             shell_hyper_args<R, MIXED, PROJECT, NA>(P, qb, lvm, ge, Np, x.vM, Hp);
-            c = R(1);
-        }
 #pragma unroll
-        for (int s = 0; s < NA; ++s) {
-            const R dh = c * lift * (Hp[s] - s_H[s * Np + x.vM]);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) s_dF[(3 * s + j) * NFN + t] = dh * nv[j];
+            for (int s = 0; s < NA; ++s) Hp[s] = fma(R(-0.5), s_H[s * Np + x.vM], Hp[s]);
         }
+        const R w = (x.fside ? R(1) : R(-1)) * KConst<R>::inv_w0(P);
+#pragma unroll
+        for (int s = 0; s < NA; ++s) s_dF[s * NFN + t] = w * Hp[s];
     }
     __syncthreads();
     chain_release();
@@ -271,9 +276,8 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
     using Ix = ShellIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp, GSTRIDE = KG_NFIELDS * Np;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R* const s_G = reinterpret_cast<R*>(smem_raw);  // [12][Np] gradients
-    R* const s_Ft = s_G + 12 * Np;                   // [3][4][Np] J dxi_d/dx . grad G_s
-    R* const s_dF = s_Ft + 12 * Np;                  // [4][NFN] lifted face terms
+    R* const s_Ft = reinterpret_cast<R*>(smem_raw);  // [3][4][Np] J dxi_d/dx . grad G_s
+    R* const s_dF = s_Ft + 12 * Np;                   // [4][NFN] face terms, over 1/J
     R* const s_Dh = s_dF + 4 * NFN;                  // weak-form Dhat
 
     const int e = blockIdx.x, t = threadIdx.x;
@@ -287,10 +291,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
         const R* gn = hg + (size_t)e * 12 * Np + t;
         R G[12];
 #pragma unroll
-        for (int w = 0; w < 12; ++w) {
-            G[w] = gn[w * Np];
-            s_G[w * Np + t] = G[w];
-        }
+        for (int w = 0; w < 12; ++w) G[w] = gn[w * Np];
         R Jx[9];
 #pragma unroll
         for (int w = 0; w < 9; ++w) Jx[w] = ge[(KG_JXI + w) * Np + t];
@@ -312,19 +313,16 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
     __syncthreads();
 
     if (x.face) {
-        R nv[3];
-        R lift = shell_face_normal<R>(P, ge, Np, x.fd, x.fside ? R(1) : R(-1), x.vM, nv);
-        if (P.hyper_horizontal && x.fd == 2) lift = R(0);  // HorizontalDirection: no terms on the xi3 faces
+        // the far side's half of the central penalty (KParams::DhatC), with
+        // vMI sM n = +-(J dxi_fd/dx) / (J w_0)
+        const R j0 = ge[(KG_JXI + x.fd * 3 + 0) * Np + x.vM];
+        const R j1 = ge[(KG_JXI + x.fd * 3 + 1) * Np + x.vM];
+        const R j2 = ge[(KG_JXI + x.fd * 3 + 2) * Np + x.vM];
+        const R w = (x.fside ? R(0.5) : R(-0.5)) * KConst<R>::inv_w0(P);
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            R acc = 0;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                const R Gm = s_G[(3 * s + j) * Np + x.vM];
-                acc += ((nb >= 0 ? Gp[3 * s + j] : Gm) + Gm) * (nv[j] / R(2));
-            }
-            s_dF[s * NFN + t] = lift * acc;
-        }
+        for (int s = 0; s < 4; ++s)
+            s_dF[s * NFN + t] = w * (nb >= 0 ? j0 * Gp[3 * s + 0] + j1 * Gp[3 * s + 1] + j2 * Gp[3 * s + 2]
+                                             : s_Ft[(x.fd * 4 + s) * Np + x.vM]);
     }
     __syncthreads();
     chain_release();
@@ -332,34 +330,36 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
     if (x.node) {
         R a[4] = {0, 0, 0, 0}, av[4] = {0, 0, 0, 0};
         const int L1 = Nq * (x.nj + Nq * x.nk), L2 = x.ni + Nfp * x.nk, L3 = x.ni + Nq * x.nj;
+        constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
-        for (int n = 0; n < Nq; ++n) {
-            const R d1 = s_Dh[x.ni * Nq + n], d2 = s_Dh[x.nj * Nq + n], d3 = s_Dh[x.nk * Nq + n];
+        for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+            const int n1 = SKIP ? others(n, x.ni) : n, n2 = SKIP ? others(n, x.nj) : n, n3 = SKIP ? others(n, x.nk) : n;
+            const R d1 = s_Dh[x.ni * Nq + n1], d2 = s_Dh[x.nj * Nq + n2], d3 = s_Dh[x.nk * Nq + n3];
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
-                a[s] = fma(d1, s_Ft[(0 * 4 + s) * Np + L1 + n], fma(d2, s_Ft[(1 * 4 + s) * Np + L2 + n * Nq], a[s]));
-                av[s] = fma(d3, s_Ft[(2 * 4 + s) * Np + L3 + n * Nfp], av[s]);
+                a[s] = fma(d1, s_Ft[(0 * 4 + s) * Np + L1 + n1], fma(d2, s_Ft[(1 * 4 + s) * Np + L2 + n2 * Nq], a[s]));
+                av[s] = fma(d3, s_Ft[(2 * 4 + s) * Np + L3 + n3 * Nfp], av[s]);
             }
         }
-        if (!P.hyper_horizontal) {
-#pragma unroll
-            for (int s = 0; s < 4; ++s) a[s] += av[s];
-        }
-        const R iJ = ge[KG_INVJ * Np + t];
-        R lap[4];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) lap[s] = -iJ * a[s];
         auto add = [&](int ff) {
             const int idx = ff * Nfp + x.on_face(ff);
 #pragma unroll
-            for (int s = 0; s < 4; ++s) lap[s] += s_dF[s * NFN + idx];
+            for (int s = 0; s < 4; ++s) a[s] -= s_dF[s * NFN + idx];
         };
         if (x.ni == 0) add(0);
         if (x.ni == N) add(1);
         if (x.nj == 0) add(2);
         if (x.nj == N) add(3);
-        if (x.nk == 0) add(4);
-        if (x.nk == N) add(5);
+        if (!P.hyper_horizontal) {  // HorizontalDirection: no xi3 terms
+#pragma unroll
+            for (int s = 0; s < 4; ++s) a[s] += av[s];
+            if (x.nk == 0) add(4);
+            if (x.nk == N) add(5);
+        }
+        const R iJ = ge[KG_INVJ * Np + t];
+        R lap[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) lap[s] = -iJ * a[s];
         R* o = hl + (size_t)e * 4 * Np + t;
 #pragma unroll
         for (int s = 0; s < 4; ++s) o[s * Np] = lap[s];
@@ -372,8 +372,8 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp, GSTRIDE = KG_NFIELDS * Np;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* const s_L = reinterpret_cast<R*>(smem_raw);  // [4][Np] laplacians
-    R* const s_dF = s_L + 4 * Np;                    // [12][NFN] lifted face terms
-    R* const s_D = s_dF + 12 * NFN;                  // strong-form D
+    R* const s_dF = s_L + 4 * Np;                    // [4][NFN] face terms of the reference derivatives
+    R* const s_D = s_dF + 4 * NFN;                   // strong-form D
 
     const int e = blockIdx.x, t = threadIdx.x;
     const Ix x(t);
@@ -398,15 +398,10 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
     __syncthreads();
 
     if (x.face) {
-        R nv[3];
-        R lift = shell_face_normal<R>(P, ge, Np, x.fd, x.fside ? R(1) : R(-1), x.vM, nv);
-        if (P.hyper_horizontal && x.fd == 2) lift = R(0);  // HorizontalDirection: no terms on the xi3 faces
+        // n (L+ - L-) / (2 w_0), without what the diagonal of D leaves out
+        const R w = (x.fside ? R(0.5) : R(-0.5)) * KConst<R>::inv_w0(P);
 #pragma unroll
-        for (int s = 0; s < 4; ++s) {
-            const R dl = nb >= 0 ? lift * (Lp[s] - s_L[s * Np + x.vM]) / R(2) : R(0);
-#pragma unroll
-            for (int j = 0; j < 3; ++j) s_dF[(3 * s + j) * NFN + t] = dl * nv[j];
-        }
+        for (int s = 0; s < 4; ++s) s_dF[s * NFN + t] = w * (nb >= 0 ? Lp[s] : s_L[s * Np + x.vM]);
     }
     __syncthreads();
     chain_release();
@@ -428,9 +423,9 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
 template <int N, typename R, bool MIXED>
 cudaError_t launch_shell_passes_typed(const KParams& P, const void* Q, void* hd, void* hl, cudaStream_t s) {
     constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp, NFN = 6 * Nfp, NT = ShellDims<N>::NT;
-    constexpr size_t b1 = sizeof(R) * (planar_pad<R>(5 * Np) + 4 * Np + 12 * NFN + Nq * Nq);
-    constexpr size_t b2 = sizeof(R) * (24 * Np + 4 * NFN + Nq * Nq);
-    constexpr size_t b3 = sizeof(R) * (4 * Np + 12 * NFN + Nq * Nq);
+    constexpr size_t b1 = sizeof(R) * (4 * Np + 4 * NFN + Nq * Nq);
+    constexpr size_t b2 = sizeof(R) * (12 * Np + 4 * NFN + Nq * Nq);
+    constexpr size_t b3 = sizeof(R) * (4 * Np + 4 * NFN + Nq * Nq);
     cudaError_t e;
     if ((e = opt_in(shell_hyper_grad_kernel<N, R, MIXED>, b1)) != cudaSuccess) return e;
     if ((e = opt_in(shell_hyper_div_kernel<N, R>, b2)) != cudaSuccess) return e;
@@ -447,7 +442,7 @@ cudaError_t launch_shell_passes_typed(const KParams& P, const void* Q, void* hd,
 template <int N, typename R, bool MIXED, int NA, bool ARRAYS = false>
 cudaError_t launch_shell_visc_typed(const KParams& P, const void* Q, void* gout, cudaStream_t s) {
     constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp, NFN = 6 * Nfp, NT = ShellDims<N>::NT;
-    constexpr size_t b1 = sizeof(R) * (planar_pad<R>(5 * Np) + NA * Np + 3 * NA * NFN + Nq * Nq);
+    constexpr size_t b1 = sizeof(R) * (NA * Np + NA * NFN + Nq * Nq);
     cudaError_t e;
     if ((e = opt_in(shell_hyper_grad_kernel<N, R, MIXED, false, NA, ARRAYS>, b1)) != cudaSuccess) return e;
     return launch_chained(s, shell_hyper_grad_kernel<N, R, MIXED, false, NA, ARRAYS>, (unsigned)P.nelem, NT, b1, P, Q,

@@ -280,11 +280,13 @@ int init_model_tables(Model* md) {
     CMDG_CUDA_CHECK(cudaMemcpy(md->d_lvl64, md->lvl64.data(), sizeof(double) * md->lvl64.size(), cudaMemcpyHostToDevice));
     CMDG_CUDA_CHECK(cudaMemcpy(md->d_lvl32, md->lvl32.data(), sizeof(float) * md->lvl32.size(), cudaMemcpyHostToDevice));
     CMDG_CUDA_CHECK(cudaMemcpy(md->d_jump32, md->jump32.data(), sizeof(float) * md->jump32.size(), cudaMemcpyHostToDevice));
-    std::vector<float> dh32(m.Dhat.size());
-    for (size_t i = 0; i < dh32.size(); ++i) dh32[i] = (float)m.Dhat[i];
+    // the kernels' copies have a zero diagonal (KParams::Dhat)
+    std::vector<double> dh64(m.Dhat);
+    for (int i = 0; i < m.Nq; ++i) dh64[(size_t)i * m.Nq + i] = 0.0;
+    std::vector<float> dh32(dh64.begin(), dh64.end());
     CMDG_CUDA_CHECK(cudaMalloc(&md->d_Dhat64, sizeof(double) * m.Dhat.size()));
     CMDG_CUDA_CHECK(cudaMalloc(&md->d_Dhat32, sizeof(float) * dh32.size()));
-    CMDG_CUDA_CHECK(cudaMemcpy(md->d_Dhat64, m.Dhat.data(), sizeof(double) * m.Dhat.size(), cudaMemcpyHostToDevice));
+    CMDG_CUDA_CHECK(cudaMemcpy(md->d_Dhat64, dh64.data(), sizeof(double) * dh64.size(), cudaMemcpyHostToDevice));
     CMDG_CUDA_CHECK(cudaMemcpy(md->d_Dhat32, dh32.data(), sizeof(float) * dh32.size(), cudaMemcpyHostToDevice));
     return CMDG_OK;
 }

@@ -6,16 +6,17 @@
 //            its state and stages the contravariant fluxes
 //            Ft_d = J (dxi_d/dx) . F, d = 1..3, in shared memory, and forms
 //            the gravity source -rho grad(Phi) with the DG gradient of Phi;
-//   phase 2  every face node takes the outward normal n = +-J dxi_d/dx / |.|
-//            and surface Jacobian |J dxi_d/dx| of its own volume node, the
-//            interior normal flux F.n = +-Ft_d / |J dxi_d/dx| from phase 1,
-//            gathers the neighbour's state at the matching node (horizontal
-//            faces through the face-orientation code of the connectivity
-//            row; walls reflect the normal momentum,
-//            rho u+ = rho u- - 2 (rho u- . n) n), and stores the lifted
-//            Rusanov or central flux vMI sM F* = |J dxi_d/dx| / (J w_0) F*;
+//   phase 2  every face node gathers the neighbour's state at the matching
+//            node (horizontal faces through the face-orientation code of the
+//            connectivity row; walls reflect the normal momentum,
+//            rho u+ = rho u- - 2 (rho u- . n) n) and forms J times the lifted
+//            Rusanov or central flux vMI sM F* = |J dxi_d/dx| / (J w_0) F*
+//            with +-J dxi_d/dx of its own volume node in the place of
+//            |J dxi_d/dx| n, so that only the wavespeed needs the length; the
+//            interior half of the central part is left out with the diagonal
+//            of the derivative (KParams::DhatC);
 //   phase 3  every node contracts Ft_d with the weak-form derivative Dhat,
-//            scales by 1/J, subtracts its face terms, adds the source and
+//            subtracts its face terms, scales by 1/J, adds the source and
 //            finishes the tendency or the LSRK 2N stage update.
 // With M = J w_i w_j w_k this is M^-1 D^T M (dxi_d/dx . F) of
 // src/Numerics/DGMethods/DGModel_kernels.jl:64-548 and the interface term of
@@ -79,6 +80,11 @@ struct ShellSmem {
 // reference jump (c_L: the larger reference sound speed, the linear model's
 // Rusanov speed).  The stiff vertical acoustic terms are then applied in
 // FP64 by the linear kernel, so FP32 rounding no longer enters them.
+//
+// Measured with the normal formed, normalised and both halves summed, against
+// this form: the cubed-shell GCM step 149 / 145 us, FP64 945 / 737 us (8 x 8 x
+// 6 elements per panel, with the FP64 operations of dg_common.cuh), grid
+// arrays (the same phases in arrays.cu) 210 / 200 us.
 //
 // Resident CTAs per SM of the FP32 kernel: the inviscid one ShellDims'
 // MIN_CTAS; with hyperdiffusion alone at N = 4, 5 (72 registers; the mixed
@@ -241,19 +247,30 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
         const R j0 = ge[(KG_JXI + fd * 3 + 0) * Np + vM];
         const R j1 = ge[(KG_JXI + fd * 3 + 1) * Np + vM];
         const R j2 = ge[(KG_JXI + fd * 3 + 2) * Np + vM];
-        const R iJm = ge[KG_INVJ * Np + vM];
-        R sJ, rs;
-        sqrt_rsqrt_r(j0 * j0 + j1 * j1 + j2 * j2, sJ, rs);
-        rs *= sgn;
-        const R nv[3] = {j0 * rs, j1 * rs, j2 * rs};
-        R qm[NSTATE], Fm[NSTATE], qp[NSTATE], S[NSTATE], jr_rho = 0, jr_rhoe = 0;
+        // |J dxi_fd/dx| n = +-J dxi_fd/dx: the normal is never normalised.  The
+        // face terms below are over 1/J, which multiplies the sum of them and
+        // the volume term, and without the interior half of the central part,
+        // which is left out with the diagonal of the derivative
+        // (KParams::DhatC).
+        const R n2 = j0 * j0 + j1 * j1 + j2 * j2;
+        const R sJ = sqrt_r(n2);
+        R qm[NSTATE], qp[NSTATE], S[NSTATE], jr_rho = 0, jr_rhoe = 0;
         PL::ld(s_node, Np, vM, qm);
         const CRV cr = s_cr[vM];
-        const R c_m = cr.x, ri_m = cr.y;
-        PL::ld(s_F + fd * SM::P5N, Np, vM, Fm);
-        R am = rs;  // Fm = am times the staged contravariant flux (on some walls Fm is the normal flux, am = 1)
-        const R mn_m = qm[1] * nv[0] + qm[2] * nv[1] + qm[3] * nv[2];
-        const R lam_m = fabs(mn_m * ri_m) + c_m;
+        const R mn_m = qm[1] * j0 + qm[2] * j1 + qm[3] * j2;
+        const R lam_m = fma(cr.x, sJ, fabs(mn_m * cr.y));
+        R F1[NSTATE] = {0, 0, 0, 0, 0};  // what stays of the interior half on some walls
+        // J dxi_fd/dx . (first-order flux) of the interior side less the staged flux
+        auto first_less_staged = [&](const Level<R>& lvm) {
+            const Thermo<R, MIXED> thm = thermo<R, MIXED>(qm, lvm, P);
+            R Ft[NSTATE];
+            PL::ld(s_F + fd * SM::P5N, Np, vM, Ft);
+            F1[0] = mn_m - Ft[0];
+            F1[1] = mn_m * thm.u[0] + thm.pflux * j0 - Ft[1];
+            F1[2] = mn_m * thm.u[1] + thm.pflux * j1 - Ft[2];
+            F1[3] = mn_m * thm.u[2] + thm.pflux * j2 - Ft[3];
+            F1[4] = mn_m * thm.rinv * thm.H - Ft[4];
+        };
         const int nb = __ldg(nbr + f);
         int ezp = ez, kP = kM;
         const R* gp = ge;  // geometry of the node across the face (own node on a wall)
@@ -281,16 +298,15 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) qp[s] = qm[s];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) qp[1 + c] = qm[1 + c] - R(2) * mn_m * nv[c];
+            for (int c = 0; c < 3; ++c) qp[1 + c] = qm[1 + c];
+            const R refl = R(2) * mn_m * rcp_r(n2);
+            qp[1] -= refl * j0;
+            qp[2] -= refl * j1;
+            qp[3] -= refl * j2;
             if (HYPER || VISC) {
-                // the staged flux holds the second-order part too: walls take the first-order one
+                // the staged flux holds the second-order part too, walls take the first-order one
                 const Level<R> lvm = shell_level<R, MIXED>(P, ge, Np, vM, ez * Nq + kM);
-                const Thermo<R, MIXED> thm = thermo<R, MIXED>(qm, lvm, P);
-                am = R(1);
-                Fm[0] = mn_m;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) Fm[1 + c] = mn_m * thm.u[c] + thm.pflux * nv[c];
-                Fm[4] = mn_m * thm.rinv * thm.H;
+                first_less_staged(lvm);
             }
         }
         Level<R> lvp = load_level<R>(P, ezp * Nq + kP);
@@ -311,13 +327,18 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
             }
         }
         const Thermo<R, MIXED> thp = thermo<R, MIXED, false>(qp, lvp, P);
-        const R mn_p = qp[1] * nv[0] + qp[2] * nv[1] + qp[3] * nv[2];
+        const R jv[3] = {j0, j1, j2};
+        const R mn_p = qp[1] * j0 + qp[2] * j1 + qp[3] * j2;
         const R un_p = mn_p * thp.rinv;
-        // S: the two sides' normal fluxes added up
-        S[0] = fma(am, Fm[0], mn_p);
+        // J dxi_fd/dx . (flux of the far side)
+        S[0] = mn_p;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) S[1 + c] = fma(am, Fm[1 + c], fma(un_p, qp[1 + c], thp.pflux * nv[c]));
-        S[4] = fma(am, Fm[4], un_p * thp.H);
+        for (int c = 0; c < 3; ++c) S[1 + c] = fma(un_p, qp[1 + c], thp.pflux * jv[c]);
+        S[4] = un_p * thp.H;
+        if (VISC || HYPER) {
+#pragma unroll
+            for (int s = 0; s < NSTATE; ++s) S[s] += F1[s];
+        }
         R cL = 0;  // REM, faces normal to xi3: the linear model's Rusanov speed
         if (REM && fd == 2) {
             // F - F_L of the node across the face (or of the reflected state on a wall)
@@ -325,10 +346,10 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
                 KConst<R>::gm1(P) * R(0.5) * ((qp[1] * qp[1] + qp[2] * qp[2] + qp[3] * qp[3]) * thp.rinv);
             const R hrem_p =
                 ((qp[4] + thp.pflux) * lvp.rho_ref - lvp.href * qp[0]) * thp.rinv * rcp_r(lvp.rho_ref);
-            S[0] = am * Fm[0];
+            S[0] = 0;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) S[1 + c] = fma(am, Fm[1 + c], fma(un_p, qp[1 + c], -(pke_p * nv[c])));
-            S[4] = fma(am, Fm[4], mn_p * hrem_p);
+            for (int c = 0; c < 3; ++c) S[1 + c] = fma(un_p, qp[1 + c], -(pke_p * jv[c]));
+            S[4] = mn_p * hrem_p;
             const Level<R> lvm = shell_level<R, MIXED>(P, ge, Np, vM, ez * Nq + kM);
             const R gam = KConst<R>::gamma(P);
             cL = fmax(sqrt_r(gam * lvm.p_ref * rcp_r(lvm.rho_ref)), sqrt_r(gam * lvp.p_ref * rcp_r(lvp.rho_ref)));
@@ -339,7 +360,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
             R hn_n[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c)
-                hn_n[c] = nv[0] * hn[(3 * c + 0) * Np] + nv[1] * hn[(3 * c + 1) * Np] + nv[2] * hn[(3 * c + 2) * Np];
+                hn_n[c] = j0 * hn[(3 * c + 0) * Np] + j1 * hn[(3 * c + 1) * Np] + j2 * hn[(3 * c + 2) * Np];
             const R rho_p = MIXED ? lvp.rho_ref + qp[0] : qp[0];
 #pragma unroll
             for (int c = 0; c < 3; ++c) S[1 + c] += rho_p * hn_n[c];
@@ -350,14 +371,13 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
             R Fv[3][NSTATE];
             shell_visc_flux<R, MIXED, VT>(P, nb, vP, Np, qp, lvp, thp.rinv, Fv);
 #pragma unroll
-            for (int s2 = 0; s2 < NSTATE; ++s2) S[s2] += nv[0] * Fv[0][s2] + nv[1] * Fv[1][s2] + nv[2] * Fv[2][s2];
+            for (int s2 = 0; s2 < NSTATE; ++s2) S[s2] += j0 * Fv[0][s2] + j1 * Fv[1][s2] + j2 * Fv[2][s2];
         }
-        const R lam_p = fabs(un_p) + thp.c;
-        const R lift = sJ * iJm * KConst<R>::inv_w0(P);
-        const R hl = R(0.5) * lift;
-        const R pl = (ph.numflux == CMDG_FLUX_RUSANOV) ? hl * max_nonneg(lam_m, lam_p) : R(0);
+        const R lam_p = fma(thp.c, sJ, fabs(un_p));
+        const R hw = R(0.5) * KConst<R>::inv_w0(P), hl = sgn * hw;
+        const R pl = (ph.numflux == CMDG_FLUX_RUSANOV) ? hw * max_nonneg(lam_m, lam_p) : R(0);
         // REM: the linear model's penalty cL/2 on the perturbation jump comes off
-        const R pq = (REM && fd == 2) ? pl - hl * cL : pl;
+        const R pq = (REM && fd == 2) ? pl - hw * (sJ * cL) : pl;
         R fs[NSTATE];
         if constexpr (MIXED) {
 #pragma unroll
@@ -377,24 +397,23 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     if (node_thread) {
         R acc[NSTATE] = {0, 0, 0, 0, 0};
         const int L1 = Nq * (nj + Nq * nk), L2 = ni + Nfp * nk, L3 = ni + Nq * nj;
+        constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
-        for (int n = 0; n < Nq; ++n) {
+        for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+            const int n1 = SKIP ? others(n, ni) : n, n2 = SKIP ? others(n, nj) : n, n3 = SKIP ? others(n, nk) : n;
             R v1[NSTATE], v2[NSTATE], v3[NSTATE];
-            PL::ld(s_F, Np, L1 + n, v1);
-            PL::ld(s_F + SM::P5N, Np, L2 + n * Nq, v2);
-            PL::ld(s_F + 2 * SM::P5N, Np, L3 + n * Nfp, v3);
-            const R d1 = s_D[ni * Nq + n], d2 = s_D[nj * Nq + n], d3 = s_D[nk * Nq + n];
+            PL::ld(s_F, Np, L1 + n1, v1);
+            PL::ld(s_F + SM::P5N, Np, L2 + n2 * Nq, v2);
+            PL::ld(s_F + 2 * SM::P5N, Np, L3 + n3 * Nfp, v3);
+            const R d1 = s_D[ni * Nq + n1], d2 = s_D[nj * Nq + n2], d3 = s_D[nk * Nq + n3];
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) acc[s] = fma(d1, v1[s], fma(d2, v2[s], fma(d3, v3[s], acc[s])));
         }
-        R rhs[NSTATE];
-#pragma unroll
-        for (int s = 0; s < NSTATE; ++s) rhs[s] = invJ * acc[s];
         auto sub_face = [&](int ff, int idx) {
             R v[NSTATE];
             PL::ld(s_fs, NFN, ff * Nfp + idx, v);
 #pragma unroll
-            for (int s = 0; s < NSTATE; ++s) rhs[s] -= v[s];
+            for (int s = 0; s < NSTATE; ++s) acc[s] -= v[s];
         };
         if (ni == 0) sub_face(0, nj + Nq * nk);
         if (ni == N) sub_face(1, nj + Nq * nk);
@@ -402,6 +421,9 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
         if (nj == N) sub_face(3, ni + Nq * nk);
         if (nk == 0) sub_face(4, ni + Nq * nj);
         if (nk == N) sub_face(5, ni + Nq * nj);
+        R rhs[NSTATE];
+#pragma unroll
+        for (int s = 0; s < NSTATE; ++s) rhs[s] = invJ * acc[s];
 #pragma unroll
         for (int c = 0; c < 3; ++c) rhs[1 + c] += src[c];
         const R rkb_dt = KConst<R>::rkb_dt(P);

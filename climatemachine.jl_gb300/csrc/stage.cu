@@ -6,7 +6,9 @@
 //            directions and stages them in shared memory;
 //   phase 2  every face node (6 (N+1)^2 of them) gathers the neighbour's
 //            state at the matching node, forms the Rusanov (or central)
-//            flux F*.n and stores it lifted, vMI*sM*F*, in shared memory;
+//            flux F*.n and stores it lifted, vMI*sM*F*, in shared memory
+//            (without the interior half of its central part, which cancels
+//            against the diagonal of the derivative: KParams::DhatC);
 //   phase 3  every node contracts the staged fluxes with the weak-form
 //            derivative Dhat = M^-1 D^T M along xi1, xi2, xi3, subtracts its
 //            face terms, adds gravity and finishes either the tendency
@@ -42,10 +44,12 @@
 //
 // The FP64 form is bound by the FP64 pipe (1.8 lane operations per cycle and
 // SM), so its operations are counted: reciprocals and roots of 3 and 5
-// operations (rcp_r, sqrt_r), one FMA per field for the sum of a face's two
-// fluxes, the metric folded into the derivative coefficients, comparisons on
-// the integer pipe.  About 240 operations per node became 185 and a step of
-// the 1 M-node bubble went from 2.304 to 1.852 ms.
+// operations (rcp_r, sqrt_r), the metric folded into the derivative
+// coefficients, no diagonal in the contraction, comparisons on the integer
+// pipe.  A step of the 1 M-node bubble went from 2.304 to 1.677 ms (1.852 ms
+// before the diagonal, and chained launches, launch.cuh).  In FP32 the same
+// identity saves the face threads five loads and ten operations (0.167 to
+// 0.164 ms).
 #include <cooperative_groups.h>
 
 #include "dg_common.cuh"
@@ -400,15 +404,10 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
 
         // ---------------- phase 2: one numerical flux per face node
         if (face_thread) {
-            R qm[NSTATE], Fm[NSTATE], Fp[NSTATE], S[NSTATE], qp[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
+            R qm[NSTATE], Fp[NSTATE], qp[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
             PL::ld(s_node, Np, vM, qm);
             const CRV cr = s_cr[vM];
             const R c_m = cr.x, ri_m = cr.y;
-            PL::ld(s_F + fd * SM::P5N, Np, fside * N * Nfp + fn, Fm);  // dir_rec(fd) of vM
-            if (MIXED) {
-#pragma unroll
-                for (int s = 0; s < NSTATE; ++s) Fm[s] *= sgn;
-            }
             const R lam_m = fabs(pick3(fd, qm[1], qm[2], qm[3]) * ri_m) + c_m;
             int ezp = ez;
             if (cur.nb >= 0) {
@@ -444,36 +443,31 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
                 PL::ld(cl.map_shared_rank(s_node, (unsigned)nrank), Np, vP, qp);
                 const CRV crp = cl.map_shared_rank(s_cr, (unsigned)nrank)[vP];
                 PL::ld(cl.map_shared_rank(s_F + fd * SM::P5N, (unsigned)nrank), Np, oside * N * Nfp + fn, Fp);
-#pragma unroll
-                for (int s = 0; s < NSTATE; ++s) {
-                    if (MIXED) Fp[s] *= sgn;
-                    else S[s] = Fm[s] + Fp[s];
-                }
                 lam_p = fabs(pick3(fd, qp[1], qp[2], qp[3]) * crp.y) + crp.x;
             } else {
                 const Level<R> lvp = load_level<R>(P, ezp * Nq + (cur.nb >= 0 ? kP : kM));
                 const Thermo<R, MIXED> thp = thermo<R, MIXED, MIXED>(qp, lvp, P);
                 if (MIXED) {
-                    normal_flux<R, MIXED>(qp, thp, fd, sgn, Fp);
+                    normal_flux<R, MIXED>(qp, thp, fd, R(1), Fp);
                     lam_p = fabs(pick3(fd, thp.u[0], thp.u[1], thp.u[2])) + thp.c;
                 } else {
                     const R mn = pick3(fd, qp[1], qp[2], qp[3]);
                     const R un = mn * thp.rinv;
-                    add_flux_d<R, MIXED>(Fm, qp, mn, un, thp.pflux, thp.H, fd, S);
+                    far_flux_d<R>(qp, mn, un, thp.pflux, thp.H, fd, Fp);
                     lam_p = fabs(un) + thp.c;
                 }
             }
+            // the central part's interior half is left out with the diagonal
+            // of the derivative (KParams::DhatC)
             const R lift = pick3(fd, xi[0], xi[1], xi[2]) * KConst<R>::inv_w0(P);
             const R hmw = (ph.numflux == CMDG_FLUX_RUSANOV) ? R(0.5) * max_nonneg(lam_m, lam_p) : R(0);
-            const R hl = R(0.5) * lift, pl = hmw * lift;
+            const R hl = (R(0.5) * sgn) * lift, pl = hmw * lift;
             R fs[NSTATE];
             if (MIXED) {
-                // FP32: the fluxes with the face's sign; the FP64 form below
-                // measured 3.8% slower here at N = 5 and the same at N = 4
 #pragma unroll
-                for (int s = 0; s < NSTATE; ++s) fs[s] = hl * (Fm[s] + Fp[s]) + pl * ((qm[s] - qp[s]) + jr[s]);
+                for (int s = 0; s < NSTATE; ++s) fs[s] = hl * Fp[s] + pl * ((qm[s] - qp[s]) + jr[s]);
             } else {
-                lifted_flux<R, MIXED>(S, qm, qp, R(0), R(0), sgn * hl, pl, fs);
+                lifted_flux<R, MIXED>(Fp, qm, qp, R(0), R(0), hl, pl, fs);
             }
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) s_fs[(fd * NSTATE + s) * Np + vM] = fs[s];
@@ -494,13 +488,16 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
             const int L3 = ni + Nq * nj;         // line along xi3 (stride Nfp)
             R acc1[NSTATE] = {0, 0, 0, 0, 0}, acc2[NSTATE] = {0, 0, 0, 0, 0}, acc3[NSTATE] = {0, 0, 0, 0, 0};
 #pragma unroll
-            for (int n = 0; n < Nq; ++n) {
+            for (int n = 0; n < (SCALED_D ? N : Nq); ++n) {
+                const int n1 = SCALED_D ? others(n, ni) : n, n2 = SCALED_D ? others(n, nj) : n,
+                          n3 = SCALED_D ? others(n, nk) : n;
                 R v1[NSTATE], v2[NSTATE], v3[NSTATE];
-                PL::ld(s_F, Np, L1 + n * Nfp, v1);
-                PL::ld(s_F + SM::P5N, Np, L2 + n * Nfp, v2);
-                PL::ld(s_F + 2 * SM::P5N, Np, L3 + n * Nfp, v3);
+                PL::ld(s_F, Np, L1 + n1 * Nfp, v1);
+                PL::ld(s_F + SM::P5N, Np, L2 + n2 * Nfp, v2);
+                PL::ld(s_F + 2 * SM::P5N, Np, L3 + n3 * Nfp, v3);
                 if constexpr (SCALED_D) {
-                    const R d1 = s_D[ni * Nq + n], d2 = s_D[Nq * Nq + nj * Nq + n], d3 = s_D[2 * Nq * Nq + nk * Nq + n];
+                    const R d1 = s_D[ni * Nq + n1], d2 = s_D[Nq * Nq + nj * Nq + n2],
+                            d3 = s_D[2 * Nq * Nq + nk * Nq + n3];
 #pragma unroll
                     for (int s = 0; s < NSTATE; ++s) {
                         acc1[s] = fma(d1, v1[s], acc1[s]);
@@ -776,9 +773,10 @@ KParams make_params(Model* md, const LaunchArgs& a) {
     P.gamma32 = (float)md->ph.gamma;
     P.ph = md->ph;
     for (int i = 0; i < (MAX_N + 1) * (MAX_N + 1); ++i) {
-        P.DhatC64[i] = i < (int)m.Dhat.size() ? m.Dhat[i] : 0.0;
+        const bool diag = i % (m.Nq + 1) == 0;
+        P.DhatC64[i] = i < (int)m.Dhat.size() && !diag ? m.Dhat[i] : 0.0;
         P.DhatC32[i] = (float)P.DhatC64[i];
-        P.DC64[i] = i < (int)m.D.size() ? m.D[i] : 0.0;
+        P.DC64[i] = i < (int)m.D.size() && !diag ? m.D[i] : 0.0;
         P.DC32[i] = (float)P.DC64[i];
     }
     P.gf = md->d_gf;

@@ -5,7 +5,7 @@
 // threads (TPE >= the element's 3 (N+1)^2 lines; a thread owns NPT nodes):
 //   phase 1  every node thread loads its state (coalesced), evaluates the dry
 //            AtmosModel thermodynamics, and stores in shared memory its
-//            state, (c, 1/rho, pressure of the momentum flux, rhoe + p) and
+//            state, (c, 1/rho) and
 //            its three directional first-order fluxes, each already scaled by
 //            the element's metric 2/dx_d;
 //   phase 2  each of the 3 (N+1)^2 element lines (xi_d line L) is one thread:
@@ -74,7 +74,7 @@ struct LSplit {
 };
 
 // node-major scalar planes of Np words per element: 15 directional fluxes
-// (d major, field minor), 5 state fields, 4 auxiliary values per node
+// (d major, field minor), 5 state fields, 2 auxiliary values per node
 template <int N, typename R>
 struct LSmem {
     static constexpr int Np = LDims<N>::Np;
@@ -82,10 +82,10 @@ struct LSmem {
     static constexpr int FLUX = 0;
     static constexpr int NODE = FLUX + 15 * PS;
     static constexpr int AUX = NODE + 5 * PS;
-    static constexpr int TOTAL = AUX + 4 * PS;  // words per element
+    static constexpr int TOTAL = AUX + 2 * PS;  // words per element
     static constexpr size_t BYTES = sizeof(R) * TOTAL;
 };
-enum { AUX_C = 0, AUX_RINV = 1, AUX_PFLUX = 2, AUX_H = 3 };
+enum { AUX_C = 0, AUX_RINV = 1 };
 
 // Weak-form derivative coefficients with compile-time indices, read from a
 // kernel parameter (the constant bank): a model's own launch parameters, or,
@@ -197,8 +197,6 @@ __device__ __forceinline__ int lines_element(const KParams& P, const DH& dhat, R
             for (int s = 0; s < NSTATE; ++s) s_q[s * PS + node] = q[k][s];
             s_a[AUX_C * PS + node] = th.c;
             s_a[AUX_RINV * PS + node] = th.rinv;
-            s_a[AUX_PFLUX * PS + node] = th.pflux;
-            s_a[AUX_H * PS + node] = th.H;
 #pragma unroll
             for (int dd = 0; dd < 3; ++dd)
 #pragma unroll
@@ -222,21 +220,10 @@ __device__ __forceinline__ int lines_element(const KParams& P, const DH& dhat, R
             const int vM = side ? vM1 : vM0;
             const int nb = side ? nb1 : nb0;
             const R sgn = side ? R(1) : R(-1);
-            R qm[NSTATE], qp[NSTATE], Fm[NSTATE], Fp[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
+            R qm[NSTATE], qp[NSTATE], Fp[NSTATE], jr[NSTATE] = {0, 0, 0, 0, 0};
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) qm[s] = s_q[s * PS + vM];
             const R c_m = s_a[AUX_C * PS + vM], ri_m = s_a[AUX_RINV * PS + vM];
-            const R pf_m = s_a[AUX_PFLUX * PS + vM], H_m = s_a[AUX_H * PS + vM];
-            // minus-side normal flux sgn F_d from the staged state
-            {
-                const R mn = pick3(ld, qm[1], qm[2], qm[3]);
-                const R un = mn * ri_m;
-                Fm[0] = sgn * mn;
-                Fm[1] = sgn * (mn * (qm[1] * ri_m) + (ld == 0 ? pf_m : R(0)));
-                Fm[2] = sgn * (mn * (qm[2] * ri_m) + (ld == 1 ? pf_m : R(0)));
-                Fm[3] = sgn * (mn * (qm[3] * ri_m) + (ld == 2 ? pf_m : R(0)));
-                Fm[4] = sgn * (un * H_m);
-            }
             const R lam_m = fabs(pick3(ld, qm[1], qm[2], qm[3]) * ri_m) + c_m;
             int ezp = ez;
             const int kM = side ? kM1 : kM0;
@@ -273,7 +260,7 @@ __device__ __forceinline__ int lines_element(const KParams& P, const DH& dhat, R
             const R hl = R(0.5) * lift, pl = hmw * lift;
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) {
-                const R v = hl * (Fm[s] + Fp[s]) + pl * ((qm[s] - qp[s]) + jr[s]);
+                const R v = hl * Fp[s] + pl * ((qm[s] - qp[s]) + jr[s]);  // far side only (KParams::DhatC)
                 if (side) fs1[s] = v;
                 else fs0[s] = v;
             }

@@ -53,8 +53,7 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
     constexpr int ESTRIDE = NSTATE * Np;
     using PL = Planar5<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    R* const s_q = reinterpret_cast<R*>(smem_raw);      // planar records: states
-    R* const s_G = s_q + planar_pad<R>(5 * Np);            // gradient arguments
+    R* const s_G = reinterpret_cast<R*>(smem_raw);         // planar records: gradient arguments
     R* const s_dG = s_G + planar_pad<R>(5 * Np);           // face terms
     // strong-form D in shared memory: each thread indexes it by its own node
     // coordinates, which from the parameter bank would be divergent
@@ -86,17 +85,26 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) q[s] = qe[s * Np];
     }
+    // the node across the face; on a wall the face's own node with the
+    // FreeSlip state of the gradient flux, rhou+ = rhou- - (rhou-.n) n
+    const bool wall = nb < 0;
     int levp = ez * Nq + vM / Nfp;
-    if (nb >= 0) {
-        const R* qn = Qin + (size_t)nb * ESTRIDE + vP;
+    if (face_thread) {
+        const R* qn = Qin + (size_t)(wall ? e : nb) * ESTRIDE + (wall ? vM : vP);
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) qp[s] = qn[s * Np];
-        int ezp = ez;
-        if (fd == 2) {
-            ezp = ez + (fside ? 1 : -1);
-            ezp = ezp < 0 ? ezp + P.nz : (ezp >= P.nz ? ezp - P.nz : ezp);
+        if (wall) {
+            qp[1] = fd == 0 ? R(0) : qp[1];
+            qp[2] = fd == 1 ? R(0) : qp[2];
+            qp[3] = fd == 2 ? R(0) : qp[3];
+        } else {
+            int ezp = ez;
+            if (fd == 2) {
+                ezp = ez + (fside ? 1 : -1);
+                ezp = ezp < 0 ? ezp + P.nz : (ezp >= P.nz ? ezp - P.nz : ezp);
+            }
+            levp = ezp * Nq + vP / Nfp;
         }
-        levp = ezp * Nq + vP / Nfp;
     }
     const R xi[3] = {KConst<R>::metric(P, e, 0), KConst<R>::metric(P, e, 1), KConst<R>::metric(P, e, 2)};
 
@@ -105,35 +113,27 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
         const int lev = ez * Nq + nk;
         R G[5];
         grad_args<R, MIXED, SMAG>(P, q, load_level<R>(P, lev), load_vlevel<R>(P, lev), G);
-        PL::st(s_q, Np, t, q);
         PL::st(s_G, Np, t, G);
     }
     __syncthreads();
 
-    // phase 2: face terms lift n (G+ - G-) c, c = 1/2 inside, 1 on walls
+    // phase 2: face terms lift n (G+ - G-) c, c = 1/2 inside, 1 on walls, as
+    // an addition to the derivative along xi_fd and without what the diagonal
+    // of D leaves out (KParams::DC): n G+ / (2 w_0) inside,
+    // n (G+ - G- / 2) / w_0 on walls
     if (face_thread) {
-        R Gm[5], Gp[5];
-        PL::ld(s_G, Np, vM, Gm);
-        R c;
-        if (nb >= 0) {
-            grad_args<R, MIXED, SMAG>(P, qp, load_level<R>(P, levp), load_vlevel<R>(P, levp), Gp);
-            c = R(0.5);
-        } else {
-            // FreeSlip state for the gradient flux: rhou+ = rhou- - (rhou-.n) n
-            R qb[NSTATE];
-            PL::ld(s_q, Np, vM, qb);
-            qb[1 + 0] = fd == 0 ? R(0) : qb[1];
-            qb[1 + 1] = fd == 1 ? R(0) : qb[2];
-            qb[1 + 2] = fd == 2 ? R(0) : qb[3];
-            grad_args<R, MIXED, SMAG>(P, qb, load_level<R>(P, levp), load_vlevel<R>(P, levp), Gp);
-            c = R(1);
-        }
-        const R sgn = fside ? R(1) : R(-1);
-        const R w = c * sgn * pick3(fd, xi[0], xi[1], xi[2]) * KConst<R>::inv_w0(P);
-        R out[5];
+        R Gp[5];
+        grad_args<R, MIXED, SMAG>(P, qp, load_level<R>(P, levp), load_vlevel<R>(P, levp), Gp);
+        if (wall) {
+            R Gm[5];
+            PL::ld(s_G, Np, vM, Gm);
 #pragma unroll
-        for (int g = 0; g < 5; ++g) out[g] = w * (Gp[g] - Gm[g]);
-        PL::st(s_dG, NFN, f * Nfp + fn, out);
+            for (int g = 0; g < 5; ++g) Gp[g] = R(2) * Gp[g] - Gm[g];
+        }
+        const R w = (fside ? R(0.5) : R(-0.5)) * KConst<R>::inv_w0(P);
+#pragma unroll
+        for (int g = 0; g < 5; ++g) Gp[g] *= w;
+        PL::st(s_dG, NFN, f * Nfp + fn, Gp);
     }
     __syncthreads();
 
@@ -143,25 +143,21 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
     if (node_thread) {
         R g1[5] = {0, 0, 0, 0, 0}, g2[5] = {0, 0, 0, 0, 0}, g3[5] = {0, 0, 0, 0, 0};
         const int L1 = Nq * (nj + Nq * nk), L2 = ni + Nfp * nk, L3 = ni + Nq * nj;
+        constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
-        for (int n = 0; n < Nq; ++n) {
+        for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+            const int n1 = SKIP ? others(n, ni) : n, n2 = SKIP ? others(n, nj) : n, n3 = SKIP ? others(n, nk) : n;
             R v1[5], v2[5], v3[5];
-            PL::ld(s_G, Np, L1 + n, v1);
-            PL::ld(s_G, Np, L2 + n * Nq, v2);
-            PL::ld(s_G, Np, L3 + n * Nfp, v3);
-            const R d1 = s_D[ni * Nq + n], d2 = s_D[nj * Nq + n], d3 = s_D[nk * Nq + n];
+            PL::ld(s_G, Np, L1 + n1, v1);
+            PL::ld(s_G, Np, L2 + n2 * Nq, v2);
+            PL::ld(s_G, Np, L3 + n3 * Nfp, v3);
+            const R d1 = s_D[ni * Nq + n1], d2 = s_D[nj * Nq + n2], d3 = s_D[nk * Nq + n3];
 #pragma unroll
             for (int g = 0; g < 5; ++g) {
                 g1[g] = fma(d1, v1[g], g1[g]);
                 g2[g] = fma(d2, v2[g], g2[g]);
                 g3[g] = fma(d3, v3[g], g3[g]);
             }
-        }
-#pragma unroll
-        for (int g = 0; g < 5; ++g) {
-            g1[g] *= xi[0];
-            g2[g] *= xi[1];
-            g3[g] *= xi[2];
         }
         auto add = [&](int ff, int idx, R* gd) {
             R v[5];
@@ -175,6 +171,12 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
         if (nj == N) add(3, ni + Nq * nk, g2);
         if (nk == 0) add(4, ni + Nq * nj, g3);
         if (nk == N) add(5, ni + Nq * nj, g3);
+#pragma unroll
+        for (int g = 0; g < 5; ++g) {
+            g1[g] *= xi[0];
+            g2[g] *= xi[1];
+            g3[g] *= xi[2];
+        }
         const int lev = ez * Nq + nk;
         const VLevel<R> vv = load_vlevel<R>(P, lev);
         R thv = 0;
@@ -225,7 +227,7 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
 template <int N, typename R, bool MIXED, bool SMAG, bool FLUX>
 cudaError_t launch_grad_kernel(const KParams& P, const void* Q, void* gf, cudaStream_t s) {
     constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp;
-    constexpr size_t bytes = sizeof(R) * (2 * planar_pad<R>(5 * Np) + planar_pad<R>(30 * Nfp) + Nq * Nq);
+    constexpr size_t bytes = sizeof(R) * (planar_pad<R>(5 * Np) + planar_pad<R>(30 * Nfp) + Nq * Nq);
     auto k = gradient_kernel<N, R, MIXED, SMAG, FLUX>;
     cudaError_t e;
     if ((e = opt_in(k, bytes)) != cudaSuccess) return e;

@@ -354,46 +354,59 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
 
     // phase 2: numerical flux per face node (Rusanov/central + central second order)
     if (face_thread) {
-        R qm[NSTATE], Fm[NSTATE], S[NSTATE], jr_rho = 0, jr_rhoe = 0;
+        R qm[NSTATE], S[NSTATE], jr_rho = 0, jr_rhoe = 0;
         PL::ld(s_node, Np, vM, qm);
         const CRV cr = s_cr[vM];
         const R c_m = cr.x, ri_m = cr.y;
         const R lam_m = fabs(pick3(fd, qm[1], qm[2], qm[3]) * ri_m) + c_m;
-        const Level<R> lvm = load_level<R>(P, ez * Nq + vM / Nfp);
+        // The far side's flux; the interior half of the central part is left
+        // out with the diagonal of the derivative (KParams::DhatC).  Walls
+        // carry the first-order flux on both sides, but the diagonal leaves
+        // out the total one: there the node's own second-order part comes off.
+        R ux, uy;  // momentum of the node whose hyperdiffusive flux is taken
         if (nb >= 0) {
-            PL::ld(s_F + fd * P5N, Np, fside * N * Nfp + fn, Fm);  // dir_rec(fd) of vM
             if (MIXED && fd == 2 && ph.numflux == CMDG_FLUX_RUSANOV) {
                 const int ej = fside ? ezp : ez;
                 const R sj = fside ? R(-1) : R(1);
                 jr_rho = sj * (R)P.jump32[2 * ej + 0];
                 jr_rhoe = sj * (R)P.jump32[2 * ej + 1];
             }
+            ux = qp[1];
+            uy = qp[2];
         } else {
-            // walls: first-order flux only on both sides
-            const Thermo<R, MIXED> thm = thermo<R, MIXED>(qm, lvm, P);
-            normal_flux<R, MIXED>(qm, thm, fd, R(1), Fm);
+            // Impenetrable(FreeSlip): rhou+ = rhou- - 2 (rhou-.n) n
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) qp[s] = qm[s];
             qp[1] = (fd == 0) ? -qm[1] : qm[1];
             qp[2] = (fd == 1) ? -qm[2] : qm[2];
             qp[3] = (fd == 2) ? -qm[3] : qm[3];
+            if (VISC) {
+                const R* gn = GF + (size_t)e * NF2 * Np + (size_t)(4 * fd) * Np + vM;
+#pragma unroll
+                for (int w = 0; w < 4; ++w) f2p[w] = -gn[(size_t)w * Np];
+            }
+            if (HYPER) {
+                const R* hn = HDS + (size_t)e * 9 * Np + (size_t)fd * Np + vM;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) hdp[c] = -hn[(size_t)c * 3 * Np];
+            }
+            ux = qm[1];
+            uy = qm[2];
         }
-        const Level<R> lvp = nb >= 0 ? load_level<R>(P, ezp * Nq + vP / Nfp) : lvm;
+        const Level<R> lvp = load_level<R>(P, nb >= 0 ? ezp * Nq + vP / Nfp : ez * Nq + vM / Nfp);
         const Thermo<R, MIXED> thp = thermo<R, MIXED, false>(qp, lvp, P);
         const R mn = pick3(fd, qp[1], qp[2], qp[3]);
         const R un = mn * thp.rinv;
-        add_flux_d<R, MIXED>(Fm, qp, mn, un, thp.pflux, thp.H, fd, S);
-        if (nb >= 0) {
-            const R rho = MIXED ? lvp.rho_ref + qp[0] : qp[0];
-            if (VISC) {
+        far_flux_d<R>(qp, mn, un, thp.pflux, thp.H, fd, S);
+        if (VISC) {
 #pragma unroll
-                for (int s = 1; s < NSTATE; ++s) S[s] += f2p[s - 1];
-            }
-            if (HYPER) {
-                S[1] += rho * hdp[0];
-                S[2] += rho * hdp[1];
-                S[4] += (hdp[0] * qp[1] + hdp[1] * qp[2]) + hdp[2] * rho;
-            }
+            for (int s = 1; s < NSTATE; ++s) S[s] += f2p[s - 1];
+        }
+        if (HYPER) {
+            const R rho = MIXED ? lvp.rho_ref + qp[0] : qp[0];
+            S[1] = fma(rho, hdp[0], S[1]);
+            S[2] = fma(rho, hdp[1], S[2]);
+            S[4] += (hdp[0] * ux + hdp[1] * uy) + hdp[2] * rho;
         }
         const R lam_p = fabs(un) + thp.c;
         const R lift = pick3(fd, xi[0], xi[1], xi[2]) * KConst<R>::inv_w0(P);
@@ -411,13 +424,15 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
     if (node_thread) {
         R acc1[NSTATE] = {0, 0, 0, 0, 0}, acc2[NSTATE] = {0, 0, 0, 0, 0}, acc3[NSTATE] = {0, 0, 0, 0, 0};
         const int L1 = nj + Nq * nk, L2 = ni + Nq * nk, L3 = ni + Nq * nj;
+        constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
-        for (int n = 0; n < Nq; ++n) {
+        for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+            const int n1 = SKIP ? others(n, ni) : n, n2 = SKIP ? others(n, nj) : n, n3 = SKIP ? others(n, nk) : n;
             R v1[NSTATE], v2[NSTATE], v3[NSTATE];
-            PL::ld(s_F, Np, L1 + n * Nfp, v1);
-            PL::ld(s_F + P5N, Np, L2 + n * Nfp, v2);
-            PL::ld(s_F + 2 * P5N, Np, L3 + n * Nfp, v3);
-            const R d1 = dhat_p<R>(P, ni * Nq + n), d2 = dhat_p<R>(P, nj * Nq + n), d3 = dhat_p<R>(P, nk * Nq + n);
+            PL::ld(s_F, Np, L1 + n1 * Nfp, v1);
+            PL::ld(s_F + P5N, Np, L2 + n2 * Nfp, v2);
+            PL::ld(s_F + 2 * P5N, Np, L3 + n3 * Nfp, v3);
+            const R d1 = dhat_p<R>(P, ni * Nq + n1), d2 = dhat_p<R>(P, nj * Nq + n2), d3 = dhat_p<R>(P, nk * Nq + n3);
 #pragma unroll
             for (int s = 0; s < NSTATE; ++s) {
                 acc1[s] = fma(d1, v1[s], acc1[s]);
