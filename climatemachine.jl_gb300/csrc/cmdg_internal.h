@@ -308,7 +308,7 @@ int launch_hyper_stage(Model* md, const LaunchArgs& a, cudaStream_t s);
 // the same passes on the cubed shell (hyper_shell.cu): tables, then Qin into
 // hd_out (nu grad^3 of u_h[0..2], h_tot, (Np, 12, nelem))
 int init_shell_hyper_tables(Model* md);
-int launch_shell_hyper_passes(Model* md, const void* Qin, void* hd_out, cudaStream_t s);
+int launch_shell_hyper_passes(Model* md, const void* Qin, void* hd_out, cudaStream_t s, bool cart);
 // ConstantDynamicViscosity on the cubed shell (hyper_shell.cu): the gradient
 // buffer (grad u, grad h_tot, (Np, 12, nelem)) and, mixed, grad h_ref; the
 // gradient pass of Qin into gout

@@ -498,6 +498,6 @@ extern "C" int cmdg_hyperdiffusive_state(cmdg_model* model, void* d_hd, const vo
     CMDG_ARG_CHECK(d_hd != nullptr && d_Q != nullptr, "NULL buffer");
     CMDG_ARG_CHECK(model->m.prm.hyperdiffusion != CMDG_HYPER_NONE, "the model has no hyperdiffusion");
     if (model->m.mesh->kind == MESH_SHELL)
-        return launch_shell_hyper_passes(&model->m, d_Q, d_hd, (cudaStream_t)stream);
+        return launch_shell_hyper_passes(&model->m, d_Q, d_hd, (cudaStream_t)stream, true);
     return launch_hyper_passes(&model->m, d_Q, d_hd, (cudaStream_t)stream);
 }

@@ -17,6 +17,14 @@
 //    2525-3000, NumericalFluxes.jl:768-790), nu_4 per node from
 //    lengthscale_horizontal (src/Numerics/Mesh/Geometry.jl:129-151).
 //
+// The passes hand contravariant components J dxi_d/dx . grad to one another
+// and to the stage kernel, which is what the divergence contracts and what a
+// face needs of the far side: a face gathers 4 words instead of 12
+// (shell_partner_dir), and the divergence pass reads no geometry but 1/J.
+// With HorizontalDirection the xi3 words, contractions and faces are left
+// out.  The passes are bound by L1/L2 traffic and latency: the mixed GCM step
+// with hyperdiffusion (425,250 nodes) went from 317 to 280 us.
+//
 // The normals, surface Jacobians and lift weights come from J dxi_d/dx at the
 // face node, as in the cubed-shell stage kernel (Metrics.jl:431-724).  In
 // mixed precision the FP32 passes carry h' = h_tot - h_ref(node); the
@@ -123,7 +131,7 @@ __device__ __forceinline__ void shell_hyper_args(const KParams& P, const R q[NST
 // 318 us)
 template <int N, typename R, int NA = 4>
 __device__ __forceinline__ void shell_strong_gradient(const ShellIdx<N>& x, const R* s_X, const R* s_dF, const R* s_D,
-                                                      const R* g, int t, bool horiz, R out[3 * NA]) {
+                                                      const R* g, int t, bool horiz, R Jx[9], R out[3 * NA]) {
     constexpr int Nq = N + 1, Np = Nq * Nq * Nq, Nfp = Nq * Nq, NFN = 6 * Nfp;
     R a[NA][3];
 #pragma unroll
@@ -132,13 +140,21 @@ __device__ __forceinline__ void shell_strong_gradient(const ShellIdx<N>& x, cons
     constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
     for (int n = 0; n < (SKIP ? N : Nq); ++n) {
-        const int n1 = SKIP ? others(n, x.ni) : n, n2 = SKIP ? others(n, x.nj) : n, n3 = SKIP ? others(n, x.nk) : n;
-        const R d1 = s_D[x.ni * Nq + n1], d2 = s_D[x.nj * Nq + n2], d3 = s_D[x.nk * Nq + n3];
+        const int n1 = SKIP ? others(n, x.ni) : n, n2 = SKIP ? others(n, x.nj) : n;
+        const R d1 = s_D[x.ni * Nq + n1], d2 = s_D[x.nj * Nq + n2];
 #pragma unroll
         for (int s = 0; s < NA; ++s) {
             a[s][0] = fma(d1, s_X[s * Np + L1 + n1], a[s][0]);
             a[s][1] = fma(d2, s_X[s * Np + L2 + n2 * Nq], a[s][1]);
-            a[s][2] = fma(d3, s_X[s * Np + L3 + n3 * Nfp], a[s][2]);
+        }
+    }
+    if (!horiz) {  // HorizontalDirection: no xi3 derivative
+#pragma unroll
+        for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+            const int n3 = SKIP ? others(n, x.nk) : n;
+            const R d3 = s_D[x.nk * Nq + n3];
+#pragma unroll
+            for (int s = 0; s < NA; ++s) a[s][2] = fma(d3, s_X[s * Np + L3 + n3 * Nfp], a[s][2]);
         }
     }
     auto add = [&](int ff) {
@@ -150,20 +166,26 @@ __device__ __forceinline__ void shell_strong_gradient(const ShellIdx<N>& x, cons
     if (x.ni == N) add(1);
     if (x.nj == 0) add(2);
     if (x.nj == N) add(3);
-    if (x.nk == 0) add(4);
-    if (x.nk == N) add(5);
-    R Jx[9];
+    if (!horiz && x.nk == 0) add(4);
+    if (!horiz && x.nk == N) add(5);
 #pragma unroll
     for (int w = 0; w < 9; ++w) Jx[w] = g[(KG_JXI + w) * Np + t];
     const R iJ = g[KG_INVJ * Np + t];
-    if (horiz) {  // HorizontalDirection: no xi3 derivative
-#pragma unroll
-        for (int s = 0; s < NA; ++s) a[s][2] = R(0);
-    }
 #pragma unroll
     for (int s = 0; s < NA; ++s)
 #pragma unroll
         for (int j = 0; j < 3; ++j) out[3 * s + j] = iJ * (Jx[j] * a[s][0] + Jx[3 + j] * a[s][1] + Jx[6 + j] * a[s][2]);
+}
+
+// contravariant components Ct[4 d + s] = J dxi_d/dx . G_s of four Cartesian
+// vectors G[3 s + j]
+template <typename R>
+__device__ __forceinline__ void contravariant(const R Jx[9], const R G[12], R Ct[12]) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            Ct[4 * d + s] = Jx[3 * d + 0] * G[3 * s + 0] + Jx[3 * d + 1] * G[3 * s + 1] + Jx[3 * d + 2] * G[3 * s + 2];
 }
 
 // level and kernel geometry of the node across face x.f (nb >= 0)
@@ -195,7 +217,12 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
     const int* nbr = P.nbr + NBR_STRIDE * e;
     const int ez = __ldg(nbr + 6);
     if (t < Nq * Nq) s_D[t] = VConst<R>::D(P, t);
-    const int nb = x.face ? __ldg(nbr + x.f) : -1;
+    const bool horiz = PROJECT && P.hyper_horizontal != 0;
+    const bool face = x.face && !(horiz && x.fd == 2);
+    const int nb = face ? __ldg(nbr + x.f) : -1;
+    const int vP = nb < 0 ? x.vM
+                   : ARRAYS ? __ldg(P.fpart + ((size_t)e * 6 + x.f) * Nfp + x.fn)
+                            : shell_partner<N>(nbr, x.f, x.fn);
     R q[NSTATE], qp[NSTATE];
     chain_wait();
     if (x.node) {
@@ -203,9 +230,6 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
 #pragma unroll
         for (int s = 0; s < NSTATE; ++s) q[s] = qe[s * Np];
     }
-    const int vP = nb < 0 ? x.vM
-                   : ARRAYS ? __ldg(P.fpart + ((size_t)e * 6 + x.f) * Nfp + x.fn)
-                            : shell_partner<N>(nbr, x.f, x.fn);
     if (nb >= 0) {
         const R* qn = Qin + (size_t)nb * ESTRIDE + vP;
 #pragma unroll
@@ -220,7 +244,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
     }
     __syncthreads();
 
-    if (x.face) {
+    if (face) {
         // c n (H+ - H-) / w_0 (c = 1/2 inside, 1 on walls) for the derivative
         // along xi_fd, without what the diagonal of D leaves out (KParams::DC)
         R Hp[NA];
@@ -263,11 +287,22 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
     chain_release();
 
     if (x.node) {
-        R g[3 * NA];
-        shell_strong_gradient<N, R, NA>(x, s_H, s_dF, s_D, ge, t, PROJECT && P.hyper_horizontal != 0, g);
+        R g[3 * NA], Jx[9];
+        shell_strong_gradient<N, R, NA>(x, s_H, s_dF, s_D, ge, t, horiz, Jx, g);
         R* o = hg + (size_t)e * 3 * NA * Np + t;
+        if constexpr (PROJECT) {
+            R Ct[12];
+            contravariant<R>(Jx, g, Ct);
 #pragma unroll
-        for (int w = 0; w < 3 * NA; ++w) o[w * Np] = g[w];
+            for (int w = 0; w < 8; ++w) o[w * Np] = Ct[w];
+            if (!horiz) {
+#pragma unroll
+                for (int w = 8; w < 12; ++w) o[w * Np] = Ct[w];
+            }
+        } else {
+#pragma unroll
+            for (int w = 0; w < 3 * NA; ++w) o[w * Np] = g[w];
+        }
     }
 }
 
@@ -282,64 +317,58 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
 
     const int e = blockIdx.x, t = threadIdx.x;
     const Ix x(t);
-    const R* __restrict__ geo = static_cast<const R*>(P.geo);
-    const R* ge = geo + (size_t)e * GSTRIDE;
+    const R* __restrict__ ge = static_cast<const R*>(P.geo) + (size_t)e * GSTRIDE;
     const int* nbr = P.nbr + NBR_STRIDE * e;
     if (t < Nq * Nq) s_Dh[t] = static_cast<const R*>(P.Dhat)[t];
-    chain_wait();
-    if (x.node) {
-        const R* gn = hg + (size_t)e * 12 * Np + t;
-        R G[12];
-#pragma unroll
-        for (int w = 0; w < 12; ++w) G[w] = gn[w * Np];
-        R Jx[9];
-#pragma unroll
-        for (int w = 0; w < 9; ++w) Jx[w] = ge[(KG_JXI + w) * Np + t];
-#pragma unroll
-        for (int d = 0; d < 3; ++d)
-#pragma unroll
-            for (int s = 0; s < 4; ++s)
-                s_Ft[(d * 4 + s) * Np + t] =
-                    Jx[3 * d + 0] * G[3 * s + 0] + Jx[3 * d + 1] * G[3 * s + 1] + Jx[3 * d + 2] * G[3 * s + 2];
-    }
-    const int nb = x.face ? __ldg(nbr + x.f) : -1;
-    R Gp[12];
+    const bool horiz = P.hyper_horizontal != 0;  // HorizontalDirection: no xi3 terms
+    const bool face = x.face && !(horiz && x.fd == 2);
+    const int nb = face ? __ldg(nbr + x.f) : -1;
+    int vP = 0, f2d = 0;
+    bool flip = false;
     if (nb >= 0) {
-        const int vP = shell_partner<N>(nbr, x.f, x.fn);
-        const R* gq = hg + (size_t)nb * 12 * Np + vP;
+        vP = shell_partner<N>(nbr, x.f, x.fn);
+        shell_partner_dir(nbr, x.f, f2d, flip);
+    }
+    chain_wait();
+    const R* gn = hg + (size_t)e * 12 * Np + t;
+    R Gp[4];
+    if (nb >= 0) {
+        const R* gq = hg + ((size_t)nb * 12 + 4 * f2d) * Np + vP;
 #pragma unroll
-        for (int w = 0; w < 12; ++w) Gp[w] = gq[(size_t)w * Np];
+        for (int s = 0; s < 4; ++s) Gp[s] = gq[s * Np];
+    }
+    if (x.node) {
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s_Ft[w * Np + t] = gn[w * Np];
+        if (!horiz) {
+#pragma unroll
+            for (int w = 8; w < 12; ++w) s_Ft[w * Np + t] = gn[w * Np];
+        }
     }
     __syncthreads();
 
-    if (x.face) {
+    if (face) {
         // the far side's half of the central penalty (KParams::DhatC), with
         // vMI sM n = +-(J dxi_fd/dx) / (J w_0)
-        const R j0 = ge[(KG_JXI + x.fd * 3 + 0) * Np + x.vM];
-        const R j1 = ge[(KG_JXI + x.fd * 3 + 1) * Np + x.vM];
-        const R j2 = ge[(KG_JXI + x.fd * 3 + 2) * Np + x.vM];
         const R w = (x.fside ? R(0.5) : R(-0.5)) * KConst<R>::inv_w0(P);
+        const R wp = flip ? -w : w;
 #pragma unroll
-        for (int s = 0; s < 4; ++s)
-            s_dF[s * NFN + t] = w * (nb >= 0 ? j0 * Gp[3 * s + 0] + j1 * Gp[3 * s + 1] + j2 * Gp[3 * s + 2]
-                                             : s_Ft[(x.fd * 4 + s) * Np + x.vM]);
+        for (int s = 0; s < 4; ++s) s_dF[s * NFN + t] = nb >= 0 ? wp * Gp[s] : w * s_Ft[(x.fd * 4 + s) * Np + x.vM];
     }
     __syncthreads();
     chain_release();
 
     if (x.node) {
-        R a[4] = {0, 0, 0, 0}, av[4] = {0, 0, 0, 0};
+        R a[4] = {0, 0, 0, 0};
         const int L1 = Nq * (x.nj + Nq * x.nk), L2 = x.ni + Nfp * x.nk, L3 = x.ni + Nq * x.nj;
         constexpr bool SKIP = sizeof(R) == 8;
 #pragma unroll
         for (int n = 0; n < (SKIP ? N : Nq); ++n) {
-            const int n1 = SKIP ? others(n, x.ni) : n, n2 = SKIP ? others(n, x.nj) : n, n3 = SKIP ? others(n, x.nk) : n;
-            const R d1 = s_Dh[x.ni * Nq + n1], d2 = s_Dh[x.nj * Nq + n2], d3 = s_Dh[x.nk * Nq + n3];
+            const int n1 = SKIP ? others(n, x.ni) : n, n2 = SKIP ? others(n, x.nj) : n;
+            const R d1 = s_Dh[x.ni * Nq + n1], d2 = s_Dh[x.nj * Nq + n2];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) {
+            for (int s = 0; s < 4; ++s)
                 a[s] = fma(d1, s_Ft[(0 * 4 + s) * Np + L1 + n1], fma(d2, s_Ft[(1 * 4 + s) * Np + L2 + n2 * Nq], a[s]));
-                av[s] = fma(d3, s_Ft[(2 * 4 + s) * Np + L3 + n3 * Nfp], av[s]);
-            }
         }
         auto add = [&](int ff) {
             const int idx = ff * Nfp + x.on_face(ff);
@@ -350,9 +379,14 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
         if (x.ni == N) add(1);
         if (x.nj == 0) add(2);
         if (x.nj == N) add(3);
-        if (!P.hyper_horizontal) {  // HorizontalDirection: no xi3 terms
+        if (!horiz) {
 #pragma unroll
-            for (int s = 0; s < 4; ++s) a[s] += av[s];
+            for (int n = 0; n < (SKIP ? N : Nq); ++n) {
+                const int n3 = SKIP ? others(n, x.nk) : n;
+                const R d3 = s_Dh[x.nk * Nq + n3];
+#pragma unroll
+                for (int s = 0; s < 4; ++s) a[s] = fma(d3, s_Ft[(2 * 4 + s) * Np + L3 + n3 * Nfp], a[s]);
+            }
             if (x.nk == 0) add(4);
             if (x.nk == N) add(5);
         }
@@ -366,7 +400,10 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
     }
 }
 
-template <int N, typename R, bool MIXED>
+// CART: nu_4 grad(lap) itself, word 3 s + j (a caller's hyperdiffusive state
+// and the reference part); otherwise its contravariant components, word
+// 4 d + s, of which the stage kernel gathers four per face node
+template <int N, typename R, bool MIXED, bool CART>
 __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(const KParams P, const R* hl, R* hd) {
     using Ix = ShellIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp, GSTRIDE = KG_NFIELDS * Np;
@@ -381,23 +418,25 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
     const R* ge = geo + (size_t)e * GSTRIDE;
     const int* nbr = P.nbr + NBR_STRIDE * e;
     if (t < Nq * Nq) s_D[t] = VConst<R>::D(P, t);
+    const bool horiz = P.hyper_horizontal != 0;
+    const bool face = x.face && !(horiz && x.fd == 2);
+    const int nb = face ? __ldg(nbr + x.f) : -1;
+    const int vP = nb >= 0 ? shell_partner<N>(nbr, x.f, x.fn) : 0;
     chain_wait();
     if (x.node) {
         const R* ln = hl + (size_t)e * 4 * Np + t;
 #pragma unroll
         for (int s = 0; s < 4; ++s) s_L[s * Np + t] = ln[s * Np];
     }
-    const int nb = x.face ? __ldg(nbr + x.f) : -1;
     R Lp[4];
     if (nb >= 0) {
-        const int vP = shell_partner<N>(nbr, x.f, x.fn);
         const R* lq = hl + (size_t)nb * 4 * Np + vP;
 #pragma unroll
         for (int s = 0; s < 4; ++s) Lp[s] = lq[(size_t)s * Np];
     }
     __syncthreads();
 
-    if (x.face) {
+    if (face) {
         // n (L+ - L-) / (2 w_0), without what the diagonal of D leaves out
         const R w = (x.fside ? R(0.5) : R(-0.5)) * KConst<R>::inv_w0(P);
 #pragma unroll
@@ -407,20 +446,28 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
     chain_release();
 
     if (x.node) {
-        R g[12];
-        shell_strong_gradient<N, R>(x, s_L, s_dF, s_D, ge, t, P.hyper_horizontal != 0, g);
+        R g[12], Jx[9];
+        shell_strong_gradient<N, R>(x, s_L, s_dF, s_D, ge, t, horiz, Jx, g);
         const R nu4 = static_cast<const R*>(P.nu4)[(size_t)e * Np + t];
-        R* o = hd + (size_t)e * 12 * Np + t;
 #pragma unroll
         for (int w = 0; w < 12; ++w) {
-            R v = nu4 * g[w];
-            if (MIXED && w >= 9) v += P.hglap_ref32[((size_t)e * 3 + (w - 9)) * Np + t];
-            o[w * Np] = v;
+            g[w] *= nu4;
+            if (MIXED && w >= 9) g[w] += P.hglap_ref32[((size_t)e * 3 + (w - 9)) * Np + t];
+        }
+        R* o = hd + (size_t)e * 12 * Np + t;
+        if constexpr (CART) {
+#pragma unroll
+            for (int w = 0; w < 12; ++w) o[w * Np] = g[w];
+        } else {
+            R Ct[12];
+            contravariant<R>(Jx, g, Ct);
+#pragma unroll
+            for (int w = 0; w < 12; ++w) o[w * Np] = Ct[w];
         }
     }
 }
 
-template <int N, typename R, bool MIXED>
+template <int N, typename R, bool MIXED, bool CART>
 cudaError_t launch_shell_passes_typed(const KParams& P, const void* Q, void* hd, void* hl, cudaStream_t s) {
     constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp, NFN = 6 * Nfp, NT = ShellDims<N>::NT;
     constexpr size_t b1 = sizeof(R) * (4 * Np + 4 * NFN + Nq * Nq);
@@ -429,13 +476,13 @@ cudaError_t launch_shell_passes_typed(const KParams& P, const void* Q, void* hd,
     cudaError_t e;
     if ((e = opt_in(shell_hyper_grad_kernel<N, R, MIXED>, b1)) != cudaSuccess) return e;
     if ((e = opt_in(shell_hyper_div_kernel<N, R>, b2)) != cudaSuccess) return e;
-    if ((e = opt_in(shell_hyper_glap_kernel<N, R, MIXED>, b3)) != cudaSuccess) return e;
+    if ((e = opt_in(shell_hyper_glap_kernel<N, R, MIXED, CART>, b3)) != cudaSuccess) return e;
     R* g = static_cast<R*>(hd);
     R* l = static_cast<R*>(hl);
     const unsigned grid = (unsigned)P.nelem;
     if ((e = launch_chained(s, shell_hyper_grad_kernel<N, R, MIXED>, grid, NT, b1, P, Q, g)) != cudaSuccess) return e;
     if ((e = launch_chained(s, shell_hyper_div_kernel<N, R>, grid, NT, b2, P, g, l)) != cudaSuccess) return e;
-    return launch_chained(s, shell_hyper_glap_kernel<N, R, MIXED>, grid, NT, b3, P, l, g);
+    return launch_chained(s, shell_hyper_glap_kernel<N, R, MIXED, CART>, grid, NT, b3, P, l, g);
 }
 
 // the viscous gradient pass: grad u, grad h_tot (Np, 12, nelem)
@@ -500,17 +547,23 @@ cudaError_t launch_shell_visc(const KParams& P, int N, bool mixed, bool smag, co
     }
 }
 
-cudaError_t launch_shell_passes(const KParams& P, int N, bool mixed, const void* Q, void* hd, void* hl,
+template <int N>
+cudaError_t launch_shell_passes_N(const KParams& P, bool mixed, bool cart, const void* Q, void* hd, void* hl,
+                                  cudaStream_t s) {
+    if (mixed)
+        return cart ? launch_shell_passes_typed<N, float, true, true>(P, Q, hd, hl, s)
+                    : launch_shell_passes_typed<N, float, true, false>(P, Q, hd, hl, s);
+    return cart ? launch_shell_passes_typed<N, double, false, true>(P, Q, hd, hl, s)
+                : launch_shell_passes_typed<N, double, false, false>(P, Q, hd, hl, s);
+}
+
+cudaError_t launch_shell_passes(const KParams& P, int N, bool mixed, bool cart, const void* Q, void* hd, void* hl,
                                 cudaStream_t s) {
     switch (N) {
-        case 2: return mixed ? launch_shell_passes_typed<2, float, true>(P, Q, hd, hl, s)
-                             : launch_shell_passes_typed<2, double, false>(P, Q, hd, hl, s);
-        case 3: return mixed ? launch_shell_passes_typed<3, float, true>(P, Q, hd, hl, s)
-                             : launch_shell_passes_typed<3, double, false>(P, Q, hd, hl, s);
-        case 4: return mixed ? launch_shell_passes_typed<4, float, true>(P, Q, hd, hl, s)
-                             : launch_shell_passes_typed<4, double, false>(P, Q, hd, hl, s);
-        case 5: return mixed ? launch_shell_passes_typed<5, float, true>(P, Q, hd, hl, s)
-                             : launch_shell_passes_typed<5, double, false>(P, Q, hd, hl, s);
+        case 2: return launch_shell_passes_N<2>(P, mixed, cart, Q, hd, hl, s);
+        case 3: return launch_shell_passes_N<3>(P, mixed, cart, Q, hd, hl, s);
+        case 4: return launch_shell_passes_N<4>(P, mixed, cart, Q, hd, hl, s);
+        case 5: return launch_shell_passes_N<5>(P, mixed, cart, Q, hd, hl, s);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -585,7 +638,7 @@ int init_shell_hyper_tables(Model* md) {
         P.geo = md->d_geo64;
         P.nu4 = dnu;
         P.hglap_ref32 = nullptr;
-        ce = launch_shell_passes(P, N, false, dq, dhd, dhl, 0);
+        ce = launch_shell_passes(P, N, false, true, dq, dhd, dhl, 0);
         if (ce == cudaSuccess) ce = cudaDeviceSynchronize();
     }
     std::vector<double> hd64;
@@ -607,7 +660,7 @@ int init_shell_hyper_tables(Model* md) {
     return CMDG_OK;
 }
 
-int launch_shell_hyper_passes(Model* md, const void* Qin, void* hd_out, cudaStream_t s) {
+int launch_shell_hyper_passes(Model* md, const void* Qin, void* hd_out, cudaStream_t s, bool cart) {
     const Mesh& m = *md->mesh;
     LaunchArgs a;
     a.Qin = Qin;
@@ -616,7 +669,7 @@ int launch_shell_hyper_passes(Model* md, const void* Qin, void* hd_out, cudaStre
     a.alpha = a.beta = a.rka = a.rkb_dt = 0;
     a.mode = 0;
     const KParams P = make_params(md, a);
-    const cudaError_t err = launch_shell_passes(P, m.N, md->precision == CMDG_MIXED, Qin, hd_out, md->d_hlap, s);
+    const cudaError_t err = launch_shell_passes(P, m.N, md->precision == CMDG_MIXED, cart, Qin, hd_out, md->d_hlap, s);
     if (err != cudaSuccess) {
         set_error("cubed-shell hyperdiffusion pass launch failed: %s", cudaGetErrorString(err));
         return CMDG_ERR_CUDA;

@@ -52,7 +52,7 @@ struct ShellSmem {
 };
 
 // HYPER: DryBiharmonic hyperdiffusion, whose state nu grad^3 (Np, 12, nelem;
-// word 3 c + d = nu d/dx_d lap(u_h[c]), 9 + d = nu d/dx_d lap(h_tot)) is read
+// word 4 d + c = nu J dxi_d/dx . grad lap(u_h[c]), c = 3: lap(h_tot)) is read
 // from P.hd: the hyperdiffusive fluxes (tendencies_momentum.jl:51-54,
 // tendencies_energy.jl:40-48) join the volume flux and, with the neighbour's
 // state, the central second-order interface flux; walls carry the
@@ -178,21 +178,6 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
             F1[s] = flux_d<R, MIXED>(q, th, 1, s);
             F2[s] = flux_d<R, MIXED>(q, th, 2, s);
         }
-        if (HYPER) {
-            const R* hn = static_cast<const R*>(P.hd) + (size_t)e * 12 * Np + t;
-            R hd[12];
-#pragma unroll
-            for (int w = 0; w < 12; ++w) hd[w] = hn[w * Np];
-            const R rho = MIXED ? lv.rho_ref + q[0] : q[0];
-            auto add_hyper = [&](R(&F)[NSTATE], int d) {
-#pragma unroll
-                for (int c = 0; c < 3; ++c) F[1 + c] += rho * hd[3 * c + d];
-                F[4] += (hd[d] * q[1] + hd[3 + d] * q[2] + hd[6 + d] * q[3]) + hd[9 + d] * rho;
-            };
-            add_hyper(F0, 0);
-            add_hyper(F1, 1);
-            add_hyper(F2, 2);
-        }
         if (VISC) {
             R Fv[3][NSTATE];
             shell_visc_flux<R, MIXED, VT>(P, e, t, Np, q, lv, th.rinv, Fv);
@@ -230,6 +215,16 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
 #pragma unroll
                 for (int s = 0; s < NSTATE; ++s)
                     Ft[s] = Jx[d * 3 + 0] * F0[s] + Jx[d * 3 + 1] * F1[s] + Jx[d * 3 + 2] * F2[s];
+                if (HYPER) {
+                    const R* hn = static_cast<const R*>(P.hd) + ((size_t)e * 12 + 4 * d) * Np + t;
+                    const R rho = MIXED ? lv.rho_ref + q[0] : q[0];
+                    R hd[4];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) hd[c] = hn[c * Np];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) Ft[1 + c] += rho * hd[c];
+                    Ft[4] += (hd[0] * q[1] + hd[1] * q[2] + hd[2] * q[3]) + hd[3] * rho;
+                }
                 PL::st(s_F + d * SM::P5N, Np, t, Ft);
             }
         }
@@ -356,11 +351,13 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
         }
         if (HYPER && nb >= 0) {
             // neighbour's hyperdiffusive flux . n
-            const R* hn = static_cast<const R*>(P.hd) + (size_t)nb * 12 * Np + vP;
+            int f2d;
+            bool flip;
+            shell_partner_dir(nbr, f, f2d, flip);
+            const R* hn = static_cast<const R*>(P.hd) + ((size_t)nb * 12 + 4 * f2d) * Np + vP;
             R hn_n[4];
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                hn_n[c] = j0 * hn[(3 * c + 0) * Np] + j1 * hn[(3 * c + 1) * Np] + j2 * hn[(3 * c + 2) * Np];
+            for (int c = 0; c < 4; ++c) hn_n[c] = flip ? -hn[c * Np] : hn[c * Np];
             const R rho_p = MIXED ? lvp.rho_ref + qp[0] : qp[0];
 #pragma unroll
             for (int c = 0; c < 3; ++c) S[1 + c] += rho_p * hn_n[c];
@@ -527,7 +524,7 @@ int launch_shell_stage(Model* md, const LaunchArgs& a, cudaStream_t s) {
         return CMDG_OK;
     }
     if (hyper) {
-        const int rc = launch_shell_hyper_passes(md, a.Qin, md->d_hd, s);
+        const int rc = launch_shell_hyper_passes(md, a.Qin, md->d_hd, s, false);
         if (rc) return rc;
     }
     if (visc) {

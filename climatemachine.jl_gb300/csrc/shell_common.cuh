@@ -35,6 +35,18 @@ __device__ __forceinline__ int shell_partner(const int* nbr, int f, int fn) {
     return (f2 < 2) ? side2 + Nq * (a2 + Nq * fb) : a2 + Nq * (side2 + Nq * fb);
 }
 
+// The face of the neighbour across face f: its direction f2d, and the factor
+// +-1 that turns the neighbour's contravariant component along its xi_f2d at
+// the facing node into this element's along xi_f.  Both elements form
+// J dxi_d/dx at a face from the face's own nodes (curl-invariant metrics), so
+// the two agree there up to the sign of the direction and rounding.
+__device__ __forceinline__ void shell_partner_dir(const int* nbr, int f, int& f2d, bool& flip) {
+    int f2 = f ^ 1;
+    if (f < 4) f2 = (int)(((unsigned)__ldg(nbr + 7) >> (4 * f)) & 3u);
+    f2d = f2 >> 1;
+    flip = (f2 & 1) == (f & 1);
+}
+
 // Reference state at node n of an element with kernel geometry g (Np nodes
 // per element): the level row of level lev plus the node's per-node parts
 // (in FP64 also the rounding-sized pressure and pressure-coefficient parts,
