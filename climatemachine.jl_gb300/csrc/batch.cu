@@ -1,11 +1,12 @@
 // Ensembles of models advanced together, by one of two kernel families:
 //   per order  the members are grouped by polynomial order; each LSRK54
 //              stage of a group is one launch of the tile-walking node kernel
-//              of that order (stage.cu), so members of uneven size share the
-//              GPU without a launch per member.  Members are independent, so
-//              the groups' stage chains run on their own streams: captured as
-//              one CUDA graph they are three independent branches that the
-//              GPU overlaps, joined at the end of the call;
+//              of that order (stage.cu), so small members share the GPU
+//              without a launch per member; members that fill it are chains
+//              of their own (Chain).  Members are independent, so the chains
+//              run on three streams: captured as one CUDA graph they are
+//              three independent branches that the GPU overlaps, joined at
+//              the end of the call;
 //   persistent one launch per stage of the line kernel (stage_lines.cu) over
 //              one list of tiles of every order, with one CTA shape for all
 //              orders: its size sets the elements per CTA pass and the nodes
@@ -28,7 +29,7 @@
 
 namespace cmdg {
 
-constexpr int BATCH_NMIN = 3, BATCH_NMAX = 5, BATCH_NGROUPS = BATCH_NMAX - BATCH_NMIN + 1;
+constexpr int BATCH_NMIN = 3, BATCH_NMAX = 5, BATCH_NGROUPS = BATCH_NMAX - BATCH_NMIN + 1, BATCH_NBRANCH = 3;
 
 struct Group {
     int N = 0;
@@ -36,9 +37,35 @@ struct Group {
     int grid = -1;                  // -1 = one CTA per tile, 0 = one wave of resident CTAs, n > 0 = n CTAs
     BatchTile* d_tiles = nullptr;
     int ntiles = 0;
-    cudaStream_t stream = nullptr;  // side stream of the group's stage chain
-    cudaEvent_t join = nullptr;
 };
+
+// Members of one order that step together, all their stages before the next
+// chain of the same branch: either one member, by the one-model kernel, or a
+// set of small members, by the tile-walking kernel over tiles [t0, t0 + nt).
+//
+// A stage of every member before the next stage of any streams all members'
+// states through L2 five times a step; a chain's working set stays there
+// from stage to stage (the sets are bounded accordingly).  And the one-model
+// kernel has its parameters in the constant bank: 56 registers and 7 CTAs per
+// SM at N = 4, against 72 with spills and 5 CTAs when they come from global
+// memory.  A step of 24 members (8 to 16 elements a side, N = 3 to 5), in us:
+// 1371 stage by stage, 1267 in sets of up to 24 MB, 1343 of 48 MB, 898 member
+// by member.
+struct Chain {
+    int group;
+    int member;  // -1 = a set
+    int t0, nt;
+    double work;  // nodes
+};
+// bytes a chain touches per node: three state buffers and the register
+constexpr size_t CHAIN_BYTES_PER_NODE = NSTATE * (3 * sizeof(float) + sizeof(double));
+constexpr size_t SET_BYTES = (size_t)24 << 20;
+// A member of at least this many nodes steps alone: below, five launches of its
+// own cost more than the better kernel gains.  24 equal members per step, one
+// by one against in sets, us: 32,768 nodes (N = 3) 268 / 196, 46,656 (N = 5)
+// 268 / 224, 64,000 (N = 3) 271 / 351, (N = 4) 270 / 338, 110,592 (N = 5)
+// 384 / 524; four members of 64,000 (N = 4) 64 / 65.
+constexpr int64_t ALONE_MIN_NODES = 64000;
 
 enum { FAMILY_PER_ORDER = 0, FAMILY_PERSISTENT = 1 };
 
@@ -59,7 +86,11 @@ struct Batch {
     std::vector<void*> scratch;     // two stage buffers per member (one allocation each)
     std::vector<size_t> state_bytes;
     KParams* d_params = nullptr;    // [5 stages][members]
+    std::vector<KParams> params;    // the same on the host
     Group groups[BATCH_NGROUPS];
+    std::vector<Chain> branches[BATCH_NBRANCH];
+    cudaStream_t stream[BATCH_NBRANCH] = {};  // side streams of the branches (the first runs on the call's)
+    cudaEvent_t join[BATCH_NBRANCH] = {};
     // members with a turbulence closure, stepped member by member on their own branch
     std::vector<int> viscous;
     cudaStream_t visc_stream = nullptr;
@@ -79,22 +110,65 @@ static void drop_graph(Batch* b) {
     b->graph = nullptr;
 }
 
-// Tiles of one order: members interleaved, tile_elems consecutive elements each.
-static int build_tiles(Batch* b, Group& g) {
-    std::vector<BatchTile> tiles;
-    std::vector<int64_t> pos(b->members.size(), 0);
-    bool more = true;
-    while (more) {
-        more = false;
-        for (size_t m = 0; m < b->members.size(); ++m) {
-            const Mesh& mesh = *b->members[m]->mesh;
-            if (mesh.N != g.N || pos[m] >= mesh.nelem || b->members[m]->prm.turbulence != CMDG_TURB_NONE) continue;
-            const int64_t e1 = std::min<int64_t>(mesh.nelem, pos[m] + g.tile_elems);
-            tiles.push_back(BatchTile{(int)m, (int)pos[m], (int)e1, mesh.N});
-            pos[m] = e1;
-            more = true;
-        }
+// The branches' chains: the largest first, each to the branch with the least
+// work so far.
+static void spread_chains(Batch* b, std::vector<Chain> chains) {
+    std::stable_sort(chains.begin(), chains.end(), [](const Chain& x, const Chain& y) { return x.work > y.work; });
+    double load[BATCH_NBRANCH] = {};
+    for (auto& br : b->branches) br.clear();
+    for (const Chain& c : chains) {
+        const int i = (int)(std::min_element(load, load + BATCH_NBRANCH) - load);
+        b->branches[i].push_back(c);
+        load[i] += c.work;
     }
+}
+
+// Tiles of one order, chain by chain; within a set members interleaved,
+// tile_elems consecutive elements each.
+static int build_tiles(Batch* b, Group& g) {
+    const int gi = (int)(&g - b->groups);
+    std::vector<Chain> chains;
+    for (const auto& br : b->branches)
+        for (const Chain& c : br)
+            if (c.group != gi) chains.push_back(c);
+    std::vector<int> mine;
+    for (size_t m = 0; m < b->members.size(); ++m)
+        if (b->members[m]->mesh->N == g.N && b->members[m]->prm.turbulence == CMDG_TURB_NONE) mine.push_back((int)m);
+    // the members that step alone to the end
+    auto alone = [&](int m) { return b->members[m]->mesh->nelem * b->members[m]->mesh->Np >= ALONE_MIN_NODES; };
+    std::stable_partition(mine.begin(), mine.end(), [&](int m) { return !alone(m); });
+    std::vector<BatchTile> tiles;
+    for (size_t i = 0; i < mine.size();) {
+        size_t j = i, bytes = 0;
+        Chain c{gi, -1, (int)tiles.size(), 0, 0.0};
+        for (; j < mine.size(); ++j) {
+            const Mesh& mesh = *b->members[mine[j]]->mesh;
+            bytes += (size_t)mesh.nelem * mesh.Np * CHAIN_BYTES_PER_NODE;
+            if (j > i && (alone(mine[j]) || bytes > SET_BYTES)) break;
+            c.work += (double)mesh.nelem * mesh.Np;
+            if (alone(mine[j])) {
+                c.member = mine[j++];
+                break;
+            }
+        }
+        std::vector<int64_t> pos(j - i, 0);
+        for (bool more = true; more;) {
+            more = false;
+            for (size_t k = i; k < j; ++k) {
+                const Mesh& mesh = *b->members[mine[k]]->mesh;
+                int64_t& p = pos[k - i];
+                if (p >= mesh.nelem) continue;
+                const int64_t e1 = std::min<int64_t>(mesh.nelem, p + g.tile_elems);
+                tiles.push_back(BatchTile{mine[k], (int)p, (int)e1, g.N});
+                p = e1;
+                more = true;
+            }
+        }
+        c.nt = (int)tiles.size() - c.t0;
+        chains.push_back(c);
+        i = j;
+    }
+    spread_chains(b, chains);
     if (g.d_tiles) cudaFree(g.d_tiles);
     g.d_tiles = nullptr;
     g.ntiles = 0;
@@ -152,10 +226,18 @@ static void build_dhat(EnsDhat& d) {
     }
 }
 
-static int grid_of(const Group& g) {
-    int grid = g.grid > 0 ? g.grid : g.grid == 0 ? batch_resident_ctas(g.N) : g.ntiles;
+// CTAs of a launch over ntiles of a group's tiles
+static int grid_of(const Group& g, int ntiles) {
+    int grid = g.grid > 0 ? g.grid : g.grid == 0 ? batch_resident_ctas(g.N) : ntiles;
     if (grid <= 0) grid = 1;
-    return std::min(grid, g.ntiles);
+    return std::min(grid, ntiles);
+}
+
+static cudaError_t launch_chain_stage(Batch* b, const Chain& c, int st, cudaStream_t s) {
+    const size_t n = b->members.size();
+    const Group& g = b->groups[c.group];
+    if (c.member >= 0) return launch_member_stage(b->params[st * n + c.member], g.N, s);
+    return launch_batch_stage(b->d_params + st * n, g.d_tiles + c.t0, c.nt, g.N, grid_of(g, c.nt), s);
 }
 
 // Uploads the per-stage launch parameters of every member when the state
@@ -168,7 +250,8 @@ static int upload_params(Batch* b, void* const* Q, double* const* dQ, const doub
     if (same) return CMDG_OK;
     const double *A, *B;
     lsrk54_coefficients(&A, &B);
-    std::vector<KParams> host(5 * n);
+    std::vector<KParams>& host = b->params;
+    host.resize(5 * n);
     for (size_t m = 0; m < n; ++m) {
         char* S1 = static_cast<char*>(b->scratch[m]);
         char* S2 = S1 + b->state_bytes[m];
@@ -200,14 +283,14 @@ static int launch_error(cudaError_t e) {
     return CMDG_ERR_CUDA;
 }
 
-// nsteps steps of every group: the first non-empty group on s, the others on
-// their side streams, forked from and joined back into s.
+// nsteps steps of every member: the first non-empty branch on s, the others
+// on their side streams, forked from and joined back into s.
 static int issue(Batch* b, int nsteps, cudaStream_t s) {
     const size_t n = b->members.size();
     bool first = true;
     cudaError_t e = cudaEventRecord(b->fork, s);
     if (e != cudaSuccess) return launch_error(e);
-    std::vector<Group*> joined;
+    std::vector<int> joined;
     if (b->family == FAMILY_PERSISTENT && b->uni.ntiles) {
         const int grid = unified_grid(b->uni);
         for (int step = 0; step < nsteps; ++step)
@@ -217,19 +300,18 @@ static int issue(Batch* b, int nsteps, cudaStream_t s) {
                     return launch_error(e);
         first = false;
     }
-    for (Group& g : b->groups) {
-        if (!g.ntiles || b->family != FAMILY_PER_ORDER) continue;
-        cudaStream_t gs = first ? s : g.stream;
+    for (int i = 0; i < BATCH_NBRANCH; ++i) {
+        if (b->branches[i].empty() || b->family != FAMILY_PER_ORDER) continue;
+        cudaStream_t bs = first ? s : b->stream[i];
         if (!first) {
-            if ((e = cudaStreamWaitEvent(gs, b->fork, 0)) != cudaSuccess) return launch_error(e);
-            joined.push_back(&g);
+            if ((e = cudaStreamWaitEvent(bs, b->fork, 0)) != cudaSuccess) return launch_error(e);
+            joined.push_back(i);
         }
         first = false;
-        const int grid = grid_of(g);
-        for (int step = 0; step < nsteps; ++step)
-            for (int st = 0; st < 5; ++st)
-                if ((e = launch_batch_stage(b->d_params + st * n, g.d_tiles, g.ntiles, g.N, grid, gs)) != cudaSuccess)
-                    return launch_error(e);
+        for (const Chain& c : b->branches[i])
+            for (int step = 0; step < nsteps; ++step)
+                for (int st = 0; st < 5; ++st)
+                    if ((e = launch_chain_stage(b, c, st, bs)) != cudaSuccess) return launch_error(e);
     }
     if (!b->viscous.empty()) {
         cudaStream_t vs = first ? s : b->visc_stream;
@@ -261,9 +343,9 @@ static int issue(Batch* b, int nsteps, cudaStream_t s) {
             if ((e = cudaStreamWaitEvent(s, b->visc_join, 0)) != cudaSuccess) return launch_error(e);
         }
     }
-    for (Group* g : joined) {
-        if ((e = cudaEventRecord(g->join, g->stream)) != cudaSuccess) return launch_error(e);
-        if ((e = cudaStreamWaitEvent(s, g->join, 0)) != cudaSuccess) return launch_error(e);
+    for (int i : joined) {
+        if ((e = cudaEventRecord(b->join[i], b->stream[i])) != cudaSuccess) return launch_error(e);
+        if ((e = cudaStreamWaitEvent(s, b->join[i], 0)) != cudaSuccess) return launch_error(e);
     }
     return CMDG_OK;
 }
@@ -273,8 +355,10 @@ static void release(Batch* b) {
     if (b->d_params) cudaFree(b->d_params);
     for (Group& g : b->groups) {
         if (g.d_tiles) cudaFree(g.d_tiles);
-        if (g.stream) cudaStreamDestroy(g.stream);
-        if (g.join) cudaEventDestroy(g.join);
+    }
+    for (int i = 0; i < BATCH_NBRANCH; ++i) {
+        if (b->stream[i]) cudaStreamDestroy(b->stream[i]);
+        if (b->join[i]) cudaEventDestroy(b->join[i]);
     }
     if (b->uni.d_tiles) cudaFree(b->uni.d_tiles);
     if (b->fork) cudaEventDestroy(b->fork);
@@ -335,13 +419,15 @@ extern "C" int cmdg_batch_create(cmdg_model* const* models, int n, cmdg_batch** 
         cuda_fail(e, "stream");
     if (!rc && (e = cudaEventCreateWithFlags(&b->visc_join, cudaEventDisableTiming)) != cudaSuccess)
         cuda_fail(e, "event");
-    for (int gi = 0; gi < BATCH_NGROUPS && !rc; ++gi) {
-        Group& g = b->groups[gi];
-        g.N = BATCH_NMIN + gi;
-        if ((e = cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking)) != cudaSuccess) cuda_fail(e, "stream");
-        if (!rc && (e = cudaEventCreateWithFlags(&g.join, cudaEventDisableTiming)) != cudaSuccess)
+    for (int i = 0; i < BATCH_NBRANCH && !rc; ++i) {
+        if ((e = cudaStreamCreateWithFlags(&b->stream[i], cudaStreamNonBlocking)) != cudaSuccess)
+            cuda_fail(e, "stream");
+        if (!rc && (e = cudaEventCreateWithFlags(&b->join[i], cudaEventDisableTiming)) != cudaSuccess)
             cuda_fail(e, "event");
-        if (!rc) rc = build_tiles(b, g);
+    }
+    for (int gi = 0; gi < BATCH_NGROUPS && !rc; ++gi) {
+        b->groups[gi].N = BATCH_NMIN + gi;
+        rc = build_tiles(b, b->groups[gi]);
     }
     if (!rc) {
         build_dhat(b->uni.dhat);
@@ -465,28 +551,27 @@ extern "C" int cmdg_batch_lsrk54_step(cmdg_batch* batch, void* const* h_Q, doubl
     return CMDG_OK;
 }
 
-// One stage launch of the per-order family, every group on its branch as in
-// issue(), with the parameters of stage index 1.
+// One stage launch of every chain of the per-order family, on the branches as
+// in issue(), with the parameters of stage index 1.
 static cudaError_t per_order_stage(Batch* b, cudaStream_t s) {
-    const size_t n = b->members.size();
     cudaError_t e = cudaEventRecord(b->fork, s);
     if (e != cudaSuccess) return e;
     bool first = true;
-    std::vector<Group*> joined;
-    for (Group& g : b->groups) {
-        if (!g.ntiles) continue;
-        cudaStream_t gs = first ? s : g.stream;
+    std::vector<int> joined;
+    for (int i = 0; i < BATCH_NBRANCH; ++i) {
+        if (b->branches[i].empty()) continue;
+        cudaStream_t bs = first ? s : b->stream[i];
         if (!first) {
-            if ((e = cudaStreamWaitEvent(gs, b->fork, 0)) != cudaSuccess) return e;
-            joined.push_back(&g);
+            if ((e = cudaStreamWaitEvent(bs, b->fork, 0)) != cudaSuccess) return e;
+            joined.push_back(i);
         }
         first = false;
-        if ((e = launch_batch_stage(b->d_params + n, g.d_tiles, g.ntiles, g.N, grid_of(g), gs)) != cudaSuccess)
-            return e;
+        for (const Chain& c : b->branches[i])
+            if ((e = launch_chain_stage(b, c, 1, bs)) != cudaSuccess) return e;
     }
-    for (Group* g : joined) {
-        if ((e = cudaEventRecord(g->join, g->stream)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(s, g->join, 0)) != cudaSuccess) return e;
+    for (int i : joined) {
+        if ((e = cudaEventRecord(b->join[i], b->stream[i])) != cudaSuccess) return e;
+        if ((e = cudaStreamWaitEvent(s, b->join[i], 0)) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
@@ -496,8 +581,8 @@ static cudaError_t per_order_stage(Batch* b, cudaStream_t s) {
 // the next step ignores because stage 1 does not read it) it times
 //   the per-order family: for each order tile_elems in {1, 2, 4, 8, 16} x
 //   grid in {one CTA per tile, one wave of resident CTAs}, keeping each
-//   order's fastest, then the whole family (every order's launch on its
-//   branch);
+//   order's fastest for its sets of small members, then the whole family
+//   (every chain on its branch);
 //   the persistent family: CTA size in {128, 256} threads (elements per CTA
 //   pass and nodes per thread of each order follow from it) x tile_elems in
 //   {1, 2, 4, 8} x grid in {one CTA per tile, one wave of resident CTAs};
@@ -516,13 +601,12 @@ extern "C" int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* 
     int rc = upload_params(b, h_Q, h_dQ, unit_dt.data(), true);
     if (rc) return rc;
     {
-        std::vector<KParams> host(n);
-        CMDG_CUDA_CHECK(cudaMemcpy(host.data(), b->d_params + n, sizeof(KParams) * n, cudaMemcpyDeviceToHost));
-        for (auto& P : host) {
-            P.rkb_dt = 0.0;
-            P.rkb_dt32 = 0.0f;
+        KParams* const host = b->params.data() + n;
+        for (size_t m = 0; m < n; ++m) {
+            host[m].rkb_dt = 0.0;
+            host[m].rkb_dt32 = 0.0f;
         }
-        CMDG_CUDA_CHECK(cudaMemcpy(b->d_params + n, host.data(), sizeof(KParams) * n, cudaMemcpyHostToDevice));
+        CMDG_CUDA_CHECK(cudaMemcpy(b->d_params + n, host, sizeof(KParams) * n, cudaMemcpyHostToDevice));
         for (size_t m = 0; m < n; ++m)
             CMDG_CUDA_CHECK(cudaMemcpyAsync(b->scratch[m], h_Q[m], b->state_bytes[m], cudaMemcpyDeviceToDevice, s));
     }
@@ -557,7 +641,7 @@ extern "C" int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* 
             g.tile_elems = tiles[c / 2];
             g.grid = grids[c % 2];
             if ((rc = build_tiles(b, g))) break;
-            const int grid = grid_of(g);
+            const int grid = grid_of(g, g.ntiles);
             rc = time_it([&] { return launch_batch_stage(b->d_params + n, g.d_tiles, g.ntiles, g.N, grid, s); },
                          ms[gi * NC + c]);
             if (!rc && ms[gi * NC + c] < best) {

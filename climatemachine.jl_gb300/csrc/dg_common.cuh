@@ -97,6 +97,8 @@ struct BatchTile {
 cudaError_t launch_batch_stage(const KParams* d_params, const BatchTile* d_tiles, int ntiles, int N, int grid,
                                cudaStream_t s);
 int batch_resident_ctas(int N);
+// Stage launch of one ensemble member of order N, one CTA per element (stage.cu).
+cudaError_t launch_member_stage(const KParams& P, int N, cudaStream_t s);
 
 // Builds the launch arguments of a model (stage.cu).
 KParams make_params(Model* md, const LaunchArgs& a);

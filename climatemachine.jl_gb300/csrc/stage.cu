@@ -868,6 +868,15 @@ cudaError_t launch_batch_stage(const KParams* d_params, const BatchTile* d_tiles
     }
 }
 
+cudaError_t launch_member_stage(const KParams& P, int N, cudaStream_t s) {
+    switch (N) {
+        case 3: return launch_N<3>(P, true, 1, -1, s);
+        case 4: return launch_N<4>(P, true, 1, -1, s);
+        case 5: return launch_N<5>(P, true, 1, -1, s);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 int batch_resident_ctas(int N) {
     switch (N) {
         case 3: return resident_N<3>();
