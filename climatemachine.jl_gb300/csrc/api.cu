@@ -70,6 +70,7 @@ static int issue_steps(Model* md, void* Q, double* dQ, double dt, int nsteps, cu
             a.mode = 1;
             a.first_stage = (st == 0);
             a.last_stage = (st == 4);
+            a.backward = st & 1;
             int rc = launch_stage(md, a, s);
             if (rc) return rc;
         }

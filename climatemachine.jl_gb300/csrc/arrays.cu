@@ -44,7 +44,7 @@ struct ArraysSmem {
 // closure at N = 4 (93-96 registers, no spills; at 6 the closure
 // kernels spilled 24-116 bytes; a mixed Smagorinsky LES of 24 x 24 x 12
 // elements through grid arrays steps in 0.762 ms against 0.766 ms).
-template <int N, typename R, bool MIXED, int MODE, int VT = CMDG_TURB_NONE>
+template <int N, typename R, bool MIXED, int MODE, int VT = CMDG_TURB_NONE, bool BACK = false>
 __global__ void __launch_bounds__(ShellDims<N>::NT,
                                   MIXED ? (VT != CMDG_TURB_NONE && N == 4 ? 4 : ShellDims<N>::MIN_CTAS)
                                         : ShellDims<N>::MIN_CTAS64)
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     R* const s_D = sm + SM::DMAT;
 
     const int t = threadIdx.x;
-    const int e = blockIdx.x;
+    const int e = element_of<BACK>();
     const R* __restrict__ Qin = static_cast<const R*>(P.Qin);
     R* __restrict__ Qout = static_cast<R*>(P.Qout);
     const R* __restrict__ ge = static_cast<const R*>(P.geo) + (size_t)e * GSTRIDE;
@@ -324,17 +324,22 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     if (__any_sync(0xffffffffu, bad) && (t & 31) == 0) atomicOr(P.status, 1u);
 }
 
-template <int N, typename R, bool MIXED, int MODE, int VT>
+template <int N, typename R, bool MIXED, int MODE, int VT, bool BACK = false>
 cudaError_t launch_arrays_typed(const KParams& P, cudaStream_t s) {
     constexpr size_t bytes = ArraysSmem<N, R>::BYTES;
-    cudaError_t e = opt_in_smem(arrays_stage_kernel<N, R, MIXED, MODE, VT>, bytes);
+    cudaError_t e = opt_in_smem(arrays_stage_kernel<N, R, MIXED, MODE, VT, BACK>, bytes);
     if (e != cudaSuccess) return e;
-    return launch_chained(s, arrays_stage_kernel<N, R, MIXED, MODE, VT>, (unsigned)P.nelem, ShellDims<N>::NT, bytes, P);
+    return launch_chained(s, arrays_stage_kernel<N, R, MIXED, MODE, VT, BACK>, (unsigned)P.nelem, ShellDims<N>::NT, bytes, P);
 }
 
 // closures run FP64 on grid-arrays meshes (cmdg_model_create)
 template <int N, int VT>
 cudaError_t launch_arrays_VT(const KParams& P, bool mixed, int mode, cudaStream_t s) {
+    if constexpr (VT == CMDG_TURB_NONE) {
+        if (mode != 0 && P.backward)
+            return mixed ? launch_arrays_typed<N, float, true, 1, VT, true>(P, s)
+                         : launch_arrays_typed<N, double, false, 1, VT, true>(P, s);
+    }
     if (mixed)
         return mode == 0 ? launch_arrays_typed<N, float, true, 0, VT>(P, s) : launch_arrays_typed<N, float, true, 1, VT>(P, s);
     return mode == 0 ? launch_arrays_typed<N, double, false, 0, VT>(P, s)

@@ -267,6 +267,7 @@ static int upload_params(Batch* b, void* const* Q, double* const* dQ, const doub
             a.mode = 1;
             a.first_stage = st == 0;
             a.last_stage = st == 4;
+            a.backward = st & 1;
             host[st * n + m] = make_params(b->members[m], a);
         }
     }

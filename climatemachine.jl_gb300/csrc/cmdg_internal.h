@@ -275,6 +275,7 @@ struct LaunchArgs {
     int mode;                // 0 = tendency, 1 = RK stage
     int first_stage = 0;     // stage 1: the register is not read (A_1 = 0)
     int last_stage = 0;      // stage 5: the register is not written
+    int backward = 0;        // stage mode: the elements are walked from the last one to the first
     int remainder = 0;       // tendency mode on a mixed cubed shell: f - l of the vertical linear model
 };
 int launch_stage(Model* md, const LaunchArgs& a, cudaStream_t s);

@@ -91,7 +91,7 @@ struct ShellSmem {
 // GCM with horizontal DryBiharmonic steps in 0.595 ms against 0.612 ms at 4
 // and 0.629 ms at 6, which spills); 4 with a closure (24-56 bytes of
 // spills at 5) and with hyperdiffusion at other N.
-template <int N, typename R, bool MIXED, int MODE, bool HYPER, int VT, bool REM = false>
+template <int N, typename R, bool MIXED, int MODE, bool HYPER, int VT, bool REM = false, bool BACK = false>
 __global__ void __launch_bounds__(ShellDims<N>::NT,
                                   MIXED ? (HYPER && VT == 0 && N == 4 ? 5
                                                                       : (HYPER || VT != 0 ? 4 : ShellDims<N>::MIN_CTAS))
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     R* const s_D = sm + SM::DMAT;
 
     const int t = threadIdx.x;
-    const int e = blockIdx.x;
+    const int e = element_of<BACK>();
     const R* __restrict__ Qin = static_cast<const R*>(P.Qin);
     R* __restrict__ Qout = static_cast<R*>(P.Qout);
     const R* __restrict__ ge = static_cast<const R*>(P.geo) + (size_t)e * GSTRIDE;
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     if (__any_sync(0xffffffffu, bad) && (t & 31) == 0) atomicOr(P.status, 1u);
 }
 
-template <int N, typename R, bool MIXED, int MODE, bool HYPER, int VT, bool REM = false>
+template <int N, typename R, bool MIXED, int MODE, bool HYPER, int VT, bool REM = false, bool BACK = false>
 cudaError_t launch_shell_typed(const KParams& P, cudaStream_t s) {
     constexpr size_t bytes = ShellSmem<N, R>::BYTES;
     static unsigned long long configured = 0;
@@ -462,16 +462,21 @@ cudaError_t launch_shell_typed(const KParams& P, cudaStream_t s) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (!(configured & (1ull << (dev & 63)))) {
-        e = cudaFuncSetAttribute(shell_stage_kernel<N, R, MIXED, MODE, HYPER, VT, REM>,
+        e = cudaFuncSetAttribute(shell_stage_kernel<N, R, MIXED, MODE, HYPER, VT, REM, BACK>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
         if (e != cudaSuccess) return e;
         configured |= 1ull << (dev & 63);
     }
-    return launch_chained(s, shell_stage_kernel<N, R, MIXED, MODE, HYPER, VT, REM>, (unsigned)P.nelem, ShellDims<N>::NT, bytes, P);
+    return launch_chained(s, shell_stage_kernel<N, R, MIXED, MODE, HYPER, VT, REM, BACK>, (unsigned)P.nelem, ShellDims<N>::NT, bytes, P);
 }
 
 template <int N, bool HYPER, int VT>
 cudaError_t launch_shell_N(const KParams& P, bool mixed, int mode, cudaStream_t s) {
+    if constexpr (!HYPER && VT == CMDG_TURB_NONE) {
+        if (mode != 0 && P.backward)
+            return mixed ? launch_shell_typed<N, float, true, 1, false, VT, false, true>(P, s)
+                         : launch_shell_typed<N, double, false, 1, false, VT, false, true>(P, s);
+    }
     if (mixed)
         return mode == 0 ? launch_shell_typed<N, float, true, 0, HYPER, VT>(P, s)
                          : launch_shell_typed<N, float, true, 1, HYPER, VT>(P, s);

@@ -579,11 +579,16 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
     }
 }
 
-template <int N, typename R, bool MIXED, int MODE, bool PERSIST>
+template <int N, typename R, bool MIXED, int MODE, bool PERSIST, bool BACK = false>
 __global__ void __launch_bounds__(Dims<N>::NT, MIXED ? (PERSIST ? Dims<N>::MIN_CTAS : Dims<N>::MIN_CTAS_DIRECT)
                                                      : Dims<N>::MIN_CTAS64) stage_kernel(const KParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    stage_body<N, R, MIXED, MODE, PERSIST, false>(P, smem_raw, blockIdx.x, PERSIST ? gridDim.x : P.nelem, P.nelem);
+    if constexpr (PERSIST) {
+        stage_body<N, R, MIXED, MODE, true, false>(P, smem_raw, blockIdx.x, gridDim.x, P.nelem);
+    } else {
+        const int e = element_of<BACK>();
+        stage_body<N, R, MIXED, MODE, false, false>(P, smem_raw, e, 1, e + 1);
+    }
 }
 
 // One CTA per element in clusters of CL CTAs that are adjacent elements
@@ -645,7 +650,7 @@ cudaError_t launch_cluster_N(const KParams& P, bool mixed, int mode, int cl, cud
                  : launch_cluster_typed<N, double, false, 2>(P, mode, s);
 }
 
-template <int N, typename R, bool MIXED, int MODE, bool PERSIST>
+template <int N, typename R, bool MIXED, int MODE, bool PERSIST, bool BACK = false>
 cudaError_t launch_mode(const KParams& P, int grid_ctas, cudaStream_t s) {
     constexpr size_t bytes = PERSIST ? SmemTma<N, R>::BYTES : Smem<N, R>::BYTES;
     // per-device set-up: opt in to > 48 KB of dynamic shared memory and size a
@@ -657,12 +662,12 @@ cudaError_t launch_mode(const KParams& P, int grid_ctas, cudaStream_t s) {
     dev &= 63;
     if (resident[dev] == 0) {
         if (bytes > 48 * 1024) {
-            e = cudaFuncSetAttribute(stage_kernel<N, R, MIXED, MODE, PERSIST>,
+            e = cudaFuncSetAttribute(stage_kernel<N, R, MIXED, MODE, PERSIST, BACK>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
             if (e != cudaSuccess) return e;
         }
         int per_sm = 0, sms = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stage_kernel<N, R, MIXED, MODE, PERSIST>,
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, stage_kernel<N, R, MIXED, MODE, PERSIST, BACK>,
                                                           Dims<N>::NT, bytes);
         if (e != cudaSuccess) return e;
         e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -671,14 +676,16 @@ cudaError_t launch_mode(const KParams& P, int grid_ctas, cudaStream_t s) {
     }
     int grid = PERSIST ? (grid_ctas > 0 ? grid_ctas : resident[dev]) : P.nelem;
     if (grid > P.nelem) grid = P.nelem;
-    return launch_chained(s, stage_kernel<N, R, MIXED, MODE, PERSIST>, (unsigned)grid, Dims<N>::NT, bytes, P);
+    return launch_chained(s, stage_kernel<N, R, MIXED, MODE, PERSIST, BACK>, (unsigned)grid, Dims<N>::NT, bytes, P);
 }
 
 template <int N, typename R, bool MIXED>
 cudaError_t launch_typed(const KParams& P, int mode, int grid, cudaStream_t s) {
     // grid < 0 selects one CTA per element; otherwise the persistent kernel
     if (grid < 0)
-        return mode == 0 ? launch_mode<N, R, MIXED, 0, false>(P, 0, s) : launch_mode<N, R, MIXED, 1, false>(P, 0, s);
+        return mode == 0    ? launch_mode<N, R, MIXED, 0, false>(P, 0, s)
+               : P.backward ? launch_mode<N, R, MIXED, 1, false, true>(P, 0, s)
+                            : launch_mode<N, R, MIXED, 1, false>(P, 0, s);
     return mode == 0 ? launch_mode<N, R, MIXED, 0, true>(P, grid, s) : launch_mode<N, R, MIXED, 1, true>(P, grid, s);
 }
 
@@ -807,6 +814,7 @@ KParams make_params(Model* md, const LaunchArgs& a) {
     P.cl_elem = md->d_cl_elem;
     P.wait_polls = md->wait_polls;
     P.staging_skip_copies = md->staging_skip_copies;
+    P.backward = a.backward;
     return P;
 }
 

@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
     R* const s_F = s_node + P5N + planar_pad<R>(2 * Np);                    // total flux, 3 directions
     R* const s_fs = s_F + 3 * P5N;                                          // lifted face flux
 
-    const int e = blockIdx.x, t = threadIdx.x;
+    const int e = element_of<true>(), t = threadIdx.x;  // after the forward gradient pass
     const R* __restrict__ Qin = static_cast<const R*>(P.Qin);
     R* __restrict__ Qout = static_cast<R*>(P.Qout);
     const R* __restrict__ GF = static_cast<const R*>(P.gf);
