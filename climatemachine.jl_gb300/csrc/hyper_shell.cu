@@ -469,7 +469,11 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
 
 template <int N, typename R, bool MIXED, bool CART>
 cudaError_t launch_shell_passes_typed(const KParams& P, const void* Q, void* hd, void* hl, cudaStream_t s) {
-    constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp, NFN = 6 * Nfp, NT = ShellDims<N>::NT;
+    constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp, NFN = 6 * Nfp;
+    // HorizontalDirection has no work for the xi3 faces' threads, the last ones
+    // (N = 4: four warps instead of five; the step above 280 -> 274 us)
+    constexpr int HT = ((Np > 4 * Nfp ? Np : 4 * Nfp) + 31) / 32 * 32;
+    const unsigned NT = P.hyper_horizontal ? HT : ShellDims<N>::NT;
     constexpr size_t b1 = sizeof(R) * (4 * Np + 4 * NFN + Nq * Nq);
     constexpr size_t b2 = sizeof(R) * (12 * Np + 4 * NFN + Nq * Nq);
     constexpr size_t b3 = sizeof(R) * (4 * Np + 4 * NFN + Nq * Nq);
