@@ -271,15 +271,18 @@ __device__ __forceinline__ double sqrt_r(double x) {
 }
 __device__ __forceinline__ float sqrt_r(float x) { return x * rsqrtf(x); }
 
-// finiteness and the larger of two non-negative values; in FP64 on the
-// integer pipe (comparisons of doubles issue on the FP64 pipe)
+// finiteness, and the larger of two non-negative values; in FP64 on the
+// integer pipe (comparisons of doubles issue on the FP64 pipe).  As fmax, the
+// larger one leaves a NaN for the other value: a NaN's bits, taken as
+// unsigned, lie above infinity's, whatever its sign.
 __device__ __forceinline__ bool finite_r(float x) { return isfinite(x); }
 __device__ __forceinline__ bool finite_r(double x) {
     return ((unsigned)__double2hiint(x) & 0x7FF00000u) != 0x7FF00000u;
 }
 __device__ __forceinline__ float max_nonneg(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ double max_nonneg(double a, double b) {
-    return __double_as_longlong(a) > __double_as_longlong(b) ? a : b;
+    const unsigned long long ia = __double_as_longlong(a), ib = __double_as_longlong(b), inf = 0x7FF0000000000000ull;
+    return ia <= inf && (ia > ib || ib > inf) ? a : b;
 }
 
 // Pointwise thermodynamics of dry air (PhaseDry: T = T0 + e_int/cv, p = rho R T,
