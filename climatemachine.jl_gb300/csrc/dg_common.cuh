@@ -237,39 +237,49 @@ __device__ __forceinline__ Level<float> load_level<float>(const KParams& P, int 
 // approximations (a few ulp), where every other operation already carries
 // FP32 rounding.  FP64: the pipe is the bound of every FP64 kernel (1/72 of
 // the FP32 rate), so the seed comes from the hardware's approximation
-// instructions (about 20 correct bits, off that pipe) and one step of
-// Householder's third-order iteration (the binomial series of (1 - h)^-1 and
-// (1 - h)^-1/2 about the seed, cut after h^2) takes its error e to e^3, under
-// FP64 rounding: 3 FP64 operations for a reciprocal, 5 for a root.  The
-// results stay within 2 ulp of the correctly rounded ones.
+// instructions, off that pipe.  They see and give 20 mantissa bits: an error
+// of at most 2^-19 (reciprocal) and 2^-19.4 (reciprocal root).
+//   1/x      3 FP64 operations: one step of Householder's third-order
+//            iteration (the binomial series of (1 - h)^-1 about the seed, cut
+//            after h^2) takes the seed's error e to e^3 <= 2^-57;
+//   sqrt(x)  5 operations: two simplified Newton steps (the slope 1 / (2
+//            sqrt(x)) taken from the seed in both) on the residual x - s^2,
+//            which an FMA gives exactly up to its own rounding, take e to
+//            3/2 e^3 <= 2^-57.6.
+// With the last FMA's rounding: within 0.57 ulp of the exact result (the root
+// below 2^-927, where the residual underflows, within 1 ulp).  Zeros,
+// infinities, NaN and negative radicands give the IEEE results; as the seeds
+// flush, subnormal arguments count as zeros and a reciprocal below the normal
+// range may be zero.  The cases are told apart by selects on the integer pipe: a
+// branch to the IEEE operations took the FP64 step of the 1 M-node bubble from
+// 1.663 to 1.788 ms (1.689 ms with those out of line).
 __device__ __forceinline__ double rcp_r(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
     const double h = fma(-x, y, 1.0);
-    return fma(y, fma(h, h, h), y);
+    const double r = fma(y, fma(h, h, h), y);
+    const bool normal = ((unsigned)__double2hiint(y) & 0x7FFFFFFFu) - 0x00100000u < 0x7FE00000u;
+    return normal ? r : y;
 }
 __device__ __forceinline__ float rcp_r(float x) { return __fdividef(1.0f, x); }
-// len = sqrt(x), rlen = 1 / sqrt(x) for x > 0
-__device__ __forceinline__ void sqrt_rsqrt_r(double x, double& len, double& rlen) {
+__device__ __forceinline__ double sqrt_r(double x) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double t = x * y;
-    const double h = fma(-t, y, 1.0);
-    const double g = h * fma(h, 0.375, 0.5);
-    len = fma(t, g, t);
-    rlen = fma(y, g, y);
-}
-__device__ __forceinline__ void sqrt_rsqrt_r(float x, float& len, float& rlen) {
-    len = x * rsqrtf(x);
-    rlen = __fdividef(1.0f, len);
-}
-// FP64: zero (and the subnormals the seed instruction flushes) gives zero
-__device__ __forceinline__ double sqrt_r(double x) {
-    double len, rlen;
-    sqrt_rsqrt_r(x, len, rlen);
-    return (unsigned)__double2hiint(x) >= 0x00100000u ? len : 0.0;
+    const double hy = __hiloint2double(__double2hiint(y) - 0x00100000, __double2loint(y));  // y / 2
+    double s = x * y;
+    s = fma(fma(-s, s, x), hy, s);
+    s = fma(fma(-s, s, x), hy, s);
+    const unsigned hi = (unsigned)__double2hiint(x);
+    s = hi == 0x7FF00000u ? x : s;
+    return (hi & 0x7FFFFFFFu) >= 0x00100000u ? s : 0.0;
 }
 __device__ __forceinline__ float sqrt_r(float x) { return x * rsqrtf(x); }
+// len = sqrt(x), rlen = 1 / sqrt(x)
+template <typename R>
+__device__ __forceinline__ void sqrt_rsqrt_r(R x, R& len, R& rlen) {
+    len = sqrt_r(x);
+    rlen = rcp_r(len);
+}
 
 // finiteness, and the larger of two non-negative values; in FP64 on the
 // integer pipe (comparisons of doubles issue on the FP64 pipe).  As fmax, the
