@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
 
     const int t = threadIdx.x;
     const int e = element_of<BACK>();
-    const R* __restrict__ Qin = static_cast<const R*>(P.Qin);
-    R* __restrict__ Qout = static_cast<R*>(P.Qout);
+    const R* Qin = static_cast<const R*>(P.Qin);
+    R* Qout = static_cast<R*>(P.Qout);
     const R* __restrict__ ge = static_cast<const R*>(P.geo) + (size_t)e * GSTRIDE;
     const Physics& ph = P.ph;
     const bool node_thread = t < Np;

@@ -73,7 +73,7 @@ __device__ __forceinline__ void hyper_args(const KParams& P, const R q[NSTATE], 
 
 template <int N, typename R, bool MIXED>
 __global__ void __launch_bounds__(VDims<N>::NT) hyper_grad_kernel(const KParams P, const void* Qv,
-                                                                  R* __restrict__ hg) {
+                                                                  R* hg) {
     using Ix = HypIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp, ESTRIDE = NSTATE * Np;
     extern __shared__ __align__(16) unsigned char smem_raw[];

@@ -200,7 +200,7 @@ __device__ __forceinline__ int shell_partner_level(const ShellIdx<N>& x, int ez,
 // the partner table) instead of the cubed shell (levels, orientation codes)
 template <int N, typename R, bool MIXED, bool PROJECT = true, int NA = 4, bool ARRAYS = false>
 __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(const KParams P, const void* Qv,
-                                                                            R* __restrict__ hg) {
+                                                                            R* hg) {
     using Ix = ShellIdx<N>;
     constexpr int Nq = Ix::Nq, Np = Ix::Np, Nfp = Ix::Nfp, NFN = 6 * Nfp, ESTRIDE = NSTATE * Np;
     constexpr int GSTRIDE = KG_NFIELDS * Np;

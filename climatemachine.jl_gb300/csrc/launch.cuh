@@ -9,6 +9,10 @@
 // before has finished and its writes are visible.  Before chain_wait a kernel
 // touches only what no kernel writes: its launch parameters and the model's
 // tables.  A kernel launched the ordinary way passes chain_wait at once.
+// For the same reason a chained kernel qualifies only tables __restrict__: of
+// a buffer that the kernel before still writes or reads the qualifier would
+// say that nothing else touches it, and the compiler could load from it before
+// chain_wait or through the non-coherent path.
 //
 // chain_release stands before a kernel's last phase, not at its start: with
 // an early release several small grids wait on the SMs at once and new CTAs

@@ -178,8 +178,8 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
     R* const s_D = sm + SM::DMAT;
 
     const int t = threadIdx.x;
-    const R* __restrict__ Qin = static_cast<const R*>(P.Qin);
-    R* __restrict__ Qout = static_cast<R*>(P.Qout);
+    const R* Qin = static_cast<const R*>(P.Qin);
+    R* Qout = static_cast<R*>(P.Qout);
     const Physics& ph = P.ph;
     const bool node_thread = t < Np;
     const bool face_thread = t < 6 * Nfp;

@@ -47,7 +47,7 @@ constexpr int grad_min_ctas() {
 
 template <int N, typename R, bool MIXED, bool SMAG, bool FLUX>
 __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
-    gradient_kernel(const KParams P, const void* Qv, R* __restrict__ gf) {
+    gradient_kernel(const KParams P, const void* Qv, R* gf) {
     using Dm = VDims<N>;
     constexpr int Nq = Dm::Nq, Np = Dm::Np, Nfp = Dm::Nfp, NFN = 6 * Nfp;
     constexpr int ESTRIDE = NSTATE * Np;

@@ -246,10 +246,10 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
     R* const s_fs = s_F + 3 * P5N;                                          // lifted face flux
 
     const int e = element_of<true>(), t = threadIdx.x;  // after the forward gradient pass
-    const R* __restrict__ Qin = static_cast<const R*>(P.Qin);
-    R* __restrict__ Qout = static_cast<R*>(P.Qout);
-    const R* __restrict__ GF = static_cast<const R*>(P.gf);
-    const R* __restrict__ HDS = static_cast<const R*>(P.hd);
+    const R* Qin = static_cast<const R*>(P.Qin);
+    R* Qout = static_cast<R*>(P.Qout);
+    const R* GF = static_cast<const R*>(P.gf);
+    const R* HDS = static_cast<const R*>(P.hd);
     constexpr bool VISC = TURB != CMDG_TURB_NONE;
     const Physics& ph = P.ph;
     const bool node_thread = t < Np, face_thread = t < 6 * Nfp;
