@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     }
     __syncthreads();
 
-    chain_release();
+    if (P.release & RELEASE_STAGE) chain_release();
 
     // ---------------- phase 3: volume contraction, face terms, source, update
     int bad = 0;
@@ -353,7 +353,31 @@ cudaError_t launch_arrays_N(const KParams& P, bool mixed, int mode, int turb, cu
     return launch_arrays_VT<N, CMDG_TURB_NONE>(P, mixed, mode, s);
 }
 
+template <int N, int VT>
+int arrays_ctas_VT(bool mixed) {
+    return mixed ? chain_ctas<arrays_stage_kernel<N, float, true, 1, VT>>(ShellDims<N>::NT, ArraysSmem<N, float>::BYTES)
+                 : chain_ctas<arrays_stage_kernel<N, double, false, 1, VT>>(ShellDims<N>::NT, ArraysSmem<N, double>::BYTES);
+}
+
+template <int N>
+int arrays_ctas_N(bool mixed, int turb) {
+    if (turb == CMDG_TURB_CONSTANT) return arrays_ctas_VT<N, CMDG_TURB_CONSTANT>(mixed);
+    if (turb == CMDG_TURB_SMAGORINSKY) return arrays_ctas_VT<N, CMDG_TURB_SMAGORINSKY>(mixed);
+    return arrays_ctas_VT<N, CMDG_TURB_NONE>(mixed);
+}
+
 }  // namespace
+
+int arrays_stage_ctas(const Model* md) {
+    const bool mixed = md->precision == CMDG_MIXED;
+    switch (md->mesh->N) {
+        case 2: return arrays_ctas_N<2>(mixed, md->prm.turbulence);
+        case 3: return arrays_ctas_N<3>(mixed, md->prm.turbulence);
+        case 4: return arrays_ctas_N<4>(mixed, md->prm.turbulence);
+        case 5: return arrays_ctas_N<5>(mixed, md->prm.turbulence);
+        default: return 0;
+    }
+}
 
 int launch_arrays_stage(Model* md, const LaunchArgs& a, cudaStream_t s) {
     const Mesh& m = *md->mesh;

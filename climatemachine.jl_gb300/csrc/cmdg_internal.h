@@ -1,6 +1,7 @@
 // Internal declarations shared by the libcmdg translation units.
 #pragma once
 
+#include <atomic>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -243,6 +244,9 @@ struct Model {
     // issuing the copies, and every wait gives up after wait_polls polls
     int staging_skip_copies = 0;
     int wait_polls = 0;              // 0 = the default limit
+    // which of a stage's kernels release the next one before they end
+    // (chain_flags), once they are known
+    std::atomic<int> release{-1};
 };
 
 // host-side setup (mesh.cpp, shell_mesh.cpp)

@@ -85,6 +85,7 @@ struct KParams {
     const int* cl_elem;
     int staging_skip_copies;
     int backward;  // host: which form of a kernel is launched (element_of)
+    int release;   // RELEASE_*: the kernel releases the next one before its last phase (chain_flags)
 };
 
 // A run of consecutive elements [e0, e1) of ensemble member `member`, of
@@ -103,6 +104,17 @@ cudaError_t launch_member_stage(const KParams& P, int N, cudaStream_t s);
 
 // Builds the launch arguments of a model (stage.cu).
 KParams make_params(Model* md, const LaunchArgs& a);
+// Kernels of a stage that release the next one (chain_releases): the stage
+// kernel, the pass before it (gradient, or the gradient of the Laplacian) and
+// the first two hyperdiffusion passes.  From the resident CTAs (chain_ctas) of
+// each kind of model's kernels: the stage kernel, or pass 1 to 3.
+enum { RELEASE_STAGE = 1, RELEASE_PASS = 2, RELEASE_HYPER1 = 4, RELEASE_HYPER2 = 8 };
+int chain_flags(Model* md);
+int viscous_ctas(const Model* md, int pass);
+int hyper_ctas(const Model* md, int pass);
+int shell_pass_ctas(const Model* md, int pass);
+int shell_stage_ctas(const Model* md);
+int arrays_stage_ctas(const Model* md);
 // Column-kernel launcher (column.cu); returns cudaErrorNotSupported when no
 // column instantiation exists for the model's N.
 cudaError_t launch_column(const KParams& P, int N, bool mixed, int mode, int grid, cudaStream_t s);

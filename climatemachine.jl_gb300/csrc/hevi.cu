@@ -70,6 +70,7 @@ struct LinParams {
     double alpha, beta;
     double kv;       // R_d / cv_d: p_L = kv rhoe + crho rho
     double D[64];    // D[kk * Nq + k] = d l_k / dxi at xi_kk
+    int release;    // chain_releases
 };
 
 struct LinNode {
@@ -162,7 +163,7 @@ __global__ void __launch_bounds__(128) linear_tendency_kernel(const LinParams P)
             lin_face(a, Pn, wall, n, F[3 * Nfp + ij], side ? flt : flb);
         }
     }
-    chain_release();
+    if (P.release) chain_release();
     double* Te = P.T + (size_t)e * 5 * Np;
     const bool unit_beta = __double_as_longlong(P.beta) == __double_as_longlong(1.0);
     const bool zero_beta = __double_as_longlong(P.beta) << 1 == 0;
@@ -679,7 +680,9 @@ int launch_linear_N(Model* md, const double* Q, double* T, double alpha, double 
     P.kv = p.R_d / p.cv_d;
     for (int i = 0; i < Nq * Nq; ++i) P.D[i] = m.D[i];
     const int64_t threads = m.nelem * (int64_t)m.Nfp;
-    CMDG_CUDA_CHECK(launch_chained(s, linear_tendency_kernel<Nq>, (unsigned)((threads + 127) / 128), 128, 0, P));
+    const unsigned grid = (unsigned)((threads + 127) / 128);
+    P.release = chain_releases(grid, chain_ctas<linear_tendency_kernel<Nq>>(128, 0, md->device));
+    CMDG_CUDA_CHECK(launch_chained(s, linear_tendency_kernel<Nq>, grid, 128, 0, P));
     return CMDG_OK;
 }
 

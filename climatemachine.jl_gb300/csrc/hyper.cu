@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_grad_kernel(const KParams 
         for (int s = 0; s < 3; ++s) s_dH[s * NFN + t] = w * Hp[s];
     }
     __syncthreads();
-    chain_release();
+    if (P.release & RELEASE_HYPER1) chain_release();
 
     if (x.node) {
         R g1[3] = {0, 0, 0}, g2[3] = {0, 0, 0}, g3[3] = {0, 0, 0};
@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_div_kernel(const KParams P
         for (int s = 0; s < 3; ++s) s_dF[s * NFN + t] = w * (nb >= 0 ? Gp[s] : s_G[(3 * s + x.fd) * Np + x.vM]);
     }
     __syncthreads();
-    chain_release();
+    if (P.release & RELEASE_HYPER2) chain_release();
 
     if (x.node) {
         R a1[3] = {0, 0, 0}, a2[3] = {0, 0, 0}, a3[3] = {0, 0, 0};
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams 
         for (int s = 0; s < 3; ++s) s_dL[s * NFN + t] = w * (nb >= 0 ? Lp[s] : s_L[s * Np + x.vM]);
     }
     __syncthreads();
-    chain_release();
+    if (P.release & RELEASE_PASS) chain_release();
 
     if (x.node) {
         R g1[3] = {0, 0, 0}, g2[3] = {0, 0, 0}, g3[3] = {0, 0, 0};
@@ -355,12 +355,17 @@ __global__ void __launch_bounds__(VDims<N>::NT) hyper_glap_kernel(const KParams 
     }
 }
 
+// shared memory of a pass that stages nw node words
+template <int N, typename R>
+constexpr size_t pass_bytes(int nw) {
+    constexpr int Nq = N + 1, Nfp = Nq * Nq;
+    return sizeof(R) * (size_t)(nw * Nq * Nfp + 3 * 6 * Nfp + Nq * Nq);
+}
+
 template <int N, typename R, bool MIXED>
 cudaError_t launch_passes_typed(const KParams& P, const void* Q, void* hd, void* hl, cudaStream_t s) {
-    constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp, NFN = 6 * Nfp, NT = VDims<N>::NT;
-    constexpr size_t b1 = sizeof(R) * (3 * Np + 3 * NFN + Nq * Nq);
-    constexpr size_t b2 = sizeof(R) * (9 * Np + 3 * NFN + Nq * Nq);
-    constexpr size_t b3 = sizeof(R) * (3 * Np + 3 * NFN + Nq * Nq);
+    constexpr int NT = VDims<N>::NT;
+    constexpr size_t b1 = pass_bytes<N, R>(3), b2 = pass_bytes<N, R>(9), b3 = b1;
     cudaError_t e;
     if ((e = opt_in(hyper_grad_kernel<N, R, MIXED>, b1)) != cudaSuccess) return e;
     if ((e = opt_in(hyper_div_kernel<N, R>, b2)) != cudaSuccess) return e;
@@ -379,7 +384,33 @@ cudaError_t launch_passes_N(const KParams& P, const void* Q, void* hd, void* hl,
                  : launch_passes_typed<N, double, false>(P, Q, hd, hl, s);
 }
 
+template <int N, typename R, bool MIXED>
+int pass_ctas_typed(int pass) {
+    constexpr unsigned NT = VDims<N>::NT;
+    return pass == 1   ? chain_ctas<hyper_grad_kernel<N, R, MIXED>>(NT, pass_bytes<N, R>(3))
+           : pass == 2 ? chain_ctas<hyper_div_kernel<N, R>>(NT, pass_bytes<N, R>(9))
+                       : chain_ctas<hyper_glap_kernel<N, R, MIXED>>(NT, pass_bytes<N, R>(3));
+}
+
+template <int N>
+int hyper_ctas_N(bool mixed, int turb, int pass) {
+    if (!pass) return vstage_ctas_N<N, true>(mixed, turb);
+    return mixed ? pass_ctas_typed<N, float, true>(pass) : pass_ctas_typed<N, double, false>(pass);
+}
+
 }  // namespace
+
+int hyper_ctas(const Model* md, int pass) {
+    const bool mixed = md->precision == CMDG_MIXED;
+    const int turb = md->prm.turbulence;
+    switch (md->mesh->N) {
+        case 2: return hyper_ctas_N<2>(mixed, turb, pass);
+        case 3: return hyper_ctas_N<3>(mixed, turb, pass);
+        case 4: return hyper_ctas_N<4>(mixed, turb, pass);
+        case 5: return hyper_ctas_N<5>(mixed, turb, pass);
+        default: return 0;
+    }
+}
 
 // Reference rows of the mixed-precision passes: with gz = the DG z-gradient
 // of the reference h_tot (VV_DHT_REF), lap = its weak-form divergence with

@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_grad_kernel(cons
         for (int s = 0; s < NA; ++s) s_dF[s * NFN + t] = w * Hp[s];
     }
     __syncthreads();
-    chain_release();
+    if (P.release & (PROJECT ? RELEASE_HYPER1 : RELEASE_PASS)) chain_release();
 
     if (x.node) {
         R g[3 * NA], Jx[9];
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_div_kernel(const
         for (int s = 0; s < 4; ++s) s_dF[s * NFN + t] = nb >= 0 ? wp * Gp[s] : w * s_Ft[(x.fd * 4 + s) * Np + x.vM];
     }
     __syncthreads();
-    chain_release();
+    if (P.release & RELEASE_HYPER2) chain_release();
 
     if (x.node) {
         R a[4] = {0, 0, 0, 0};
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
         for (int s = 0; s < 4; ++s) s_dF[s * NFN + t] = w * (nb >= 0 ? Lp[s] : s_L[s * Np + x.vM]);
     }
     __syncthreads();
-    chain_release();
+    if (P.release & RELEASE_PASS) chain_release();
 
     if (x.node) {
         R g[12], Jx[9];
@@ -467,16 +467,26 @@ __global__ void __launch_bounds__(ShellDims<N>::NT) shell_hyper_glap_kernel(cons
     }
 }
 
+// threads of a hyperdiffusion pass: HorizontalDirection has no work for the
+// xi3 faces' threads, the last ones (N = 4: four warps instead of five; the
+// step above 280 -> 274 us)
+template <int N>
+constexpr unsigned pass_threads(bool horizontal) {
+    constexpr int Nfp = (N + 1) * (N + 1), Np = (N + 1) * Nfp;
+    return horizontal ? ((Np > 4 * Nfp ? Np : 4 * Nfp) + 31) / 32 * 32 : ShellDims<N>::NT;
+}
+
+// shared memory of a pass that stages nw node words and nf face words
+template <int N, typename R>
+constexpr size_t pass_bytes(int nw, int nf) {
+    constexpr int Nq = N + 1, Nfp = Nq * Nq;
+    return sizeof(R) * (size_t)(nw * Nq * Nfp + nf * 6 * Nfp + Nq * Nq);
+}
+
 template <int N, typename R, bool MIXED, bool CART>
 cudaError_t launch_shell_passes_typed(const KParams& P, const void* Q, void* hd, void* hl, cudaStream_t s) {
-    constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp, NFN = 6 * Nfp;
-    // HorizontalDirection has no work for the xi3 faces' threads, the last ones
-    // (N = 4: four warps instead of five; the step above 280 -> 274 us)
-    constexpr int HT = ((Np > 4 * Nfp ? Np : 4 * Nfp) + 31) / 32 * 32;
-    const unsigned NT = P.hyper_horizontal ? HT : ShellDims<N>::NT;
-    constexpr size_t b1 = sizeof(R) * (4 * Np + 4 * NFN + Nq * Nq);
-    constexpr size_t b2 = sizeof(R) * (12 * Np + 4 * NFN + Nq * Nq);
-    constexpr size_t b3 = sizeof(R) * (4 * Np + 4 * NFN + Nq * Nq);
+    const unsigned NT = pass_threads<N>(P.hyper_horizontal != 0);
+    constexpr size_t b1 = pass_bytes<N, R>(4, 4), b2 = pass_bytes<N, R>(12, 4), b3 = b1;
     cudaError_t e;
     if ((e = opt_in(shell_hyper_grad_kernel<N, R, MIXED>, b1)) != cudaSuccess) return e;
     if ((e = opt_in(shell_hyper_div_kernel<N, R>, b2)) != cudaSuccess) return e;
@@ -492,8 +502,8 @@ cudaError_t launch_shell_passes_typed(const KParams& P, const void* Q, void* hd,
 // the viscous gradient pass: grad u, grad h_tot (Np, 12, nelem)
 template <int N, typename R, bool MIXED, int NA, bool ARRAYS = false>
 cudaError_t launch_shell_visc_typed(const KParams& P, const void* Q, void* gout, cudaStream_t s) {
-    constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp, NFN = 6 * Nfp, NT = ShellDims<N>::NT;
-    constexpr size_t b1 = sizeof(R) * (NA * Np + NA * NFN + Nq * Nq);
+    constexpr int NT = ShellDims<N>::NT;
+    constexpr size_t b1 = pass_bytes<N, R>(NA, NA);
     cudaError_t e;
     if ((e = opt_in(shell_hyper_grad_kernel<N, R, MIXED, false, NA, ARRAYS>, b1)) != cudaSuccess) return e;
     return launch_chained(s, shell_hyper_grad_kernel<N, R, MIXED, false, NA, ARRAYS>, (unsigned)P.nelem, NT, b1, P, Q,
@@ -572,7 +582,43 @@ cudaError_t launch_shell_passes(const KParams& P, int N, bool mixed, bool cart, 
     }
 }
 
+// resident CTAs of the viscous gradient pass, or of hyperdiffusion pass 1 to 3
+template <int N, typename R, bool MIXED, bool ARRAYS>
+int visc_pass_ctas(bool smag) {
+    return smag ? chain_ctas<shell_hyper_grad_kernel<N, R, MIXED, false, 5, ARRAYS>>(ShellDims<N>::NT, pass_bytes<N, R>(5, 5))
+                : chain_ctas<shell_hyper_grad_kernel<N, R, MIXED, false, 4, ARRAYS>>(ShellDims<N>::NT, pass_bytes<N, R>(4, 4));
+}
+
+template <int N, typename R, bool MIXED>
+int shell_pass_ctas_typed(const Model* md, int pass) {
+    if (md->prm.turbulence != CMDG_TURB_NONE) {
+        const bool smag = md->prm.turbulence == CMDG_TURB_SMAGORINSKY;
+        return md->mesh->kind == MESH_ARRAYS ? visc_pass_ctas<N, R, MIXED, true>(smag)
+                                             : visc_pass_ctas<N, R, MIXED, false>(smag);
+    }
+    const unsigned NT = pass_threads<N>(md->prm.hyper_direction == CMDG_DIR_HORIZONTAL);
+    return pass == 1   ? chain_ctas<shell_hyper_grad_kernel<N, R, MIXED>>(NT, pass_bytes<N, R>(4, 4))
+           : pass == 2 ? chain_ctas<shell_hyper_div_kernel<N, R>>(NT, pass_bytes<N, R>(12, 4))
+                       : chain_ctas<shell_hyper_glap_kernel<N, R, MIXED, false>>(NT, pass_bytes<N, R>(4, 4));
+}
+
+template <int N>
+int shell_pass_ctas_N(const Model* md, int pass) {
+    return md->precision == CMDG_MIXED ? shell_pass_ctas_typed<N, float, true>(md, pass)
+                                       : shell_pass_ctas_typed<N, double, false>(md, pass);
+}
+
 }  // namespace
+
+int shell_pass_ctas(const Model* md, int pass) {
+    switch (md->mesh->N) {
+        case 2: return shell_pass_ctas_N<2>(md, pass);
+        case 3: return shell_pass_ctas_N<3>(md, pass);
+        case 4: return shell_pass_ctas_N<4>(md, pass);
+        case 5: return shell_pass_ctas_N<5>(md, pass);
+        default: return 0;
+    }
+}
 
 // nu_4 per node from the curl-invariant metric (lengthscale_horizontal:
 // |columns 1 and 2 of (dxi/dx)^-1| 2/N, averaged), the buffers of the

@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(ShellDims<N>::NT,
     }
     __syncthreads();
 
-    chain_release();
+    if (P.release & RELEASE_STAGE) chain_release();
 
     // ---------------- phase 3: volume contraction, face terms, source, update
     int bad = 0;
@@ -493,7 +493,33 @@ cudaError_t launch_shell_N(const KParams& P, bool mixed, int mode, bool hyper, i
     return launch_shell_N<N, false, CMDG_TURB_NONE>(P, mixed, mode, s);
 }
 
+template <int N, bool HYPER, int VT>
+int shell_ctas_VT(bool mixed) {
+    return mixed ? chain_ctas<shell_stage_kernel<N, float, true, 1, HYPER, VT>>(ShellDims<N>::NT, ShellSmem<N, float>::BYTES)
+                 : chain_ctas<shell_stage_kernel<N, double, false, 1, HYPER, VT>>(ShellDims<N>::NT,
+                                                                                  ShellSmem<N, double>::BYTES);
+}
+
+template <int N>
+int shell_ctas_N(bool mixed, bool hyper, int turb) {
+    if (hyper) return shell_ctas_VT<N, true, CMDG_TURB_NONE>(mixed);
+    if (turb == CMDG_TURB_CONSTANT) return shell_ctas_VT<N, false, CMDG_TURB_CONSTANT>(mixed);
+    if (turb == CMDG_TURB_SMAGORINSKY) return shell_ctas_VT<N, false, CMDG_TURB_SMAGORINSKY>(mixed);
+    return shell_ctas_VT<N, false, CMDG_TURB_NONE>(mixed);
+}
+
 }  // namespace
+
+int shell_stage_ctas(const Model* md) {
+    const bool mixed = md->precision == CMDG_MIXED, hyper = md->prm.hyperdiffusion != CMDG_HYPER_NONE;
+    switch (md->mesh->N) {
+        case 2: return shell_ctas_N<2>(mixed, hyper, md->prm.turbulence);
+        case 3: return shell_ctas_N<3>(mixed, hyper, md->prm.turbulence);
+        case 4: return shell_ctas_N<4>(mixed, hyper, md->prm.turbulence);
+        case 5: return shell_ctas_N<5>(mixed, hyper, md->prm.turbulence);
+        default: return 0;
+    }
+}
 
 bool shell_remainder_supported(const Model* md) {
     return md->mesh->kind == MESH_SHELL && md->precision == CMDG_MIXED && md->prm.ref_state &&

@@ -161,7 +161,7 @@ __device__ __forceinline__ double dhat_const<double>(const KParams& P, int idx) 
 
 template <int N, typename R, bool MIXED, int MODE, bool PERSIST, bool PARAM_D, int CL = 0>
 __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem_raw, int e_first, int e_stride,
-                                           int e_end) {
+                                           int e_end, int release) {
     static_assert(CL == 0 || CL == 2 || CL == 4 || CL == 8, "clusters of 2 (z), 4 (x, z) or 8 (x, y, z) elements");
     static_assert(CL == 0 || !PERSIST, "a cluster CTA computes one element");
     using Dm = Dims<N>;
@@ -477,7 +477,7 @@ __device__ __forceinline__ void stage_body(const KParams& P, unsigned char* smem
         if constexpr (CL > 0) cg::this_cluster().sync();
         else __syncthreads();
 
-        chain_release();
+        if (release) chain_release();
 
         // ---------------- phase 3: volume contraction, face terms, source, update
         int bad = 0;
@@ -584,10 +584,10 @@ __global__ void __launch_bounds__(Dims<N>::NT, MIXED ? (PERSIST ? Dims<N>::MIN_C
                                                      : Dims<N>::MIN_CTAS64) stage_kernel(const KParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if constexpr (PERSIST) {
-        stage_body<N, R, MIXED, MODE, true, false>(P, smem_raw, blockIdx.x, gridDim.x, P.nelem);
+        stage_body<N, R, MIXED, MODE, true, false>(P, smem_raw, blockIdx.x, gridDim.x, P.nelem, P.release & RELEASE_STAGE);
     } else {
         const int e = element_of<BACK>();
-        stage_body<N, R, MIXED, MODE, false, false>(P, smem_raw, e, 1, e + 1);
+        stage_body<N, R, MIXED, MODE, false, false>(P, smem_raw, e, 1, e + 1, P.release & RELEASE_STAGE);
     }
 }
 
@@ -602,7 +602,7 @@ __global__ void __launch_bounds__(Dims<N>::NT, MIXED ? Dims<N>::MIN_CTAS_DIRECT 
     stage_cluster_kernel(const KParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int e = __ldg(P.cl_elem + blockIdx.x);
-    stage_body<N, R, MIXED, MODE, false, true, CL>(P, smem_raw, e, 1, e + 1);
+    stage_body<N, R, MIXED, MODE, false, true, CL>(P, smem_raw, e, 1, e + 1, P.release & RELEASE_STAGE);
 }
 
 template <int N, typename R, bool MIXED, int MODE, int CL>
@@ -711,12 +711,13 @@ constexpr int batch_min_ctas() {
 
 template <int N>
 __global__ void __launch_bounds__(Dims<N>::NT, batch_min_ctas<N>())
-    batch_stage_kernel(const KParams* __restrict__ params, const BatchTile* __restrict__ tiles, int ntiles) {
+    batch_stage_kernel(const KParams* __restrict__ params, const BatchTile* __restrict__ tiles, int ntiles,
+                       int release) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     chain_wait();
     for (int it = blockIdx.x; it < ntiles; it += gridDim.x) {
         const BatchTile T = tiles[it];
-        stage_body<N, float, true, 1, false, false>(params[T.member], smem_raw, T.e0, 1, T.e1);
+        stage_body<N, float, true, 1, false, false>(params[T.member], smem_raw, T.e0, 1, T.e1, release);
     }
 }
 
@@ -732,7 +733,14 @@ cudaError_t launch_batch_N(const KParams* d_params, const BatchTile* d_tiles, in
         if (e != cudaSuccess) return e;
         configured |= 1ull << (dev & 63);
     }
-    return launch_chained(s, batch_stage_kernel<N>, (unsigned)grid, Dims<N>::NT, bytes, d_params, d_tiles, ntiles);
+    return launch_chained(s, batch_stage_kernel<N>, (unsigned)grid, Dims<N>::NT, bytes, d_params, d_tiles, ntiles,
+                          chain_releases(grid, chain_ctas<batch_stage_kernel<N>>(Dims<N>::NT, bytes, dev)));
+}
+
+template <int N>
+int stage_ctas_N(bool mixed) {
+    return mixed ? chain_ctas<stage_kernel<N, float, true, 1, false, false>>(Dims<N>::NT, Smem<N, float>::BYTES)
+                 : chain_ctas<stage_kernel<N, double, false, 1, false, false>>(Dims<N>::NT, Smem<N, double>::BYTES);
 }
 
 template <int N>
@@ -749,6 +757,36 @@ int resident_N() {
 }
 
 }  // namespace
+
+static int brick_stage_ctas(const Model* md) {
+    const bool mixed = md->precision == CMDG_MIXED;
+    switch (md->mesh->N) {
+        case 2: return stage_ctas_N<2>(mixed);
+        case 3: return stage_ctas_N<3>(mixed);
+        case 4: return stage_ctas_N<4>(mixed);
+        case 5: return stage_ctas_N<5>(mixed);
+        default: return 0;
+    }
+}
+
+int chain_flags(Model* md) {
+    const int known = md->release.load(std::memory_order_relaxed);
+    if (known >= 0) return known;
+    const bool hyper = md->prm.hyperdiffusion != CMDG_HYPER_NONE, visc = md->prm.turbulence != CMDG_TURB_NONE;
+    const int kind = md->mesh->kind;
+    auto ctas = [&](int pass) {
+        if (kind != MESH_BRICK)
+            return pass ? shell_pass_ctas(md, pass) : kind == MESH_SHELL ? shell_stage_ctas(md) : arrays_stage_ctas(md);
+        return hyper ? hyper_ctas(md, pass) : visc ? viscous_ctas(md, pass) : brick_stage_ctas(md);
+    };
+    const int64_t grid = md->mesh->nelem;
+    int flags = chain_releases(grid, ctas(hyper || visc ? 1 : 0)) ? RELEASE_STAGE : 0;
+    if ((hyper || visc) && chain_releases(grid, ctas(0))) flags |= RELEASE_PASS;
+    if (hyper && chain_releases(grid, ctas(2))) flags |= RELEASE_HYPER1;
+    if (hyper && chain_releases(grid, ctas(3))) flags |= RELEASE_HYPER2;
+    md->release.store(flags, std::memory_order_relaxed);
+    return flags;
+}
 
 KParams make_params(Model* md, const LaunchArgs& a) {
     const Mesh& m = *md->mesh;
@@ -815,6 +853,7 @@ KParams make_params(Model* md, const LaunchArgs& a) {
     P.wait_polls = md->wait_polls;
     P.staging_skip_copies = md->staging_skip_copies;
     P.backward = a.backward;
+    P.release = chain_flags(md);
     return P;
 }
 

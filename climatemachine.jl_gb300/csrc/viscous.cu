@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
     }
     __syncthreads();
 
-    chain_release();
+    if (P.release & RELEASE_PASS) chain_release();
 
     // phase 3: volume gradient (strong form), face terms, reference part, transform
     if (node_thread) {
@@ -224,10 +224,15 @@ __global__ void __launch_bounds__(VDims<N>::NT, grad_min_ctas<N, R>())
 }
 
 
+template <int N, typename R>
+constexpr size_t grad_bytes() {
+    constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp;
+    return sizeof(R) * (planar_pad<R>(5 * Np) + planar_pad<R>(30 * Nfp) + Nq * Nq);
+}
+
 template <int N, typename R, bool MIXED, bool SMAG, bool FLUX>
 cudaError_t launch_grad_kernel(const KParams& P, const void* Q, void* gf, cudaStream_t s) {
-    constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp;
-    constexpr size_t bytes = sizeof(R) * (planar_pad<R>(5 * Np) + planar_pad<R>(30 * Nfp) + Nq * Nq);
+    constexpr size_t bytes = grad_bytes<N, R>();
     auto k = gradient_kernel<N, R, MIXED, SMAG, FLUX>;
     cudaError_t e;
     if ((e = opt_in(k, bytes)) != cudaSuccess) return e;
@@ -250,7 +255,32 @@ cudaError_t launch_grad_N(const KParams& P, const void* Q, void* gf, bool mixed,
                  : launch_grad_typed<N, double, false>(P, Q, gf, turb, flux, s);
 }
 
+template <int N, typename R, bool MIXED>
+int grad_ctas_typed(int turb) {
+    return turb == CMDG_TURB_SMAGORINSKY
+               ? chain_ctas<gradient_kernel<N, R, MIXED, true, true>>(VDims<N>::NT, grad_bytes<N, R>())
+               : chain_ctas<gradient_kernel<N, R, MIXED, false, true>>(VDims<N>::NT, grad_bytes<N, R>());
+}
+
+template <int N>
+int viscous_ctas_N(bool mixed, int turb, int pass) {
+    if (!pass) return vstage_ctas_N<N, false>(mixed, turb);
+    return mixed ? grad_ctas_typed<N, float, true>(turb) : grad_ctas_typed<N, double, false>(turb);
+}
+
 }  // namespace
+
+int viscous_ctas(const Model* md, int pass) {
+    const bool mixed = md->precision == CMDG_MIXED;
+    const int turb = md->prm.turbulence;
+    switch (md->mesh->N) {
+        case 2: return viscous_ctas_N<2>(mixed, turb, pass);
+        case 3: return viscous_ctas_N<3>(mixed, turb, pass);
+        case 4: return viscous_ctas_N<4>(mixed, turb, pass);
+        case 5: return viscous_ctas_N<5>(mixed, turb, pass);
+        default: return 0;
+    }
+}
 
 int launch_gradient(Model* md, const void* Qin, void* gf_out, cudaStream_t s, bool flux) {
     const Mesh& m = *md->mesh;

@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(VDims<N>::NT, vstage_min_ctas<N, R, TURB, HYPE
     }
     __syncthreads();
 
-    chain_release();
+    if (P.release & RELEASE_STAGE) chain_release();
 
     // phase 3: volume contraction, face terms, source, update
     int bad = 0;
@@ -494,12 +494,16 @@ cudaError_t opt_in(K kernel, size_t bytes) {
 }
 
 
+template <int N, typename R>
+constexpr size_t vstage_bytes() {
+    constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp;
+    return sizeof(R) * (4 * planar_pad<R>(5 * Np) + planar_pad<R>(2 * Np) + planar_pad<R>(30 * Nfp) + Nq * Nq);
+}
+
 // Launches the stage kernel with second-order fluxes for closure `turb`.
 template <int N, typename R, bool MIXED, int MODE, bool HYPER>
 cudaError_t launch_vstage_typed(const KParams& P, int turb, cudaStream_t s) {
-    constexpr int Nq = N + 1, Nfp = Nq * Nq, Np = Nq * Nfp;
-    constexpr size_t bytes =
-        sizeof(R) * (4 * planar_pad<R>(5 * Np) + planar_pad<R>(2 * Np) + planar_pad<R>(30 * Nfp) + Nq * Nq);
+    constexpr size_t bytes = vstage_bytes<N, R>();
     cudaError_t e;
     if (turb == CMDG_TURB_SMAGORINSKY) {
         auto k = viscous_stage_kernel<N, R, MIXED, MODE, CMDG_TURB_SMAGORINSKY, HYPER>;
@@ -519,6 +523,24 @@ cudaError_t launch_vstage_typed(const KParams& P, int turb, cudaStream_t s) {
         }
     }
     return e;
+}
+
+// resident CTAs of that kernel (stage mode)
+template <int N, typename R, bool MIXED, bool HYPER>
+int vstage_ctas_typed(int turb) {
+    constexpr unsigned NT = VDims<N>::NT;
+    constexpr size_t bytes = vstage_bytes<N, R>();
+    if (turb == CMDG_TURB_SMAGORINSKY)
+        return chain_ctas<viscous_stage_kernel<N, R, MIXED, 1, CMDG_TURB_SMAGORINSKY, HYPER>>(NT, bytes);
+    if (turb == CMDG_TURB_CONSTANT)
+        return chain_ctas<viscous_stage_kernel<N, R, MIXED, 1, CMDG_TURB_CONSTANT, HYPER>>(NT, bytes);
+    if constexpr (HYPER) return chain_ctas<viscous_stage_kernel<N, R, MIXED, 1, CMDG_TURB_NONE, true>>(NT, bytes);
+    else return 0;
+}
+
+template <int N, bool HYPER>
+int vstage_ctas_N(bool mixed, int turb) {
+    return mixed ? vstage_ctas_typed<N, float, true, HYPER>(turb) : vstage_ctas_typed<N, double, false, HYPER>(turb);
 }
 
 template <int N, bool HYPER>
