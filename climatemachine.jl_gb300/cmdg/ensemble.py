@@ -78,9 +78,9 @@ class Ensemble:
         return {v: k for k, v in self.FAMILIES.items()}[f.value], c.value, t.value, g.value
 
     def autotune(self, Qs, dQs, reps=5):
-        """Times both families and keeps the faster.  Returns the ms per
-        stage launch of every candidate -- {3, 4, 5: the 10 per-order
-        tilings, "persistent": the 16 persistent candidates (CTA size 128
+        """Times steps of both families and keeps the faster.  Returns the ms
+        per stage of every candidate -- {3, 4, 5: the 10 per-order tilings of
+        the order's small members (0 where it has none), "persistent": the 16 persistent candidates (CTA size 128
         then 256, tile_elems 1, 2, 4, 8, grid one CTA per tile / one wave),
         "per_order": the whole per-order family} -- and the choice: the
         per-order tilings and {"kernel": get_kernel()}."""

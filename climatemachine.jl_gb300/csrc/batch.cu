@@ -128,8 +128,8 @@ static void spread_chains(Batch* b, std::vector<Chain> chains) {
     }
 }
 
-// Tiles of one order, chain by chain; within a set members interleaved,
-// tile_elems consecutive elements each.
+// Chains of one order, and the tiles of its sets, set by set: members
+// interleaved, tile_elems consecutive elements each.
 static int build_tiles(Batch* b, Group& g) {
     const int gi = (int)(&g - b->groups);
     std::vector<Chain> chains;
@@ -157,7 +157,7 @@ static int build_tiles(Batch* b, Group& g) {
             }
         }
         std::vector<int64_t> pos(j - i, 0);
-        for (bool more = true; more;) {
+        for (bool more = c.member < 0; more;) {
             more = false;
             for (size_t k = i; k < j; ++k) {
                 const Mesh& mesh = *b->members[mine[k]]->mesh;
@@ -313,35 +313,74 @@ static int launch_error(cudaError_t e) {
     return CMDG_ERR_CUDA;
 }
 
-// nsteps steps of every member: the first non-empty branch on s, the others
-// on their side streams, forked from and joined back into s.
-static int issue(Batch* b, int nsteps, cudaStream_t s) {
+// nsteps steps of a chain
+static cudaError_t issue_chain(Batch* b, const Chain& c, int nsteps, cudaStream_t s) {
+    for (int step = 0; step < nsteps; ++step)
+        for (int st = 0; st < 5; ++st) {
+            const cudaError_t e = launch_chain_stage(b, c, st, s);
+            if (e != cudaSuccess) return e;
+        }
+    return cudaSuccess;
+}
+
+// nsteps steps of every chain: the first non-empty branch on s, the others on
+// their side streams, forked from s (b->fork) and joined back by join_chains.
+static cudaError_t issue_chains(Batch* b, int nsteps, cudaStream_t s, std::vector<int>& joined) {
+    cudaError_t e = cudaSuccess;
+    bool first = true;
+    for (int i = 0; i < BATCH_NBRANCH; ++i) {
+        if (b->branches[i].empty()) continue;
+        cudaStream_t bs = first ? s : b->stream[i];
+        if (!first) {
+            if ((e = cudaStreamWaitEvent(bs, b->fork, 0)) != cudaSuccess) return e;
+            joined.push_back(i);
+        }
+        first = false;
+        for (const Chain& c : b->branches[i])
+            if ((e = issue_chain(b, c, nsteps, bs)) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+static cudaError_t join_chains(Batch* b, cudaStream_t s, const std::vector<int>& joined) {
+    cudaError_t e = cudaSuccess;
+    for (int i : joined) {
+        if ((e = cudaEventRecord(b->join[i], b->stream[i])) != cudaSuccess) return e;
+        if ((e = cudaStreamWaitEvent(s, b->join[i], 0)) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+static bool any_chain(const Batch* b) {
+    return std::any_of(b->branches, b->branches + BATCH_NBRANCH, [](const auto& br) { return !br.empty(); });
+}
+
+// one step of the persistent family
+static cudaError_t issue_unified(Batch* b, cudaStream_t s) {
     const size_t n = b->members.size();
+    const int grid = unified_grid(b->uni);
+    for (int st = 0; st < 5; ++st) {
+        const cudaError_t e = launch_ens_lines(b->d_params + st * n, b->uni.d_tiles, b->uni.ntiles, b->uni.cta_threads,
+                                               grid, b->uni.dhat, s);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+// nsteps steps of every member, the viscous ones on a branch of their own
+static int issue(Batch* b, int nsteps, cudaStream_t s) {
     bool first = true;
     cudaError_t e = cudaEventRecord(b->fork, s);
     if (e != cudaSuccess) return launch_error(e);
     std::vector<int> joined;
     if (b->family == FAMILY_PERSISTENT && b->uni.ntiles) {
-        const int grid = unified_grid(b->uni);
         for (int step = 0; step < nsteps; ++step)
-            for (int st = 0; st < 5; ++st)
-                if ((e = launch_ens_lines(b->d_params + st * n, b->uni.d_tiles, b->uni.ntiles, b->uni.cta_threads,
-                                          grid, b->uni.dhat, s)) != cudaSuccess)
-                    return launch_error(e);
+            if ((e = issue_unified(b, s)) != cudaSuccess) return launch_error(e);
         first = false;
     }
-    for (int i = 0; i < BATCH_NBRANCH; ++i) {
-        if (b->branches[i].empty() || b->family != FAMILY_PER_ORDER) continue;
-        cudaStream_t bs = first ? s : b->stream[i];
-        if (!first) {
-            if ((e = cudaStreamWaitEvent(bs, b->fork, 0)) != cudaSuccess) return launch_error(e);
-            joined.push_back(i);
-        }
+    if (b->family == FAMILY_PER_ORDER && any_chain(b)) {
+        if ((e = issue_chains(b, nsteps, s, joined)) != cudaSuccess) return launch_error(e);
         first = false;
-        for (const Chain& c : b->branches[i])
-            for (int step = 0; step < nsteps; ++step)
-                for (int st = 0; st < 5; ++st)
-                    if ((e = launch_chain_stage(b, c, st, bs)) != cudaSuccess) return launch_error(e);
     }
     if (!b->viscous.empty()) {
         cudaStream_t vs = first ? s : b->visc_stream;
@@ -373,10 +412,7 @@ static int issue(Batch* b, int nsteps, cudaStream_t s) {
             if ((e = cudaStreamWaitEvent(s, b->visc_join, 0)) != cudaSuccess) return launch_error(e);
         }
     }
-    for (int i : joined) {
-        if ((e = cudaEventRecord(b->join[i], b->stream[i])) != cudaSuccess) return launch_error(e);
-        if ((e = cudaStreamWaitEvent(s, b->join[i], 0)) != cudaSuccess) return launch_error(e);
-    }
+    if ((e = join_chains(b, s, joined)) != cudaSuccess) return launch_error(e);
     return CMDG_OK;
 }
 
@@ -602,44 +638,23 @@ extern "C" int cmdg_batch_lsrk54_step(cmdg_batch* batch, void* const* h_Q, doubl
     return CMDG_OK;
 }
 
-// One stage launch of every chain of the per-order family, on the branches as
-// in issue(), with the parameters of stage index 1.
-static cudaError_t per_order_stage(Batch* b, cudaStream_t s) {
-    cudaError_t e = cudaEventRecord(b->fork, s);
-    if (e != cudaSuccess) return e;
-    bool first = true;
-    std::vector<int> joined;
-    for (int i = 0; i < BATCH_NBRANCH; ++i) {
-        if (b->branches[i].empty()) continue;
-        cudaStream_t bs = first ? s : b->stream[i];
-        if (!first) {
-            if ((e = cudaStreamWaitEvent(bs, b->fork, 0)) != cudaSuccess) return e;
-            joined.push_back(i);
-        }
-        first = false;
-        for (const Chain& c : b->branches[i])
-            if ((e = launch_chain_stage(b, c, 1, bs)) != cudaSuccess) return e;
-    }
-    for (int i : joined) {
-        if ((e = cudaEventRecord(b->join[i], b->stream[i])) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(s, b->join[i], 0)) != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-}
-
-// Autotuner.  On stage launches that leave the members' states unchanged
-// (B dt = 0 on copies of the states; the RK register is overwritten, which
-// the next step ignores because stage 1 does not read it) it times
-//   the per-order family: for each order tile_elems in {1, 2, 4, 8, 16} x
-//   grid in {one CTA per tile, one wave of resident CTAs}, keeping each
-//   order's fastest for its sets of small members, then the whole family
+// Autotuner.  It times whole steps that leave the members' states unchanged
+// (B dt = 0, the last stage into a stage buffer; the RK register is
+// overwritten, which the next step ignores because stage 1 does not read it),
+// issued as a call issues them and, on a stream of its own, replayed from a
+// graph:
+//   the per-order family: for each order with sets of small members
+//   tile_elems in {1, 2, 4, 8, 16} x grid in {one CTA per tile, one wave of
+//   resident CTAs} on those sets, keeping the fastest, then the whole family
 //   (every chain on its branch);
 //   the persistent family: CTA size in {128, 256} threads (elements per CTA
 //   pass and nodes per thread of each order follow from it) x tile_elems in
 //   {1, 2, 4, 8} x grid in {one CTA per tile, one wave of resident CTAs};
-// and keeps the faster family with its fastest tiling.  h_ms receives ms per
-// stage launch: [order 3, 4, 5][10 per-order candidates] (0 for an order
-// without members), then the 16 persistent candidates, then the whole
+// and keeps the faster family with its fastest tiling.  A stage of every chain
+// before the next stage of any, which the tuner timed before, pays L2 misses
+// that the chains avoid: 64 uneven members 2.23 ms per step, which take 2.02.
+// h_ms receives ms per stage: [order 3, 4, 5][10 per-order candidates] (0 for
+// an order without sets), then the 16 persistent candidates, then the whole
 // per-order family; n_candidates = 47.
 extern "C" int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* const* h_dQ, int reps, double* h_ms,
                                    int h_ms_len, int* n_candidates, void* stream) {
@@ -651,16 +666,14 @@ extern "C" int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* 
     std::vector<double> unit_dt(n, 1.0);
     int rc = upload_params(b, h_Q, h_dQ, unit_dt.data(), true, s);
     if (rc) return rc;
-    {
-        KParams* const host = b->params.data() + n;
-        for (size_t m = 0; m < n; ++m) {
-            host[m].rkb_dt = 0.0;
-            host[m].rkb_dt32 = 0.0f;
-        }
-        CMDG_CUDA_CHECK(cudaMemcpyAsync(b->d_params + n, host, sizeof(KParams) * n, cudaMemcpyHostToDevice, s));
-        for (size_t m = 0; m < n; ++m)
-            CMDG_CUDA_CHECK(cudaMemcpyAsync(b->scratch[m], h_Q[m], b->state_bytes[m], cudaMemcpyDeviceToDevice, s));
+    b->cur_Q.clear();  // the next step re-uploads its real parameters
+    for (size_t i = 0; i < 5 * n; ++i) {
+        KParams& P = b->params[i];
+        P.rkb_dt = 0.0;
+        P.rkb_dt32 = 0.0f;
+        if (i >= 4 * n) P.Qout = b->scratch[i - 4 * n];
     }
+    CMDG_CUDA_CHECK(cudaMemcpyAsync(b->d_params, b->params.data(), sizeof(KParams) * 5 * n, cudaMemcpyHostToDevice, s));
     const int tiles[5] = {1, 2, 4, 8, 16};
     const int grids[2] = {-1, 0};
     constexpr int NC = 10, NU = 16, NTOT = BATCH_NGROUPS * NC + NU + 1;
@@ -668,20 +681,39 @@ extern "C" int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* 
     cudaEvent_t t0, t1;
     CMDG_CUDA_CHECK(cudaEventCreate(&t0));
     CMDG_CUDA_CHECK(cudaEventCreate(&t1));
-    // times `reps` launches of fn (after one untimed launch), in ms per launch
+    // times `reps` steps issued by fn (after an untimed one), in ms per stage
     auto time_it = [&](auto fn, double& out) -> int {
+        cudaGraphExec_t graph = nullptr;
         cudaError_t e = cudaSuccess;
+        if (s) {
+            cudaGraph_t g = nullptr;
+            if ((e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return launch_error(e);
+            e = fn();
+            const cudaError_t ce = cudaStreamEndCapture(s, &g);
+            if (e == cudaSuccess) e = ce;
+            if (e == cudaSuccess) e = cudaGraphInstantiate(&graph, g, 0);
+            if (g) cudaGraphDestroy(g);
+        }
         for (int r = -1; r < reps && e == cudaSuccess; ++r) {
             if (r == 0) cudaEventRecord(t0, s);
-            e = fn();
+            e = graph ? cudaGraphLaunch(graph, s) : fn();
         }
         cudaEventRecord(t1, s);
         if (e == cudaSuccess) e = cudaEventSynchronize(t1);
+        if (graph) cudaGraphExecDestroy(graph);
         if (e != cudaSuccess) return launch_error(e);
         float el = 0;
         cudaEventElapsedTime(&el, t0, t1);
-        out = el / reps;
+        out = el / reps / 5;
         return CMDG_OK;
+    };
+    // a step of the sets of one order, on s
+    auto sets = [&](int gi) {
+        cudaError_t e = cudaSuccess;
+        for (const auto& br : b->branches)
+            for (const Chain& c : br)
+                if (c.group == gi && c.member < 0 && e == cudaSuccess) e = issue_chain(b, c, 1, s);
+        return e;
     };
     for (int gi = 0; gi < BATCH_NGROUPS && !rc; ++gi) {
         Group& g = b->groups[gi];
@@ -692,9 +724,7 @@ extern "C" int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* 
             g.tile_elems = tiles[c / 2];
             g.grid = grids[c % 2];
             if ((rc = build_tiles(b, g))) break;
-            const int grid = grid_of(g, g.ntiles);
-            rc = time_it([&] { return launch_batch_stage(b->d_params + n, g.d_tiles, g.ntiles, g.N, grid, s); },
-                         ms[gi * NC + c]);
+            rc = time_it([&] { return sets(gi); }, ms[gi * NC + c]);
             if (!rc && ms[gi * NC + c] < best) {
                 best = ms[gi * NC + c];
                 best_tile = g.tile_elems;
@@ -707,10 +737,16 @@ extern "C" int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* 
         if (!rc) rc = rc2;
     }
     double per_order = 0;
-    bool any_tiles = false;
-    for (const Group& g : b->groups) any_tiles |= g.ntiles > 0;
-    if (!rc && any_tiles) {
-        rc = time_it([&] { return per_order_stage(b, s); }, ms[BATCH_NGROUPS * NC + NU]);
+    const bool any_chains = any_chain(b);
+    if (!rc && any_chains) {
+        auto step = [&] {
+            std::vector<int> joined;
+            cudaError_t e = cudaEventRecord(b->fork, s);
+            if (e == cudaSuccess) e = issue_chains(b, 1, s, joined);
+            if (e == cudaSuccess) e = join_chains(b, s, joined);
+            return e;
+        };
+        rc = time_it(step, ms[BATCH_NGROUPS * NC + NU]);
         per_order = ms[BATCH_NGROUPS * NC + NU];
     }
     // the persistent family
@@ -723,10 +759,8 @@ extern "C" int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* 
         u.tile_elems = u_tiles[(c / 2) % 4];
         u.grid = grids[c % 2];
         if ((rc = build_unified_tiles(b))) break;
-        const int grid = unified_grid(u);
         double& out = ms[BATCH_NGROUPS * NC + c];
-        rc = time_it([&] { return launch_ens_lines(b->d_params + n, u.d_tiles, u.ntiles, u.cta_threads, grid, u.dhat, s); },
-                     out);
+        rc = time_it([&] { return issue_unified(b, s); }, out);
         if (!rc && out < best_u) {
             best_u = out;
             best_threads = u.cta_threads;
@@ -739,10 +773,9 @@ extern "C" int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* 
     u.grid = best_grid;
     const int rc3 = build_unified_tiles(b);
     if (!rc) rc = rc3;
-    if (!rc && any_tiles) b->family = (u.ntiles && best_u < per_order) ? FAMILY_PERSISTENT : FAMILY_PER_ORDER;
+    if (!rc && any_chains) b->family = (u.ntiles && best_u < per_order) ? FAMILY_PERSISTENT : FAMILY_PER_ORDER;
     cudaEventDestroy(t0);
     cudaEventDestroy(t1);
-    b->cur_Q.clear();  // the next step re-uploads its real parameters
     drop_graph(b);
     for (Model* md : b->members) cudaMemsetAsync(md->d_status, 0, sizeof(unsigned), s);
     if (n_candidates) *n_candidates = NTOT;

@@ -323,16 +323,17 @@ int cmdg_batch_lsrk54_step(cmdg_batch* batch, void* const* h_Q, double* const* h
 enum { CMDG_BATCH_PER_ORDER = 0, CMDG_BATCH_PERSISTENT = 1 };
 int cmdg_batch_set_kernel(cmdg_batch* batch, int family, int cta_threads, int tile_elems, int grid_ctas);
 int cmdg_batch_get_kernel(const cmdg_batch* batch, int* family, int* cta_threads, int* tile_elems, int* grid_ctas);
-/* Autotuner: times `reps` stage launches of every candidate on copies of the
- * members' states (the states are not changed; the RK registers are
- * overwritten, which the next step ignores): per order tile_elems {1, 2, 4,
- * 8, 16} x grid {one CTA per tile, one wave of resident CTAs}, keeping each
- * order's fastest, then the whole per-order family; and the persistent kernel
- * over cta_threads {128, 256} x tile_elems {1, 2, 4, 8} x grid {one CTA per
- * tile, one wave}.  Keeps the faster family with its fastest tiling.  h_ms
- * receives ms per stage launch: [order 3, 4, 5][10 per-order candidates] (0
- * for an order without members), the 16 persistent candidates, the whole
- * per-order family (n_candidates = 47). */
+/* Autotuner: times `reps` steps of every candidate (the states are not
+ * changed; the RK registers are overwritten, which the next step ignores),
+ * issued as a call issues them, on stream != NULL from a graph: per order with
+ * sets of small members, on those sets, tile_elems {1, 2, 4, 8, 16} x grid
+ * {one CTA per tile, one wave of resident CTAs}, keeping each order's fastest,
+ * then the whole per-order family; and the persistent kernel over cta_threads
+ * {128, 256} x tile_elems {1, 2, 4, 8} x grid {one CTA per tile, one wave}.
+ * Keeps the faster family with its fastest tiling.  h_ms receives ms per
+ * stage (a fifth of a step): [order 3, 4, 5][10 per-order candidates] (0 for
+ * an order without sets), the 16 persistent candidates, the whole per-order
+ * family (n_candidates = 47). */
 int cmdg_batch_autotune(cmdg_batch* batch, void* const* h_Q, double* const* h_dQ, int reps, double* h_ms,
                         int h_ms_len, int* n_candidates, void* stream);
 
