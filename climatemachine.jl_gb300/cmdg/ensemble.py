@@ -1,9 +1,11 @@
 """Ensembles of mixed-precision models advanced together on one GPU.
 
 ``Ensemble(members)`` wraps ``cmdg_batch_*``.  Two kernel families advance
-the inviscid members: "per_order" (members grouped by polynomial order,
-every LSRK54 stage of a group one launch of a tile-walking kernel, the groups
-independent stream branches of one CUDA graph per call) and "persistent"
+the inviscid members: "per_order" (chains on three stream branches, each
+through all its stages before the next: a member of 64,000 nodes or more
+alone, by the one-model stage kernel; the smaller ones of an order in sets,
+one launch of a tile-walking kernel per set and stage; repeated calls on a
+stream of their own replay one CUDA graph) and "persistent"
 (one launch per stage of one kernel over tiles of every order, whose CTA
 size sets each order's elements per CTA pass and nodes per thread).  LES
 members (a turbulence closure) take their gradient and viscous stage kernels
@@ -50,8 +52,9 @@ class Ensemble:
         call("cmdg_batch_lsrk54_step", self.h, q, d, dt, int(nsteps), _stream())
 
     def set_tiling(self, tile_elems=1, grid_ctas=-1, N=0):
-        """Tiling of the members of order N (0 = all): elements per tile and
-        grid (-1 = one CTA per tile, 0 = one wave of resident CTAs)."""
+        """Tiling of the sets of small members of order N (0 = all): elements
+        per tile and grid (-1 = one CTA per tile, 0 = one wave of resident
+        CTAs).  Members of 64,000 nodes or more step alone and have none."""
         call("cmdg_batch_set_tiling", self.h, int(N), int(tile_elems), int(grid_ctas))
 
     def get_tiling(self):

@@ -1,12 +1,11 @@
 // Ensembles of models advanced together, by one of two kernel families:
-//   per order  the members are grouped by polynomial order; each LSRK54
-//              stage of a group is one launch of the tile-walking node kernel
-//              of that order (stage.cu), so small members share the GPU
-//              without a launch per member; members that fill it are chains
-//              of their own (Chain).  Members are independent, so the chains
-//              run on three streams: captured as one CUDA graph they are
-//              three independent branches that the GPU overlaps, joined at
-//              the end of the call;
+//   per order  the small members of a polynomial order step in sets, one
+//              launch of the tile-walking node kernel of that order (stage.cu)
+//              per set and LSRK54 stage, so that they share the GPU without a
+//              launch per member; members that fill it are chains of their own
+//              (Chain).  Members are independent, so the chains run on three
+//              streams: captured as one CUDA graph they are three independent
+//              branches that the GPU overlaps, joined at the end of the call;
 //   persistent one launch per stage of the line kernel (stage_lines.cu) over
 //              one list of tiles of every order, with one CTA shape for all
 //              orders: its size sets the elements per CTA pass and the nodes
@@ -47,8 +46,7 @@ struct Group {
 // states through L2 five times a step; a chain's working set stays there
 // from stage to stage (the sets are bounded accordingly).  And the one-model
 // kernel has its parameters in the constant bank: 56 registers and 7 CTAs per
-// SM at N = 4, against 72 with spills and 5 CTAs when they come from global
-// memory.  A step of 24 members (8 to 16 elements a side, N = 3 to 5), in us:
+// SM at N = 4, against 72 and 5 CTAs when they come from global memory.  A step of 24 members (8 to 16 elements a side, N = 3 to 5), in us:
 // 1371 stage by stage, 1267 in sets of up to 24 MB, 1343 of 48 MB, 898 member
 // by member.
 struct Chain {
@@ -60,11 +58,16 @@ struct Chain {
 // bytes a chain touches per node: three state buffers and the register
 constexpr size_t CHAIN_BYTES_PER_NODE = NSTATE * (3 * sizeof(float) + sizeof(double));
 constexpr size_t SET_BYTES = (size_t)24 << 20;
-// A member of at least this many nodes steps alone: below, five launches of its
-// own cost more than the better kernel gains.  24 equal members per step, one
-// by one against in sets, us: 32,768 nodes (N = 3) 268 / 196, 46,656 (N = 5)
-// 268 / 224, 64,000 (N = 3) 271 / 351, (N = 4) 270 / 338, 110,592 (N = 5)
-// 384 / 524; four members of 64,000 (N = 4) 64 / 65.
+// A member of at least this many nodes steps alone, with five launches of its
+// own per step.  On the default stream the launches bound small members: 24 take
+// 257 us per step one by one at any size up to 64,000 nodes (120 launches of
+// 2.1 us), in sets 195 (32,768 nodes, N = 3), 226 (46,656, N = 5), 259 (46,656,
+// N = 3), 342 (64,000, N = 4) and 524 (110,592, N = 5, alone 389): the kernels
+// cross near 50,000 nodes, and at the line members alone are the faster ones
+// from 2 to 48 of them.  Replayed from a graph, where a launch takes less, they
+// cross lower: 24 alone / in sets 169 / 196 (32,768), 213 / 226 (46,656, N = 5),
+// 240 / 341 (64,000, N = 4), but 156 / 87 (15,625, N = 4).  One line serves
+// both.
 constexpr int64_t ALONE_MIN_NODES = 64000;
 
 enum { FAMILY_PER_ORDER = 0, FAMILY_PERSISTENT = 1 };

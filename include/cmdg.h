@@ -283,11 +283,15 @@ int cmdg_lsrk54_step_noalloc(cmdg_model* model, void* d_Q, double* d_dQ, double 
                              void* stream);
 
 /* Ensembles.  A batch advances n mixed-precision brick models of any sizes
- * and polynomial orders N = 3..5 together.  Inviscid members are grouped by
- * order; each LSRK54 stage of a group is one launch of a tile-walking kernel
- * (a tile is a run of consecutive elements of one member), the groups' stage
- * chains run on their own streams, and the steps of a call are captured in one
- * CUDA graph (stream != NULL).  Members with a turbulence closure (LES
+ * and polynomial orders N = 3..5 together.  Inviscid members run in chains,
+ * each through all its stages before the next of its branch: a member of
+ * 64,000 nodes or more alone, one launch of the one-model stage kernel per
+ * stage; the smaller ones of an order in sets of up to 24 MB of states and
+ * registers, one launch of a tile-walking kernel per set and stage (a tile is a
+ * run of consecutive elements of one member).  The chains are spread over three
+ * branches on streams of their own.  On stream != NULL, calls that repeat (the
+ * same states, time steps, stream and nsteps <= 64) replay one captured CUDA
+ * graph.  Members with a turbulence closure (LES
  * members: ConstantDynamicViscosity or SmagorinskyLilly) take the gradient
  * pass and the viscous stage kernel at every stage, member by member, on a
  * further branch of the same graph.  The batch owns two stage buffers per
@@ -297,9 +301,10 @@ int cmdg_lsrk54_step_noalloc(cmdg_model* model, void* d_Q, double* d_dQ, double 
 typedef struct cmdg_batch cmdg_batch;
 int cmdg_batch_create(cmdg_model* const* models, int n, cmdg_batch** out);
 int cmdg_batch_destroy(cmdg_batch* batch);
-/* Tiling of the members of order N (0 = every order): tile_elems elements per
+/* Tiling of the sets of order N (0 = every order): tile_elems elements per
  * tile; grid_ctas -1 = one CTA per tile, 0 = one wave of resident CTAs,
- * n > 0 = n CTAs. */
+ * n > 0 = n CTAs.  It has no effect on members that step alone (64,000 nodes
+ * or more).  States do not depend on it. */
 int cmdg_batch_set_tiling(cmdg_batch* batch, int N, int tile_elems, int grid_ctas);
 int cmdg_batch_get_tiling(const cmdg_batch* batch, int N, int* tile_elems, int* grid_ctas);
 /* nsteps LSRK54 steps of every member; h_Q, h_dQ, h_dt: host arrays of n
@@ -308,8 +313,7 @@ int cmdg_batch_get_tiling(const cmdg_batch* batch, int N, int* tile_elems, int* 
 int cmdg_batch_lsrk54_step(cmdg_batch* batch, void* const* h_Q, double* const* h_dQ, const double* h_dt, int nsteps,
                            void* stream);
 /* Kernel family of the inviscid members:
- *   CMDG_BATCH_PER_ORDER  one tile-walking launch per order and stage, the
- *                         orders on independent branches (tiling per order:
+ *   CMDG_BATCH_PER_ORDER  the chains described above (tiling of the sets:
  *                         cmdg_batch_set_tiling);
  *   CMDG_BATCH_PERSISTENT one launch per stage of one persistent kernel over
  *                         tiles of every order with one CTA shape:
