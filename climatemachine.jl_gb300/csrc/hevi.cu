@@ -36,6 +36,7 @@
 // One thread per line keeps every lane of GB300's narrow FP64 pipe busy;
 // the substitutions skip the band entries that the element coupling makes
 // exact zeros (see fwd_len / bwd_len).
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -195,6 +196,7 @@ __global__ void __launch_bounds__(128) linear_tendency_kernel(const LinParams P)
 struct LineMap {
     int64_t nline;
     int nz, n;
+    int64_t line0;  // first line (set-up runs over parts of the lines)
 };
 
 // state index of unknown r of line `line`
@@ -202,8 +204,8 @@ template <int Nq>
 __device__ __forceinline__ size_t line_index(const LineMap& lm, int64_t line, int r) {
     constexpr int Nfp = Nq * Nq, Np = Nfp * Nq;
     const int s = r % 5, k = (r / 5) % Nq, v = r / (5 * Nq);
-    const int64_t col = line / Nfp;
-    const int ij = (int)(line % Nfp);
+    const int64_t col = (lm.line0 + line) / Nfp;
+    const int ij = (int)((lm.line0 + line) % Nfp);
     const int64_t e = v + (int64_t)lm.nz * col;
     return ((size_t)e * 5 + s) * Np + ij + Nfp * k;
 }
@@ -299,24 +301,6 @@ __global__ void band_pattern_kernel(double* AB, LineMap lm, int bw, unsigned* er
     if (bad) atomicOr(err, 4u);
 }
 
-// SingleColumnLU: every line's factors must equal the first line's to
-// rounding (entries within 1e-10 of the larger of the entry and the pivot
-// row's scale)
-__global__ void band_single_kernel(const double* AB, LineMap lm, int bw, unsigned* err) {
-    const int64_t line = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (line >= lm.nline) return;
-    const int nb = 2 * bw + 1;
-    bool bad = false;
-    for (int b = 0; b < nb; ++b)
-        for (int col = 0; col < lm.n; ++col) {
-            const size_t i0 = ((size_t)b * lm.n + col) * lm.nline;
-            const double v = AB[i0 + line], v0 = AB[i0];
-            const double scale = fabs(v0) + fabs(1.0 / AB[((size_t)bw * lm.n + col) * lm.nline]);
-            bad |= !(fabs(v - v0) <= 1e-10 * scale);
-        }
-    if (bad) atomicOr(err, 8u);
-}
-
 // The factors as the substitution reads them: only the structurally non-zero
 // entries, per group of L lines and element level v the forward entries of
 // the NB columns (distance 1, 2, ... below the pivot), then the backward ones
@@ -353,6 +337,29 @@ __global__ void band_pack_kernel(double* AB, double* F, LineMap lm, int L, int64
         dst[(size_t)(PK::fwd_off(p) + i - 1) * L] = col + i < lm.n ? band_at(AB, lm, PK::BW, line, col + i, col) : 0.0;
     for (int i = 0; i <= bwd_len(p, PK::BW); ++i)
         dst[(size_t)(PK::bwd_off(p) + i) * L] = col >= i ? band_at(AB, lm, PK::BW, line, col - i, col) : 0.0;
+}
+
+// SingleColumnLU: every line's factors must equal the first line's, packed in
+// F, to rounding (entries within 1e-10 of the larger of the entry and the
+// pivot row's scale)
+template <int Nq>
+__global__ void band_single_kernel(double* AB, const double* F, LineMap lm, unsigned* err) {
+    using PK = PackedLU<Nq>;
+    const int64_t line = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (line >= lm.nline) return;
+    bool bad = false;
+    for (int col = 0; col < lm.n; ++col) {
+        const int v = col / PK::NB, p = col % PK::NB;
+        const double* f = F + (size_t)v * PK::PER;
+        const double pivot = fabs(1.0 / f[PK::bwd_off(p)]);
+        auto check = [&](int row, double v0) {
+            const double a = band_at(AB, lm, PK::BW, line, row, col);
+            bad |= !(fabs(a - v0) <= 1e-10 * (fabs(v0) + pivot));
+        };
+        for (int i = 1; i <= fwd_len(p, PK::BW) && col + i < lm.n; ++i) check(col + i, f[PK::fwd_off(p) + i - 1]);
+        for (int i = 0; i <= bwd_len(p, PK::BW) && i <= col; ++i) check(col - i, f[PK::bwd_off(p) + i]);
+    }
+    if (bad) atomicOr(err, 8u);
 }
 
 // one warp per CTA: the column count is small (a few warps per SM), so the
@@ -664,22 +671,24 @@ int init_linear_tables(Model* md) {
     return CMDG_OK;
 }
 
+// the linear tendency of elements [e0, e0 + ne), whole columns (ne < 0: to the last element)
 template <int Nq>
-int launch_linear_N(Model* md, const double* Q, double* T, double alpha, double beta, cudaStream_t s) {
+int launch_linear_N(Model* md, const double* Q, double* T, double alpha, double beta, cudaStream_t s, int64_t e0 = 0,
+                    int64_t ne = -1) {
     const Mesh& m = *md->mesh;
     const cmdg_atmos_params& p = md->prm;
     LinParams P{};
-    P.Q = Q;
-    P.T = T;
-    P.lt = md->d_lin64;
-    P.lf = md->d_linface64;
-    P.nelem = m.nelem;
+    P.Q = Q + (size_t)e0 * 5 * m.Np;
+    P.T = T + (size_t)e0 * 5 * m.Np;
+    P.lt = md->d_lin64 + (size_t)e0 * LT_NFIELDS * m.Np;
+    P.lf = md->d_linface64 + (size_t)e0 * 2 * LF_NFIELDS * m.Nfp;
+    P.nelem = ne < 0 ? m.nelem - e0 : ne;
     P.nz = stack_height(md);
     P.alpha = alpha;
     P.beta = beta;
     P.kv = p.R_d / p.cv_d;
     for (int i = 0; i < Nq * Nq; ++i) P.D[i] = m.D[i];
-    const int64_t threads = m.nelem * (int64_t)m.Nfp;
+    const int64_t threads = P.nelem * (int64_t)m.Nfp;
     const unsigned grid = (unsigned)((threads + 127) / 128);
     P.release = chain_releases(grid, chain_ctas<linear_tendency_kernel<Nq>>(128, 0, md->device));
     CMDG_CUDA_CHECK(launch_chained(s, linear_tendency_kernel<Nq>, grid, 128, 0, P));
@@ -713,7 +722,7 @@ struct Hevi {
     LineMap lm{};
     int bw = 0;
     size_t len = 0;
-    double* d_AB = nullptr;   // set-up: band matrix, then its LU factors (reciprocal pivots), line-fastest
+    double* d_AB = nullptr;   // set-up: band matrix of a part of the lines, then its LU factors (reciprocal pivots), line-fastest
     int single = 0;           // SingleColumnLU: d_F holds the first line's factors
     double* d_F = nullptr;    // the factors as the substitution reads them (PackedLU)
     double* d_y = nullptr;    // the substitution's scratch, (n, 32) per warp of lines
@@ -730,46 +739,72 @@ struct Hevi {
 
 namespace {
 
+// The packed factors of every line.  The band storage that they are computed
+// in, 1.6 to 1.9 times their size, is taken for all lines at once if it fits
+// beside them, else for a quarter of the lines at a time and so on: the
+// factors of a mesh that nearly fills the device have to fit, not the band
+// (the 21,600 lines of the acoustic wave: 1.53 GB of band, 0.82 GB of factors).
 template <int Nq>
 int hevi_assemble_N(Hevi* h, cudaStream_t s) {
+    using PK = PackedLU<Nq>;
+    constexpr int Nfp = Nq * Nq, Np = Nfp * Nq;
     Model* md = h->md;
-    const Mesh& m = *md->mesh;
     double* E = h->Y();
     double* R = h->Qhat();
-    const size_t len = h->len;
     const double eps = -h->alpha;
-    const int64_t ntot = h->lm.nline * h->lm.n;
-    for (int vi = 0; vi < 3 && vi < h->lm.nz; ++vi)
-        for (int k = 0; k < Nq; ++k)
-            for (int st = 0; st < 5; ++st) {
-                unit_state_kernel<Nq><<<(unsigned)((len + 255) / 256), 256, 0, s>>>(E, m.nelem, h->lm.nz, vi, k, st);
-                int rc = launch_linear_N<Nq>(md, E, R, 1.0, 0.0, s);
-                if (rc) return rc;
-                band_scatter_kernel<Nq><<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(E, R, h->d_AB, h->lm, h->bw, vi,
-                                                                                       k, st, eps, h->d_err);
-                CMDG_CUDA_CHECK(cudaGetLastError());
-            }
-    band_lu_kernel<<<(unsigned)((h->lm.nline + 127) / 128), 128, 0, s>>>(h->d_AB, h->lm, h->bw, h->d_err);
-    CMDG_CUDA_CHECK(cudaGetLastError());
-    band_pattern_kernel<<<(unsigned)((h->lm.nline + 127) / 128), 128, 0, s>>>(h->d_AB, h->lm, h->bw, h->d_err);
-    CMDG_CUDA_CHECK(cudaGetLastError());
-    if (h->single) {
-        band_single_kernel<<<(unsigned)((h->lm.nline + 127) / 128), 128, 0, s>>>(h->d_AB, h->lm, h->bw, h->d_err);
-        CMDG_CUDA_CHECK(cudaGetLastError());
-    }
-    // the factors in the substitution's layout
+    const int nz = h->lm.nz, n = h->lm.n;
+    const int64_t nline = h->lm.nline;
     const int L = h->single ? 1 : SOLVE_THREADS;
-    const int64_t nlines = h->single ? 1 : h->lm.nline, groups = (nlines + L - 1) / L;
-    const size_t entries = (size_t)groups * h->lm.nz * PackedLU<Nq>::PER * L;
-    const int64_t warps = (h->lm.nline + SOLVE_THREADS - 1) / SOLVE_THREADS;
-    if (cudaMalloc(&h->d_F, sizeof(double) * entries) != cudaSuccess ||
-        cudaMalloc(&h->d_y, sizeof(double) * (size_t)warps * SOLVE_THREADS * h->lm.n) != cudaSuccess) {
-        cudaGetLastError();
-        set_error("allocation of the column factors (%zu bytes) failed", sizeof(double) * entries);
+    const size_t group = (size_t)nz * PK::PER * L;  // factors of L lines
+    const int64_t warps = (nline + SOLVE_THREADS - 1) / SOLVE_THREADS;
+    const size_t band = sizeof(double) * (2 * PK::BW + 1) * n, factors = sizeof(double) * group * (h->single ? 1 : warps);
+    int64_t part = nline;
+    bool ok = cudaMalloc(&h->d_F, factors) == cudaSuccess &&
+              cudaMalloc(&h->d_y, sizeof(double) * (size_t)warps * SOLVE_THREADS * n) == cudaSuccess;
+    while (ok && cudaMalloc(&h->d_AB, band * part) != cudaSuccess) {
+        h->d_AB = nullptr;
+        ok = part > SOLVE_THREADS;
+        part = ((part + 3) / 4 + SOLVE_THREADS - 1) / SOLVE_THREADS * SOLVE_THREADS;
+    }
+    cudaGetLastError();
+    if (!ok) {
+        set_error("HEVI: device allocation of the column factors (%zu bytes, and a part of the band's %zu) failed", factors,
+                  band * (size_t)nline);
         return CMDG_ERR_ALLOC;
     }
-    band_pack_kernel<Nq><<<(unsigned)((nlines * h->lm.n + 127) / 128), 128, 0, s>>>(h->d_AB, h->d_F, h->lm, L, nlines);
-    CMDG_CUDA_CHECK(cudaGetLastError());
+    for (int64_t line0 = 0; line0 < nline; line0 += part) {
+        const LineMap lm{std::min(part, nline - line0), nz, n, line0};
+        // the elements of the columns that hold these lines
+        const int64_t e0 = line0 / Nfp * nz, ne = ((line0 + lm.nline + Nfp - 1) / Nfp) * nz - e0;
+        const int64_t len = ne * 5 * Np, ntot = lm.nline * n;
+        const unsigned per_line = (unsigned)((lm.nline + 127) / 128);
+        CMDG_CUDA_CHECK(cudaMemsetAsync(h->d_AB, 0, band * lm.nline, s));
+        for (int vi = 0; vi < 3 && vi < nz; ++vi)
+            for (int k = 0; k < Nq; ++k)
+                for (int st = 0; st < 5; ++st) {
+                    unit_state_kernel<Nq><<<(unsigned)((len + 255) / 256), 256, 0, s>>>(E + e0 * 5 * Np, ne, nz, vi, k, st);
+                    const int rc = launch_linear_N<Nq>(md, E, R, 1.0, 0.0, s, e0, ne);
+                    if (rc) return rc;
+                    band_scatter_kernel<Nq><<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(E, R, h->d_AB, lm, PK::BW, vi, k,
+                                                                                           st, eps, h->d_err);
+                    CMDG_CUDA_CHECK(cudaGetLastError());
+                }
+        band_lu_kernel<<<per_line, 128, 0, s>>>(h->d_AB, lm, PK::BW, h->d_err);
+        CMDG_CUDA_CHECK(cudaGetLastError());
+        band_pattern_kernel<<<per_line, 128, 0, s>>>(h->d_AB, lm, PK::BW, h->d_err);
+        CMDG_CUDA_CHECK(cudaGetLastError());
+        // into the substitution's layout; of SingleColumnLU the first line alone
+        const int64_t nlines = h->single ? (line0 == 0) : lm.nline;
+        if (nlines) {
+            band_pack_kernel<Nq><<<(unsigned)((nlines * n + 127) / 128), 128, 0, s>>>(
+                h->d_AB, h->d_F + (line0 / L) * group, lm, L, nlines);
+            CMDG_CUDA_CHECK(cudaGetLastError());
+        }
+        if (h->single) {
+            band_single_kernel<Nq><<<per_line, 128, 0, s>>>(h->d_AB, h->d_F, lm, h->d_err);
+            CMDG_CUDA_CHECK(cudaGetLastError());
+        }
+    }
     return CMDG_OK;
 }
 
@@ -947,21 +982,18 @@ int cmdg_hevi_create(cmdg_model* model, double dt, int split_explicit_implicit, 
     h->lm.nline = (m.nelem / nz) * m.Nfp;
     h->bw = 5 * m.Nq - 1;
     h->len = (size_t)m.nelem * 5 * m.Np;
-    const size_t ab = (size_t)(2 * h->bw + 1) * h->lm.n * h->lm.nline;
-    cudaError_t e1 = cudaMalloc(&h->d_AB, sizeof(double) * ab);
     cudaError_t e2 = cudaMalloc(&h->d_buf, sizeof(double) * 7 * h->len);
     cudaError_t e3 = cudaMalloc(&h->d_err, sizeof(unsigned));
     cudaError_t e4 = md->precision == CMDG_MIXED ? cudaMalloc(&h->d_Sp, sizeof(float) * h->len) : cudaSuccess;
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess) {
+    if (e2 != cudaSuccess || e3 != cudaSuccess || e4 != cudaSuccess) {
         cudaGetLastError();
         cmdg_hevi_destroy(ho);
-        set_error("HEVI: device allocation of %zu bytes failed", sizeof(double) * (ab + 7 * h->len));
+        set_error("HEVI: device allocation of %zu bytes failed", sizeof(double) * 7 * h->len);
         return CMDG_ERR_ALLOC;
     }
     cudaStream_t s = 0;
     rc = CMDG_OK;
-    if (cudaMemsetAsync(h->d_AB, 0, sizeof(double) * ab, s) != cudaSuccess ||
-        cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), s) != cudaSuccess) {
+    if (cudaMemsetAsync(h->d_err, 0, sizeof(unsigned), s) != cudaSuccess) {
         set_error("HEVI: cudaMemsetAsync failed");
         rc = CMDG_ERR_CUDA;
     }

@@ -398,7 +398,10 @@ int cmdg_apply_mp_filter(cmdg_model* model, void* d_Q, const double* h_Wh, const
  * single_column = 1 is SingleColumnLU(): one factorization (the first
  * line's) serves every line; refused with CMDG_ERR_ARG unless all column
  * matrices agree to 1e-10 (e.g. an affine brick with level-dependent
- * coefficients).  Owns the factors and seven state-sized FP64 buffers.
+ * coefficients).  Owns the packed factors (54% to 63% of the band's bytes),
+ * seven state-sized FP64 buffers and an eighth in the substitution's order; a
+ * mixed model's solver also an FP32 state.  Set-up holds the band beside them
+ * if it fits, else of a quarter of the lines at a time and so on.
  * cmdg_hevi_solve: besolver!(Q, Qhat, alpha): d_Q = d_Qhat + alpha L(d_Q)
  * (BackwardEulerSolvers.jl; linearsolve! columnwise_lu_solver.jl:110-127,
  * 615-780); d_Q may alias d_Qhat.
