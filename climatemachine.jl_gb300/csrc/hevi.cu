@@ -367,10 +367,7 @@ __global__ void band_single_kernel(double* AB, const double* F, LineMap lm, unsi
 constexpr int SOLVE_THREADS = 32;
 
 // columns ahead whose factor entries are prefetched into L2
-#ifndef CMDG_SOLVE_PREFETCH
-#define CMDG_SOLVE_PREFETCH 6
-#endif
-constexpr int SOLVE_PREFETCH = CMDG_SOLVE_PREFETCH;
+constexpr int SOLVE_PREFETCH = 6;
 
 // band_forward! then band_back! (Golub & Van Loan Alg. 4.3.2, 4.3.3), one
 // thread per line (all lanes do useful FP64 work).  The window of bw + 1
@@ -395,6 +392,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS) band_solve_kernel(const double*
                                                                    double* y, double* out, LineMap lm,
                                                                    int accumulate) {
     static_assert(L == 1 || L == SOLVE_THREADS, "a warp reads one group of lines, or the same line");
+    static_assert(SOLVE_PREFETCH < PackedLU<Nq>::NB, "prefetches reach into the next level, not past it");
     using PK = PackedLU<Nq>;
     constexpr int NB = PK::NB, BW = PK::BW, Nfp = Nq * Nq, Np = Nfp * Nq;
     constexpr size_t FV = (size_t)PK::PER * L, QV = (size_t)5 * Np, YV = (size_t)NB * SOLVE_THREADS;
