@@ -131,6 +131,29 @@ WORKLOADS = {
 }
 
 
+def hevi_factor_entries(N):
+    """Entries of the column LU that the substitution reads per line and element
+    level: L and U of an element's block, which is dense, and of the coupling of
+    the facing node layers of two elements, 5 x 5 each; the diagonal once
+    (reciprocal pivots)."""
+    nb = 5 * (N + 1)
+    return nb * nb + 2 * 5 * 5
+
+
+def ensemble_launches(members, alone=64000, set_bytes=24 << 20, node_bytes=100):
+    """Stage launches of one step's stage of an ensemble's inviscid members, given
+    as (N, nodes): one per member of at least `alone` nodes, and one per set of
+    the smaller members of an order, filled in their order up to `set_bytes`."""
+    n = sum(nodes >= alone for _, nodes in members)
+    for N in sorted({N for N, _ in members}):
+        size = 0
+        for nodes in (m for k, m in members if k == N and m < alone):
+            if size == 0 or size + nodes * node_bytes > set_bytes:
+                n, size = n + 1, 0
+            size += nodes * node_bytes
+    return n
+
+
 def measure_ensemble(args, cmdg, workloads, torch, barrier, stream, flush):
     """64 seeded bubble members (8^3..16^3 elements, N = 3..5), mixed:
     batched steps (one CUDA graph per call, the tiling the autotuner picks)
@@ -193,10 +216,12 @@ def measure_ensemble(args, cmdg, workloads, torch, barrier, stream, flush):
                                       "persistent_best": min(cand_ms["persistent"])},
             "roofline": {"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                          "peak_source": peak_kind,
-                         "kernel": ("ens_lines_kernel (one persistent launch per stage, every order)"
-                                    if persistent else "batch_stage_kernel<N> (one launch per order and stage)"),
+                         "kernel": ("ens_lines_kernel (one persistent launch per stage, every order)" if persistent else
+                                    "stage_kernel<N> (members of 64,000 nodes or more, a launch each per stage) and "
+                                    "batch_stage_kernel<N> (sets of the smaller ones)"),
                          "bytes_per_node_stage": BYTES_MIXED},
-            "gpu_launches": args.steps * NSTAGE * (1 if persistent else 3), "clocks": clk.summary()}
+            "gpu_launches": args.steps * NSTAGE * (1 if persistent else ensemble_launches(
+                [(dg.grid.N, dg.grid.nelem * dg.grid.Np) for dg in dgs])), "clocks": clk.summary()}
 
 
 def bench_ensemble(args, cmdg, workloads, torch, barrier, stream, flush):
@@ -331,10 +356,8 @@ def bench_hevi(args, cmdg, workloads, torch, barrier, stream, flush):
     dg64, _, _, Q64, ark64 = setup("fp64")
     nodes = dg.grid.nelem * dg.grid.Np
     nz = dg.grid.ne[2]
-    NB = 5 * (dg.grid.N + 1)
-    fwd = sum(NB - 1 - max(0, p - 5) for p in range(NB))
-    bwd = sum((NB - 1 if p < 5 else p) + 1 for p in range(NB))
-    solve_bytes = 8 * ark.nline * (fwd + bwd) * nz + 8 * 5 * nodes * 5  # factors + b, y (w, r), out (r, w)
+    # factors, and per unknown b, the scratch written and read back, and the result
+    solve_bytes = 8 * ark.nline * hevi_factor_entries(dg.grid.N) * nz + 8 * 5 * nodes * 4
 
     filt = ExponentialFilter(dg64.grid, 0, 18)
     with ClockSampler(int(os.environ.get("LOCAL_RANK", "0"))) as clk:
