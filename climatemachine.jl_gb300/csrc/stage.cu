@@ -46,7 +46,7 @@
 // SM), so its operations are counted: reciprocals and roots of 3 and 5
 // operations (rcp_r, sqrt_r), the metric folded into the derivative
 // coefficients, no diagonal in the contraction, comparisons on the integer
-// pipe.  A step of the 1 M-node bubble went from 2.304 to 1.677 ms (1.852 ms
+// pipe.  A step of the 1 M-node bubble went from 2.304 to 1.665 ms (1.852 ms
 // before the diagonal, and chained launches, launch.cuh).  In FP32 the same
 // identity saves the face threads five loads and ten operations (0.167 to
 // 0.164 ms).
