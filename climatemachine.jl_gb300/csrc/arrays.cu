@@ -355,8 +355,9 @@ cudaError_t launch_arrays_N(const KParams& P, bool mixed, int mode, int turb, cu
 
 template <int N, int VT>
 int arrays_ctas_VT(bool mixed) {
-    return mixed ? chain_ctas<arrays_stage_kernel<N, float, true, 1, VT>>(ShellDims<N>::NT, ArraysSmem<N, float>::BYTES)
-                 : chain_ctas<arrays_stage_kernel<N, double, false, 1, VT>>(ShellDims<N>::NT, ArraysSmem<N, double>::BYTES);
+    constexpr unsigned NT = ShellDims<N>::NT;
+    return mixed ? chain_ctas<arrays_stage_kernel<N, float, true, 1, VT>>(NT, ArraysSmem<N, float>::BYTES)
+                 : chain_ctas<arrays_stage_kernel<N, double, false, 1, VT>>(NT, ArraysSmem<N, double>::BYTES);
 }
 
 template <int N>

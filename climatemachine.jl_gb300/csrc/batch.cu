@@ -46,9 +46,9 @@ struct Group {
 // states through L2 five times a step; a chain's working set stays there
 // from stage to stage (the sets are bounded accordingly).  And the one-model
 // kernel has its parameters in the constant bank: 56 registers and 7 CTAs per
-// SM at N = 4, against 72 and 5 CTAs when they come from global memory.  A step of 24 members (8 to 16 elements a side, N = 3 to 5), in us:
-// 1371 stage by stage, 1267 in sets of up to 24 MB, 1343 of 48 MB, 898 member
-// by member.
+// SM at N = 4, against 72 and 5 CTAs when they come from global memory.  A step
+// of 24 members (8 to 16 elements a side, N = 3 to 5), in us: 1371 stage by
+// stage, 1267 in sets of up to 24 MB, 1343 of 48 MB, 898 member by member.
 struct Chain {
     int group;
     int member;  // -1 = a set

@@ -720,7 +720,7 @@ struct Hevi {
     LineMap lm{};
     int bw = 0;
     size_t len = 0;
-    double* d_AB = nullptr;   // set-up: band matrix of a part of the lines, then its LU factors (reciprocal pivots), line-fastest
+    double* d_AB = nullptr;   // set-up: band of a part of the lines, then its LU factors (reciprocal pivots), line-fastest
     int single = 0;           // SingleColumnLU: d_F holds the first line's factors
     double* d_F = nullptr;    // the factors as the substitution reads them (PackedLU)
     double* d_y = nullptr;    // the substitution's scratch, (n, 32) per warp of lines
@@ -755,7 +755,8 @@ int hevi_assemble_N(Hevi* h, cudaStream_t s) {
     const int L = h->single ? 1 : SOLVE_THREADS;
     const size_t group = (size_t)nz * PK::PER * L;  // factors of L lines
     const int64_t warps = (nline + SOLVE_THREADS - 1) / SOLVE_THREADS;
-    const size_t band = sizeof(double) * (2 * PK::BW + 1) * n, factors = sizeof(double) * group * (h->single ? 1 : warps);
+    const size_t band = sizeof(double) * (2 * PK::BW + 1) * n;
+    const size_t factors = sizeof(double) * group * (h->single ? 1 : warps);
     int64_t part = nline;
     bool ok = cudaMalloc(&h->d_F, factors) == cudaSuccess &&
               cudaMalloc(&h->d_y, sizeof(double) * (size_t)warps * SOLVE_THREADS * n) == cudaSuccess;
@@ -766,8 +767,8 @@ int hevi_assemble_N(Hevi* h, cudaStream_t s) {
     }
     cudaGetLastError();
     if (!ok) {
-        set_error("HEVI: device allocation of the column factors (%zu bytes, and a part of the band's %zu) failed", factors,
-                  band * (size_t)nline);
+        set_error("HEVI: device allocation of the column factors (%zu bytes, and a part of the band's %zu) failed",
+                  factors, band * (size_t)nline);
         return CMDG_ERR_ALLOC;
     }
     for (int64_t line0 = 0; line0 < nline; line0 += part) {
@@ -780,11 +781,12 @@ int hevi_assemble_N(Hevi* h, cudaStream_t s) {
         for (int vi = 0; vi < 3 && vi < nz; ++vi)
             for (int k = 0; k < Nq; ++k)
                 for (int st = 0; st < 5; ++st) {
-                    unit_state_kernel<Nq><<<(unsigned)((len + 255) / 256), 256, 0, s>>>(E + e0 * 5 * Np, ne, nz, vi, k, st);
+                    unit_state_kernel<Nq><<<(unsigned)((len + 255) / 256), 256, 0, s>>>(E + e0 * 5 * Np, ne, nz, vi, k,
+                                                                                        st);
                     const int rc = launch_linear_N<Nq>(md, E, R, 1.0, 0.0, s, e0, ne);
                     if (rc) return rc;
-                    band_scatter_kernel<Nq><<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(E, R, h->d_AB, lm, PK::BW, vi, k,
-                                                                                           st, eps, h->d_err);
+                    band_scatter_kernel<Nq><<<(unsigned)((ntot + 255) / 256), 256, 0, s>>>(E, R, h->d_AB, lm, PK::BW, vi,
+                                                                                           k, st, eps, h->d_err);
                     CMDG_CUDA_CHECK(cudaGetLastError());
                 }
         band_lu_kernel<<<per_line, 128, 0, s>>>(h->d_AB, lm, PK::BW, h->d_err);

@@ -585,8 +585,9 @@ cudaError_t launch_shell_passes(const KParams& P, int N, bool mixed, bool cart, 
 // resident CTAs of the viscous gradient pass, or of hyperdiffusion pass 1 to 3
 template <int N, typename R, bool MIXED, bool ARRAYS>
 int visc_pass_ctas(bool smag) {
-    return smag ? chain_ctas<shell_hyper_grad_kernel<N, R, MIXED, false, 5, ARRAYS>>(ShellDims<N>::NT, pass_bytes<N, R>(5, 5))
-                : chain_ctas<shell_hyper_grad_kernel<N, R, MIXED, false, 4, ARRAYS>>(ShellDims<N>::NT, pass_bytes<N, R>(4, 4));
+    constexpr unsigned NT = ShellDims<N>::NT;
+    return smag ? chain_ctas<shell_hyper_grad_kernel<N, R, MIXED, false, 5, ARRAYS>>(NT, pass_bytes<N, R>(5, 5))
+                : chain_ctas<shell_hyper_grad_kernel<N, R, MIXED, false, 4, ARRAYS>>(NT, pass_bytes<N, R>(4, 4));
 }
 
 template <int N, typename R, bool MIXED>

@@ -495,9 +495,9 @@ cudaError_t launch_shell_N(const KParams& P, bool mixed, int mode, bool hyper, i
 
 template <int N, bool HYPER, int VT>
 int shell_ctas_VT(bool mixed) {
-    return mixed ? chain_ctas<shell_stage_kernel<N, float, true, 1, HYPER, VT>>(ShellDims<N>::NT, ShellSmem<N, float>::BYTES)
-                 : chain_ctas<shell_stage_kernel<N, double, false, 1, HYPER, VT>>(ShellDims<N>::NT,
-                                                                                  ShellSmem<N, double>::BYTES);
+    constexpr unsigned NT = ShellDims<N>::NT;
+    return mixed ? chain_ctas<shell_stage_kernel<N, float, true, 1, HYPER, VT>>(NT, ShellSmem<N, float>::BYTES)
+                 : chain_ctas<shell_stage_kernel<N, double, false, 1, HYPER, VT>>(NT, ShellSmem<N, double>::BYTES);
 }
 
 template <int N>

@@ -584,7 +584,8 @@ __global__ void __launch_bounds__(Dims<N>::NT, MIXED ? (PERSIST ? Dims<N>::MIN_C
                                                      : Dims<N>::MIN_CTAS64) stage_kernel(const KParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if constexpr (PERSIST) {
-        stage_body<N, R, MIXED, MODE, true, false>(P, smem_raw, blockIdx.x, gridDim.x, P.nelem, P.release & RELEASE_STAGE);
+        stage_body<N, R, MIXED, MODE, true, false>(P, smem_raw, blockIdx.x, gridDim.x, P.nelem,
+                                                   P.release & RELEASE_STAGE);
     } else {
         const int e = element_of<BACK>();
         stage_body<N, R, MIXED, MODE, false, false>(P, smem_raw, e, 1, e + 1, P.release & RELEASE_STAGE);
