@@ -28,7 +28,9 @@
 // every CTA has ended, still ahead of an ordinary launch (16.0 / 17.9 us for
 // the 729 elements).  A grid of at most half the SMs releases too: both grids'
 // CTAs find SMs of their own (64 FP64 elements with hyperdiffusion, N = 4,
-// 133 / 139).  The element-wise kernels release first: a successor's
+// 133 / 139).  Of FP32 CTAs of two warps (N = 2) an SM issues two at once, and
+// grids of up to twice the SMs release (252 elements with hyperdiffusion 45.3 /
+// 48.8).  The element-wise kernels release first: a successor's
 // CTAs find their SMs evenly loaded.  One-wave kernels whose balance over the
 // SMs decides (the column substitution) are launched the ordinary way: chained
 // behind an early release, a HEVI step took 1.218 against 1.075 ms.
@@ -71,10 +73,10 @@ cudaError_t launch_chained(cudaStream_t s, void (*kernel)(Formal...), unsigned g
 }
 
 // whether a grid of this many CTAs releases the next kernel, which the device
-// keeps next_ctas CTAs of resident
-inline int chain_releases(int64_t grid, int next_ctas) {
+// keeps next_ctas CTAs of resident; light: FP32 CTAs of two warps
+inline int chain_releases(int64_t grid, int next_ctas, bool light = false) {
     constexpr int64_t SMS = 152;
-    return grid > next_ctas || 2 * grid <= SMS;
+    return grid > next_ctas || 2 * grid <= (light ? 4 * SMS : SMS);
 }
 
 // CTAs of kernel K that the current device keeps resident, 0 if it cannot be

@@ -780,11 +780,12 @@ int chain_flags(Model* md) {
             return pass ? shell_pass_ctas(md, pass) : kind == MESH_SHELL ? shell_stage_ctas(md) : arrays_stage_ctas(md);
         return hyper ? hyper_ctas(md, pass) : visc ? viscous_ctas(md, pass) : brick_stage_ctas(md);
     };
-    const int64_t grid = md->mesh->nelem;
-    int flags = chain_releases(grid, ctas(hyper || visc ? 1 : 0)) ? RELEASE_STAGE : 0;
-    if ((hyper || visc) && chain_releases(grid, ctas(0))) flags |= RELEASE_PASS;
-    if (hyper && chain_releases(grid, ctas(2))) flags |= RELEASE_HYPER1;
-    if (hyper && chain_releases(grid, ctas(3))) flags |= RELEASE_HYPER2;
+    const bool light = md->mesh->N == 2 && md->precision == CMDG_MIXED;
+    auto before = [&](int pass) { return chain_releases(md->mesh->nelem, ctas(pass), light); };
+    int flags = before(hyper || visc ? 1 : 0) ? RELEASE_STAGE : 0;
+    if ((hyper || visc) && before(0)) flags |= RELEASE_PASS;
+    if (hyper && before(2)) flags |= RELEASE_HYPER1;
+    if (hyper && before(3)) flags |= RELEASE_HYPER2;
     md->release.store(flags, std::memory_order_relaxed);
     return flags;
 }
